@@ -1,0 +1,358 @@
+// CGGI blind rotation with double-precision transforms (fft_block.cuh): same words as
+// br_kernels.cuh, whose modular transforms it replaces where the key passes the error
+// bound (binary and ternary, N = 1024 and 2048, 2 to 4 digits).
+//
+// One block per rotation, the accumulator in shared memory as coefficients (pairs j,
+// j + N/2) for all n iterations. Per iteration (cggi_blind_rotation.cpp:364-432):
+//   digits of the accumulator (binary: of (X^-a - 1) acc) -> 2l forward FFTs at once ->
+//   per slot the 2l rows times the key's limbs (ternary: E_lo - X^a E_hi) -> 2L backward
+//   FFTs at once -> round, recombine the L limbs mod p -> acc += G (ternary: the two
+//   terms (X^-a - 1) E_lo + (X^a - 1) E_hi = (X^-a - 1)(E_lo - X^a E_hi), the outer
+//   factor applied to the recombined coefficients, exactly).
+// The products by monomials outside the transforms are index shifts.
+//
+// What bounds it: the key words grow from 8 bytes a coefficient to 8 per limb (1.18 MB an
+// iteration, ternary N = 2048), read at 71 of the 75 bytes a clock that one SM gets from L2;
+// that phase takes 45% of an iteration, the FP64 pipe is busy for a third of it, and the rest
+// are the transforms' passes through shared memory and their barriers. Measured against the
+// modular kernels: ternary N = 2048, n = 630, 4096 rotations 452.7 -> 317.3 ms; 1024
+// bootstraps of binary N = 1024, n = 500 55.7 -> 40.6 ms.
+//
+// The key stream, 16 bytes per slot, component, limb and row, is read from L2 straight
+// into registers several steps ahead of its use.
+#pragma once
+
+#include "br_kernels.cuh"
+#include "fft_block.cuh"
+
+namespace tp {
+
+struct BrFftParams {
+    const double2* key;       // [it][limb][m < 8][row][component][lane < n/8]
+    const double2* tab_fwd;   // pass tables, fft_table_len(log2 n) entries
+    const double2* tab_inv;
+    const double2* roots;     // 2N: exp(2 pi i k / 2N)
+    const uint64_t* lwes;
+    uint64_t lwe_stride;
+    const uint64_t* accs;
+    uint64_t acc_stride;
+    uint64_t* out;            // coefficients
+    uint64_t batch;
+    uint32_t n;
+    uint64_t corr;
+    uint32_t dshift[8];
+    uint64_t dmask[8];
+    uint64_t ddelta[8];
+    unsigned int* err;
+    FftHead head;
+};
+
+__host__ __device__ constexpr int br_fft_threads(int logn, int dl, int limbs) {
+    return (1 << (logn - 4)) * (dl > limbs ? dl : limbs);
+}
+// The products of a slot replace its digits in place, but other threads may still read those:
+// a thread holds its products in registers until all are done, except the first of its eight
+// slots', which go to a spare area as far as shared memory allows (one block per SM from
+// N = 2048 up, two below; 4 KB are left for the LWE words).
+__host__ __device__ constexpr size_t br_fft_base_bytes(int logn, int dl, int limbs) {
+    return ((size_t)(2 * (dl > limbs ? dl : limbs)) << (logn - 1)) * 16 + ((size_t)2 << (logn - 1)) * 16 +
+           (size_t)2 * fft_table_len(logn - 1) * 16 + 8 * 16;
+}
+__host__ __device__ constexpr int br_fft_spare(int logn, int dl, int limbs) {
+    const size_t room = (logn >= 11 ? 227u * 1024u : 113u * 1024u) - 4096 - br_fft_base_bytes(logn, dl, limbs);
+    const int m = (int)(room / ((size_t)2 * limbs * (1 << (logn - 4)) * 16));
+    return m > 8 ? 8 : m;
+}
+// Shared memory in bytes: transform buffers (max(2l, 2L) polynomials), accumulator, pass
+// tables of both directions, the iteration's eight monomial factors, the spare area, LWE
+// words (32-bit).
+__host__ __device__ constexpr size_t br_fft_smem(int logn, int dl, int limbs, uint32_t n) {
+    return br_fft_base_bytes(logn, dl, limbs) +
+           (size_t)2 * limbs * br_fft_spare(logn, dl, limbs) * (1 << (logn - 4)) * 16 + (((size_t)n + 4) / 4) * 16;
+}
+
+// Asks for `bytes` (a multiple of 16, 16-byte aligned) in L2.
+__device__ __forceinline__ void l2_prefetch(const void* p, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
+// A key word pair. Volatile loads stay as far ahead of their use as the code puts them; other
+// forms sink towards it in the assembler (ternary N = 2048: 35.3k clocks an iteration, against
+// 50.2k for ld.global.nc and 41.9k for that with a warp barrier after each batch).
+__device__ __forceinline__ double2 key_ld(const double2* p) {
+    double2 v;
+    asm volatile("ld.volatile.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+    return v;
+}
+
+// The pair (coefficients j, j + n) of X^-s a, s < 4n, from a's pairs.
+template <int LOGK, typename Load>
+__device__ __forceinline__ ulonglong2 rot_pair(Load&& at, uint32_t j, uint32_t s) {
+    const uint32_t idx = j + s;
+    const ulonglong2 v = at(idx & ((1u << LOGK) - 1u));
+    const uint32_t q = (idx >> LOGK) & 3u;
+    const uint64_t a = (q & 1u) ? v.y : v.x, b = (q & 1u) ? v.x : v.y;
+    return make_ulonglong2((q & 2u) ? gl_neg(a) : a, (q == 1u || q == 2u) ? gl_neg(b) : b);
+}
+
+template <int LOGN, int VARIANT, int DL, int L>
+__global__ void __launch_bounds__(br_fft_threads(LOGN, DL, L), LOGN <= 10 ? 2 : 1)
+br_fft_kernel(const __grid_constant__ BrFftParams prm) {
+    static_assert(VARIANT == kCggiBinary || VARIANT == kCggiTernary, "CGGI only");
+    constexpr int LOGK = LOGN - 1;
+    using F = Fft<LOGK>;
+    constexpr int N = 1 << LOGN, n = F::n, TG = F::T;
+    constexpr int G = br_rgsw_per_group(VARIANT);
+    constexpr int C = 2 * G, R = 2 * DL;
+    constexpr int T = br_fft_threads(LOGN, DL, L);
+    constexpr int P = 2 * (DL > L ? DL : L);   // polynomial buffers
+    constexpr int LANES = n / 8;
+    constexpr int SPARE = br_fft_spare(LOGN, DL, L);
+    constexpr uint32_t MASK2N = 2u * N - 1u;
+    constexpr bool SIGNED = VARIANT != kCggiBinary;
+
+    extern __shared__ __align__(16) uint64_t smem[];
+    double2* buf = reinterpret_cast<double2*>(smem);                   // P n
+    ulonglong2* acc = reinterpret_cast<ulonglong2*>(buf + P * n);      // 2 n: plus corr (signed)
+    double2* tab_f = reinterpret_cast<double2*>(acc + 2 * n);
+    double2* tab_i = tab_f + fft_table_len(LOGK);
+    double2* mono_s = tab_i + fft_table_len(LOGK);
+    double2* spare = mono_s + 8;               // products of the first SPARE slot eighths
+    uint32_t* lwe_s = reinterpret_cast<uint32_t*>(spare + 2 * L * SPARE * LANES);
+
+    const int t = threadIdx.x;
+    const int grp = t / TG, tg = t % TG;       // transform group, thread in it
+    const int limb = t / LANES, lane = t % LANES;
+    for (int i = t; i < fft_table_len(LOGK); i += T) {
+        tab_f[i] = prm.tab_fwd[i];
+        tab_i[i] = prm.tab_inv[i];
+    }
+
+    for (uint64_t b = blockIdx.x; b < prm.batch; b += gridDim.x) {
+        __syncthreads();  // previous ciphertext done with lwe_s / acc
+        const uint64_t* lwe = prm.lwes + b * prm.lwe_stride;
+        bool bad = false;
+        for (uint32_t i = t; i <= prm.n; i += T) {
+            const uint64_t v = lwe[i];
+            bad |= v > MASK2N;
+            lwe_s[i] = (uint32_t)v & MASK2N;
+        }
+        if (bad) atomicOr(prm.err, 1u);
+        __syncthreads();
+        {
+            // acc = acc_in X^b (cggi_blind_rotation.cpp:242,333-358), plus the signed digits' corrector
+            const uint64_t* ain = prm.accs + b * prm.acc_stride;
+            const uint32_t s = (2u * N - lwe_s[prm.n]) & MASK2N;
+            for (int u = t; u < 2 * n; u += T) {
+                const uint64_t* a = ain + (u >> LOGK) * N;
+                ulonglong2 v = rot_pair<LOGK>(
+                    [&](uint32_t j) { return make_ulonglong2(gl_canon(a[j]), gl_canon(a[j + n])); }, u & (n - 1), s);
+                if constexpr (SIGNED) v = make_ulonglong2(gl_add(v.x, prm.corr), gl_add(v.y, prm.corr));
+                acc[u] = v;
+            }
+        }
+        __syncthreads();
+
+        // This block's share of an iteration's key, requested into L2 two iterations ahead: all
+        // blocks walk the key at the same pace, so without it each of them waits for HBM.
+        auto prefetch = [&](uint32_t it) {
+            constexpr uint32_t bytes = (uint32_t)L * 8 * R * C * LANES * 16;
+            const uint32_t share = ((bytes + gridDim.x - 1) / gridDim.x + 127u) & ~127u;
+            const uint32_t off = blockIdx.x * share;
+            if (it < prm.n && off < bytes) l2_prefetch(reinterpret_cast<const char*>(prm.key) + (uint64_t)it * bytes + off,
+                                                       min(share, bytes - off));
+        };
+        if (t == 0) {
+            prefetch(0);
+            prefetch(1);
+        }
+#pragma unroll 1
+        for (uint32_t it = 0; it < prm.n; ++it) {
+            if (t == 0) prefetch(it + 2);
+            const uint32_t a = lwe_s[it];
+            if (a == 0) continue;  // cggi_blind_rotation.cpp:369-370
+
+            if constexpr (VARIANT == kCggiTernary) {
+                // X^a in slot e = lane + m LANES: w^(a (1 + 4 brv(e))), brv(e) = 8 brv(lane) + brv3(m);
+                // the factors of m, read after the next barrier (the last readers are behind it)
+                if (t < 8) mono_s[t] = __ldg(prm.roots + ((4u * a * (__brev((uint32_t)t) >> 29)) & MASK2N));
+            }
+
+            // ---- digits and forward transforms: group grp takes digit grp % DL of half grp / DL ----
+            if (grp < R) {
+                const int h = grp / DL, d = grp - h * DL;
+                const uint32_t sh = prm.dshift[d];
+                const uint32_t mk = (uint32_t)prm.dmask[d];
+                const double off = 4503599627370496.0 + (SIGNED ? (double)prm.ddelta[d] : 0.0);
+                const ulonglong2* ah = acc + h * n;
+                double2 x[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const int j = tg + i * TG;
+                    ulonglong2 v = ah[j];
+                    if constexpr (!SIGNED) {
+                        const ulonglong2 w = rot_pair<LOGK>([&](uint32_t k) { return ah[k]; }, j, a);
+                        v = make_ulonglong2(gl_sub(w.x, v.x), gl_sub(w.y, v.y));
+                    }
+                    x[i] = make_double2(__hiloint2double(0x43300000, (int)((uint32_t)(v.x >> sh) & mk)) - off,
+                                        __hiloint2double(0x43300000, (int)((uint32_t)(v.y >> sh) & mk)) - off);
+                }
+                F::head(x, prm.head);
+                double2* pb = buf + grp * n;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) pb[fft_pos(tg + i * TG)] = x[i];
+                F::group_sync(grp);
+                F::tail(pb, tab_f, tg, grp);
+            }
+
+            // ---- slot-wise products; this thread's slots lane + m LANES, one limb ----
+            double2 o[2][8 - SPARE];
+            {
+                // Rows go in batches of BR: a batch's key words are requested while the one before it
+                // is multiplied, which keeps 8 to 12 16-byte loads per thread in flight.
+                constexpr int BR = C == 4 ? (R % 3 == 0 ? 3 : 2) : (R % 4 == 0 ? 4 : R), NB = 8 * R / BR;
+                static_assert(R % BR == 0, "a batch lies in one slot");
+                const double2* kp = prm.key + (((uint64_t)it * L + limb) * (8 * R * C)) * LANES + lane;
+                double2 kv[2][BR][C];
+                auto load = [&](int q, double2 (&k)[BR][C]) {
+#pragma unroll
+                    for (int r = 0; r < BR; ++r)
+#pragma unroll
+                        for (int c = 0; c < C; ++c) k[r][c] = key_ld(kp + ((q * BR + r) * C + c) * LANES);
+                };
+                double2 wb = make_double2(1.0, 0.0);
+                const bool on = limb < L;
+                if (on) {
+                    load(0, kv[0]);
+                    if constexpr (VARIANT == kCggiTernary)
+                        wb = __ldg(prm.roots + ((a * (1u + 32u * (__brev((uint32_t)lane) >> (35 - LOGK)))) & MASK2N));
+                }
+                __syncthreads();
+                if (on) {
+                    double2 s[C];
+#pragma unroll
+                    for (int q = 0; q < NB; ++q) {
+                        const int m = q * BR / R, pos = fft_pos(lane + m * LANES);
+                        if (q + 1 < NB) load(q + 1, kv[(q + 1) & 1]);
+                        if (q * BR % R == 0) {
+#pragma unroll
+                            for (int c = 0; c < C; ++c) s[c] = make_double2(0.0, 0.0);
+                        }
+#pragma unroll
+                        for (int r = 0; r < BR; ++r) {
+                            const double2 x = buf[(q * BR % R + r) * n + pos];
+#pragma unroll
+                            for (int c = 0; c < C; ++c) {
+                                const double2 k = kv[q & 1][r][c];
+                                s[c].x = fma(x.x, k.x, s[c].x);
+                                s[c].y = fma(x.x, k.y, s[c].y);
+                                s[c].x = fma(-x.y, k.y, s[c].x);
+                                s[c].y = fma(x.y, k.x, s[c].y);
+                            }
+                        }
+                        if ((q + 1) * BR % R != 0) continue;
+                        double2 v[2] = {s[0], s[1]};
+                        if constexpr (VARIANT == kCggiTernary) {
+                            const double2 f = mono_s[m];
+                            const double2 w = make_double2(fma(wb.x, f.x, -(wb.y * f.y)), fma(wb.x, f.y, wb.y * f.x));
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                const double2 e = s[C - 2 + h];
+                                v[h] = make_double2(fma(w.y, e.y, fma(-w.x, e.x, s[h].x)),
+                                                    fma(-w.y, e.x, fma(-w.x, e.y, s[h].y)));
+                            }
+                        }
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            if (m < SPARE) spare[(h * L + limb) * (SPARE * LANES) + pos] = v[h];
+                            else o[h][m - SPARE] = v[h];
+                        }
+                    }
+                }
+                __syncthreads();  // every read of the digits' slots before the products take their place
+                if (on) {
+#pragma unroll
+                    for (int m = SPARE; m < 8; ++m) {
+                        const int pos = fft_pos(lane + m * LANES);
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) buf[(h * L + limb) * n + pos] = o[h][m - SPARE];
+                    }
+                }
+                __syncthreads();
+            }
+
+            // ---- backward transforms, rounded coefficients back in place ----
+            if (grp < 2 * L) {
+                double2* pb = buf + grp * n;
+                F::itail(pb, tab_i, tg, grp, [&](int e) {
+                    return (e < SPARE * LANES ? spare + grp * (SPARE * LANES) : pb) + fft_pos(e);
+                });
+                F::group_sync(grp);
+                double2 x[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) x[i] = pb[fft_pos(tg + i * TG)];
+                F::ihead(x, prm.head);
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    *reinterpret_cast<ulonglong2*>(pb + fft_pos(tg + i * TG)) =
+                        make_ulonglong2(fft_round(x[i].x), fft_round(x[i].y));
+            }
+            __syncthreads();
+
+            // ---- limbs to words mod p; accumulator ----
+            const ulonglong2* wb = reinterpret_cast<const ulonglong2*>(buf);
+            ulonglong2* gb = reinterpret_cast<ulonglong2*>(buf);
+            constexpr int U = (2 * n + T - 1) / T;
+            ulonglong2 gv[U];
+#pragma unroll
+            for (int k = 0; k < U; ++k) {
+                const int u = t + k * T;
+                if ((2 * n) % T == 0 || u < 2 * n) {
+                    const int h = u >> LOGK, pos = fft_pos(u & (n - 1));
+                    uint64_t cx[L], cy[L];
+#pragma unroll
+                    for (int l = 0; l < L; ++l) {
+                        const ulonglong2 v = wb[(h * L + l) * n + pos];
+                        cx[l] = v.x;
+                        cy[l] = v.y;
+                    }
+                    gv[k] = make_ulonglong2(fft_recombine<L>(cx), fft_recombine<L>(cy));
+                    if constexpr (VARIANT == kCggiBinary) {
+                        // acc += ExtProd (mux_operator.cpp:151)
+                        const ulonglong2 v = acc[u];
+                        acc[u] = make_ulonglong2(gl_add(v.x, gv[k].x), gl_add(v.y, gv[k].y));
+                    } else {
+                        gb[(h * L) * n + pos] = gv[k];
+                    }
+                }
+            }
+            __syncthreads();
+            if constexpr (VARIANT == kCggiTernary) {
+#pragma unroll
+                for (int k = 0; k < U; ++k) {
+                    const int u = t + k * T;
+                    if ((2 * n) % T == 0 || u < 2 * n) {
+                        const ulonglong2* gh = gb + (u >> LOGK) * (L * n);
+                        const ulonglong2 w = rot_pair<LOGK>([&](uint32_t j) { return gh[fft_pos((int)j)]; },
+                                                            u & (n - 1), a);
+                        const ulonglong2 v = acc[u];
+                        acc[u] = make_ulonglong2(gl_add(v.x, gl_sub(w.x, gv[k].x)),
+                                                 gl_add(v.y, gl_sub(w.y, gv[k].y)));
+                    }
+                }
+                __syncthreads();
+            }
+        }
+
+        uint64_t* res = prm.out + b * (2ull * N);
+        for (int u = t; u < 2 * n; u += T) {
+            ulonglong2 v = acc[u];
+            if constexpr (SIGNED) v = make_ulonglong2(gl_sub(v.x, prm.corr), gl_sub(v.y, prm.corr));
+            uint64_t* r = res + (u >> LOGK) * N + (u & (n - 1));
+            r[0] = v.x;
+            r[n] = v.y;
+        }
+    }
+}
+
+}  // namespace tp

@@ -15,6 +15,8 @@
 #include "br_pair_kernel.cuh"
 #include "dispatch.h"
 #include "br_launch.h"
+#include "br_fft_kernel.cuh"
+#include "fft_host.h"
 #include "misc_kernels.cuh"
 #include "util_kernels.cuh"
 #include "ks_kernels.cuh"
@@ -233,6 +235,15 @@ struct tp_br_ctx {
     const void* quad_kernel = nullptr;
     size_t quad_smem = 0;
     int quad_cap = 0;             // resident four-CTA clusters on the device (0: unavailable)
+    // Double-precision transform kernel (br_fft_kernel.cuh), where one is built for the set and
+    // the uploaded key passes its exactness bound; runs unless a launch form was set by name.
+    const void* fft_kernel = nullptr;
+    int fft_limbs = 0, fft_cap = 0;
+    size_t fft_smem = 0;
+    const tp::FftTables* fft_tab = nullptr;
+    double2* fft_key = nullptr;
+    bool fft_ready = false;       // the key is resident and exact in this form
+    bool fft_on = true;
     // workspace for host-pointer calls
     uint64_t* ws = nullptr;
     uint64_t ws_words = 0;
@@ -298,7 +309,54 @@ static tp_status br_setup_cluster(tp_br_ctx* c) {
     return TP_OK;
 }
 
+// Whether the products of this set's digits with limb polynomials of squared norm `norm2` are exact.
+static bool br_fft_key_exact(const tp_br_ctx* c, double norm2) {
+    double dmax = 0;  // signed digits lie in [-delta, delta), unsigned ones in [0, mask]
+    for (uint32_t d = 0; d < c->prm.digits; ++d)
+        dmax = std::max(dmax, (double)(c->prm.variant == TP_BR_CGGI_BINARY ? c->kp.dmask[d] : c->kp.ddelta[d]));
+    return tp::fft_exact(c->logn - 1, 2 * c->prm.digits, dmax, norm2, c->fft_limbs, c->G);
+}
+
+// Picks the double-precision kernel of a parameter set: the fewest limbs whose error bound
+// holds for keys of random words (fewer limbs: less key to read and fewer transforms). The
+// key itself is checked at upload. Without a kernel the modular forms run.
+static void br_setup_fft(tp_br_ctx* c) {
+    if (c->prm.variant == TP_BR_BMMP_BINARY) return;
+    for (int limbs = 3; limbs <= 4; ++limbs) {
+        const void* k = tp::br_fft_kernel_ptr(c->logn, c->prm.variant, c->prm.digits, limbs);
+        c->fft_limbs = limbs;
+        if (!k || !br_fft_key_exact(c, tp::fft_typical_norm2(c->logn - 1, limbs))) continue;
+        const size_t smem = tp::br_fft_smem(c->logn, (int)c->prm.digits, limbs, c->prm.lwe_dim);
+        int per_sm = 0;
+        cudaError_t e = smem <= 227u * 1024u
+                            ? cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                            : cudaErrorInvalidValue;
+        if (e == cudaSuccess)
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k,
+                                                              tp::br_fft_threads(c->logn, (int)c->prm.digits, limbs), smem);
+        if (e == cudaSuccess && per_sm > 0) e = tp::fft_tables(c->device, c->logn - 1, &c->fft_tab);
+        if (e != cudaSuccess || per_sm < 1) {
+            cudaGetLastError();  // clear the optional probe's error
+            continue;
+        }
+        c->fft_kernel = k;
+        c->fft_smem = smem;
+        c->fft_cap = per_sm * sm_count(c->device);
+        return;
+    }
+}
+
+// A launch of a few rotations at N = 2048 leaves each of them to stream a key three times the
+// modular one (1.2 MB an iteration) through one SM, from HBM: one rotation measured 18.4 ms
+// against 17.0 in the modular form, eight 11.8.
+static bool br_uses_fft(const tp_br_ctx* c, uint64_t batch) {
+    return c->fft_ready && c->fft_on && (c->logn < 11 || batch >= 8);
+}
+
 extern "C" {
+
+static tp_status ntt_launch(uint32_t ring_dim, uint64_t count, uint64_t* out, const uint64_t* in, void* stream,
+                            bool forward, uint64_t in_stride = 0, uint64_t out_stride = 0);
 
 const char* tp_last_error(void) { return g_err.c_str(); }
 
@@ -483,6 +541,7 @@ tp_status tp_br_create(const tp_br_params* p, int device, tp_br_ctx** out) {
             cudaGetLastError();  // clear the optional probe's error
         }
     }
+    br_setup_fft(c);
     *out = c;
     return TP_OK;
 }
@@ -491,6 +550,7 @@ tp_status tp_br_destroy(tp_br_ctx* c) {
     if (!c) return TP_OK;
     cudaSetDevice(c->device);
     cudaFree(c->key);
+    cudaFree(c->fft_key);
     cudaFree(c->err);
     cudaFree(c->ws);
     delete c;
@@ -516,6 +576,19 @@ tp_status tp_br_upload_key(tp_br_ctx* c, const uint64_t* brk, uint64_t words) {
     uint64_t* stage = nullptr;
     TP_CUDA(cudaMalloc(&stage, chunk * per_group * 8));
     tp_status st = TP_OK;
+    // the limbs' transforms (one double2 per two words and limb), where there is room for them
+    unsigned long long* norm2 = nullptr;
+    bool fft = c->fft_kernel != nullptr;
+    c->fft_ready = false;
+    if (fft) {
+        cudaError_t e = cudaMalloc(&norm2, sizeof *norm2);
+        if (e == cudaSuccess) e = cudaMemset(norm2, 0, sizeof *norm2);
+        if (e == cudaSuccess && !c->fft_key) e = cudaMalloc(&c->fft_key, c->key_words * 8 * c->fft_limbs);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            fft = false;
+        }
+    }
     for (uint64_t g0 = 0; g0 < c->groups && st == TP_OK; g0 += chunk) {
         const uint64_t ng = std::min(chunk, c->groups - g0);
         cudaError_t e = cudaMemcpy(stage, brk + g0 * per_group, ng * per_group * 8, cudaMemcpyHostToDevice);
@@ -527,11 +600,32 @@ tp_status tp_br_upload_key(tp_br_ctx* c, const uint64_t* brk, uint64_t words) {
                                                                     2 * c->prm.digits, c->logn, c->loge, c->logs);
             tp::note_launch();
             e = cudaGetLastError();
+            if (e == cudaSuccess && fft) {
+                // canonical words, coefficients, limb transforms
+                tp::scale_kernel<<<(unsigned)blocks, threads>>>(stage, stage, total, 1);
+                tp::note_launch();
+                st = ntt_launch((uint32_t)N, total / N, stage, stage, nullptr, false);
+                tp::fft_key_launch(c->fft_key, stage, total / N, g0 * c->G * 4 * c->prm.digits, c->G,
+                                   2 * c->prm.digits, c->fft_limbs, *c->fft_tab, norm2, nullptr);
+                tp::note_launch();
+                e = cudaGetLastError();
+            }
         }
         if (e == cudaSuccess) e = cudaDeviceSynchronize();
         if (e != cudaSuccess) st = fail(TP_ERR_CUDA, "key upload: %s", cudaGetErrorString(e));
     }
     cudaFree(stage);
+    if (st == TP_OK && fft) {
+        unsigned long long v = 0;
+        cudaError_t e = cudaMemcpy(&v, norm2, sizeof v, cudaMemcpyDeviceToHost);
+        if (e != cudaSuccess) st = fail(TP_ERR_CUDA, "key upload: %s", cudaGetErrorString(e));
+        else c->fft_ready = br_fft_key_exact(c, (double)v);
+    }
+    cudaFree(norm2);
+    if (!c->fft_ready) {  // the modular forms run
+        cudaFree(c->fft_key);
+        c->fft_key = nullptr;
+    }
     if (st == TP_OK) c->key_ready = true;
     return st;
 }
@@ -577,7 +671,9 @@ tp_status tp_br_set_tile(tp_br_ctx* c, uint32_t coef_per_thread) {
         return fail(TP_ERR_PARAM, "ring dimension %u rotates on a CTA cluster with 4 coefficients per thread only",
                     c->prm.ring_dim);
     TP_CUDA(cudaSetDevice(c->device));
-    return br_retile(c, coef_per_thread == 4 ? 2 : 3);
+    tp_status s = br_retile(c, coef_per_thread == 4 ? 2 : 3);
+    if (s == TP_OK) c->fft_on = false;
+    return s;
 }
 
 uint32_t tp_br_get_tile(const tp_br_ctx* c) { return c ? 1u << c->loge : 0u; }
@@ -596,6 +692,7 @@ tp_status tp_br_set_split(tp_br_ctx* c, uint32_t blocks_per_rotation) {
                         blocks_per_rotation);
     }
     c->split = (int)blocks_per_rotation;
+    c->fft_on = false;
     return TP_OK;
 }
 
@@ -610,6 +707,7 @@ tp_status tp_br_set_mac_form(tp_br_ctx* c, uint32_t form) {
         return fail(TP_ERR_PARAM, "the digit-staged kernel is not built for this parameter set on this device "
                                   "(digits 3 or 4, N <= 2048, shared memory permitting)");
     c->mac = (int)form;
+    c->fft_on = false;
     return TP_OK;
 }
 
@@ -623,6 +721,7 @@ tp_status tp_br_set_radix(tp_br_ctx* c, uint32_t radix) {
         return fail(TP_ERR_PARAM, "fused radix-4 rotation kernels are not built for this parameter set "
                                   "(N = 1024 .. 4096, shared memory permitting)");
     c->radix = (int)radix;
+    c->fft_on = false;
     return TP_OK;
 }
 
@@ -633,7 +732,8 @@ tp_status tp_br_autotune(tp_br_ctx* c, uint64_t batch, uint32_t* best_coef_per_t
     if (!c->key_ready) return fail(TP_ERR_STATE, "no key uploaded");
     if (batch == 0) return fail(TP_ERR_PARAM, "empty batch");
     const uint64_t N = c->prm.ring_dim, n = c->prm.lwe_dim;
-    const uint64_t cap = (uint64_t)std::max(std::max(c->grid_caps[2], c->grid_caps[3]), c->pair_cap);  // >= quad_cap
+    const uint64_t cap = (uint64_t)std::max(std::max(c->grid_caps[2], c->grid_caps[3]),
+                                            std::max(c->pair_cap, c->fft_cap));  // >= quad_cap
     const uint64_t tb = std::min<uint64_t>(batch, 2 * cap);  // at most two waves per trial
     std::vector<uint64_t> lw(tb * (n + 1));
     uint64_t z = 0x5eedull;
@@ -674,12 +774,17 @@ tp_status tp_br_autotune(tp_br_ctx* c, uint64_t batch, uint32_t* best_coef_per_t
     int best_split = c->split;
     int best_mac = c->mac;
     int best_radix = c->radix;
-    // tile (coefficients per thread), blocks per rotation, multiply-accumulate form, NTT radix
-    struct Cand { int loge, split, mac, radix; };
-    const Cand cands[] = {{3, 1, TP_MAC_ROWWISE, 2},      {2, 1, TP_MAC_ROWWISE, 2}, {2, 1, TP_MAC_DIGIT_STAGED, 2},
+    bool best_fft = c->fft_on;
+    // tile (coefficients per thread), blocks per rotation, multiply-accumulate form, NTT radix;
+    // or the double-precision kernel (the other settings then stay as they are)
+    struct Cand { int loge, split, mac, radix; bool fft; };
+    const Cand cands[] = {{c->loge, c->split, c->mac, c->radix, true},
+                          {3, 1, TP_MAC_ROWWISE, 2},      {2, 1, TP_MAC_ROWWISE, 2}, {2, 1, TP_MAC_DIGIT_STAGED, 2},
                           {2, 1, TP_MAC_ROWWISE, 4},      {2, 1, TP_MAC_DIGIT_STAGED, 4},
                           {2, 2, TP_MAC_ROWWISE, 2},      {2, 4, TP_MAC_ROWWISE, 2}};
     for (const Cand& cd : cands) {
+        if (cd.fft && !c->fft_ready) continue;
+        c->fft_on = cd.fft;
         if ((cd.split == 2 && c->pair_cap == 0) || (cd.split == 4 && c->quad_cap == 0)) continue;
         if (cd.mac == TP_MAC_DIGIT_STAGED && !c->ds_kernel) continue;
         if (cd.radix == 4 && !(cd.mac == TP_MAC_DIGIT_STAGED ? c->r4_ds.k : c->r4_row.k)) continue;
@@ -709,6 +814,7 @@ tp_status tp_br_autotune(tp_br_ctx* c, uint64_t batch, uint32_t* best_coef_per_t
             best_split = cd.split;
             best_mac = cd.mac;
             best_radix = cd.radix;
+            best_fft = cd.fft;
         }
     }
     c->split = 1;
@@ -718,6 +824,7 @@ tp_status tp_br_autotune(tp_br_ctx* c, uint64_t batch, uint32_t* best_coef_per_t
         c->mac = best_mac;
         c->radix = best_radix;
     }
+    c->fft_on = best_fft;
     cleanup();
     if (s != TP_OK) return s;
     if (best_coef_per_thread) *best_coef_per_thread = 1u << best;
@@ -1216,9 +1323,6 @@ static tp_status ks_trace_steps(tp_ks_ctx* c, uint64_t items, uint64_t* data, ui
     }
     return TP_OK;
 }
-
-static tp_status ntt_launch(uint32_t ring_dim, uint64_t count, uint64_t* out, const uint64_t* in, void* stream,
-                            bool fwd, uint64_t in_stride, uint64_t out_stride);
 
 tp_status tp_trace_eval_batch(tp_ks_ctx* c, uint64_t batch, uint64_t* out, const uint64_t* in, void* stream) {
     if (!c || c->kind != 2) return fail(TP_ERR_PARAM, "not a packing (trace) context");
@@ -1791,7 +1895,7 @@ tp_status tp_lwe_ks_upload_key_file(tp_lwe_ks_ctx* c, const char* path) {
 }
 
 static tp_status ntt_launch(uint32_t ring_dim, uint64_t count, uint64_t* out, const uint64_t* in, void* stream,
-                            bool fwd, uint64_t in_stride = 0, uint64_t out_stride = 0) {
+                            bool fwd, uint64_t in_stride, uint64_t out_stride) {
     if (ring_dim < 128 || ring_dim > 65536 || (ring_dim & (ring_dim - 1)))
         return fail(TP_ERR_PARAM, "ring_dim must be a power of two in [128, 65536]");
     if (count == 0) return TP_OK;
@@ -2476,7 +2580,7 @@ uint64_t br_concurrency(const tp_br_ctx* c, int split) {
     if (!c) return 0;
     if (split == 2) return c->loge == 2 ? (uint64_t)c->pair_cap : 0;
     if (split == 4) return c->loge == 2 ? (uint64_t)c->quad_cap : 0;
-    return (uint64_t)br_one_block(c).cap;
+    return c->fft_ready && c->fft_on ? (uint64_t)c->fft_cap : (uint64_t)br_one_block(c).cap;
 }
 
 tp_status br_batch_launch(tp_br_ctx* c, uint64_t batch, uint64_t* results, const uint64_t* lwes,
@@ -2490,6 +2594,33 @@ tp_status br_batch_launch(tp_br_ctx* c, uint64_t batch, uint64_t* results, const
     if (acc_stride != 0 && acc_stride < 2ull * c->prm.ring_dim) return fail(TP_ERR_PARAM, "acc_stride below 2N");
     if (((uintptr_t)results & 15) || ((uintptr_t)accs & 7) || ((uintptr_t)lwes & 7))
         return fail(TP_ERR_PARAM, "results must be 16-byte aligned, lwes/accs 8-byte aligned");
+    if (br_uses_fft(c, batch)) {
+        TP_CUDA(cudaSetDevice(c->device));
+        tp::BrFftParams fp{};
+        fp.key = c->fft_key;
+        fp.tab_fwd = c->fft_tab->pass_fwd;
+        fp.tab_inv = c->fft_tab->pass_inv;
+        fp.roots = c->fft_tab->roots;
+        fp.lwes = lwes;
+        fp.lwe_stride = lwe_stride;
+        fp.accs = accs;
+        fp.acc_stride = acc_stride;
+        fp.out = results;
+        fp.batch = batch;
+        fp.n = c->prm.lwe_dim;
+        fp.corr = c->kp.corr;
+        memcpy(fp.dshift, c->kp.dshift, sizeof fp.dshift);
+        memcpy(fp.dmask, c->kp.dmask, sizeof fp.dmask);
+        memcpy(fp.ddelta, c->kp.ddelta, sizeof fp.ddelta);
+        fp.err = c->err;
+        fp.head = c->fft_tab->head;
+        void* fargs[] = {&fp};
+        TP_CUDA(cudaLaunchKernel(c->fft_kernel, dim3((unsigned)std::min<uint64_t>(batch, c->fft_cap)),
+                                 dim3(tp::br_fft_threads(c->logn, (int)c->prm.digits, c->fft_limbs)), fargs,
+                                 c->fft_smem, (cudaStream_t)stream));
+        tp::note_launch();
+        return out_coef ? TP_OK : ntt_launch(c->prm.ring_dim, 2 * batch, results, results, stream, true);
+    }
     if (split == 0) split = c->split;
     if (split == 4 && br_concurrency(c, 4) == 0) split = 2;
     if (split == 2 && br_concurrency(c, 2) == 0) split = 1;
@@ -2513,7 +2644,7 @@ tp_status br_batch_launch(tp_br_ctx* c, uint64_t batch, uint64_t* results, const
         return TP_OK;
     }
     const bool ds = br_uses_ds(c);
-    const unsigned grid = (unsigned)std::min<uint64_t>(batch, br_concurrency(c, 1));
+    const unsigned grid = (unsigned)std::min<uint64_t>(batch, br_one_block(c).cap);
     if (c->logs > 0) {
         // one rotation per cluster of 2^logs CTAs
         cudaLaunchConfig_t cfg = {};
