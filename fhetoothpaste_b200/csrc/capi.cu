@@ -21,6 +21,7 @@
 #include "util_kernels.cuh"
 #include "ks_kernels.cuh"
 #include "ks_util_kernels.cuh"
+#include "lwe_mma.cuh"
 #include "sap_kernels.cuh"
 #include "ss_kernels.cuh"
 
@@ -909,6 +910,7 @@ tp_status tp_sample_extract_batch(uint32_t ring_dim, uint64_t batch, uint64_t* o
 
 struct tp_graph {
     cudaGraphExec_t exec = nullptr;
+    uint8_t* ws = nullptr; // workspace that the graph's kernels use
     int device = 0;
     uint64_t kernels = 0;  // kernel nodes of the graph: launches per replay
 };
@@ -978,6 +980,7 @@ tp_status tp_graph_destroy(tp_graph* g) {
     if (!g) return TP_OK;
     cudaSetDevice(g->device);
     cudaGraphExecDestroy(g->exec);
+    cudaFree(g->ws);
     delete g;
     return TP_OK;
 }
@@ -1631,7 +1634,171 @@ struct tp_lwe_ks_ctx {
     uint64_t* cterm = nullptr;    // n_out + 1 words, from the key (see lwe_ks_kernel)
     bool key_ready = false;
     tp::LweKsParams kp{};
+    // tensor-core form (lwe_mma.cuh): 0 planes where it does not apply
+    int planes = 0;
+    uint32_t kpad = 0;            // n_in * digits rounded up to the K step
+    uint8_t* kbytes = nullptr;    // key bytes, 8 (n_out + 1) rows of kpad
+    cudaMemPool_t pool = nullptr; // workspaces of the calls in flight; kept up to 512 MB, gone with the context
+    int* err = nullptr;           // host-mapped: a kernel's wait ran out
 };
+
+namespace {
+
+// The tensor-map encoder of the driver, looked up once (no link dependency on libcuda).
+using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiled tensor_map_encoder() {
+    static const EncodeTiled fn = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult st;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &st) != cudaSuccess ||
+            st != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            return (EncodeTiled) nullptr;
+        }
+        return (EncodeTiled)f;
+    }();
+    return fn;
+}
+
+// `rows` rows of kpad bytes, read as boxes of box_rows x 128 bytes in the 128-byte swizzle.
+bool byte_map(CUtensorMap* m, void* base, uint64_t kpad, uint64_t rows, uint32_t box_rows) {
+    const cuuint64_t dims[2] = {kpad, rows}, strides[1] = {kpad};
+    const cuuint32_t box[2] = {(cuuint32_t)tp::kMmaK, box_rows}, step[2] = {1, 1};
+    return tensor_map_encoder()(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, base, dims, strides, box, step,
+                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// One pass of the tensor-core key switch over up to rows() ciphertexts.
+struct LweMmaPlan {
+    uint32_t rows, rows_pad, splits;
+    uint64_t plane_bytes, part_bytes;  // digit planes, then partial sums
+    uint64_t bytes() const { return plane_bytes + part_bytes; }
+};
+LweMmaPlan lwe_mma_plan(const tp_lwe_ks_ctx* c, uint64_t batch) {
+    LweMmaPlan p{};
+    // at most 256 MB of digit planes at a time
+    const uint64_t most = std::max<uint64_t>(1, (256ull << 20) / ((uint64_t)c->planes * c->kpad * tp::kMmaRows)) * tp::kMmaRows;
+    p.rows = (uint32_t)std::min(batch, most);
+    p.rows_pad = (p.rows + tp::kMmaRows - 1) / tp::kMmaRows * tp::kMmaRows;
+    const uint32_t steps = c->kpad / tp::kMmaK;
+    const uint64_t tiles = (uint64_t)(p.rows_pad / tp::kMmaRows) * ((c->n_out + tp::kMmaWords) / tp::kMmaWords);
+    const uint64_t sms = (uint64_t)sm_count(c->device);
+    // splits of K: the fewest block-steps over the waves, a block costing about six steps
+    // beside its share (fill, drain, epilogue); at least enough for exact 32-bit sums
+    uint64_t best = ~0ull;
+    for (uint32_t s = (steps + tp::kMmaMaxSteps - 1) / tp::kMmaMaxSteps; s <= steps && s <= 64; ++s) {
+        const uint32_t share = (steps + s - 1) / s;
+        if ((steps + share - 1) / share != s) continue;  // every split has steps
+        const uint64_t cost = (tiles * s + sms - 1) / sms * (share + 6) + s / 4;
+        if (cost < best) {
+            best = cost;
+            p.splits = s;
+        }
+    }
+    p.plane_bytes = (uint64_t)c->planes * p.rows_pad * c->kpad;
+    p.part_bytes = (uint64_t)p.splits * p.rows * (c->n_out + 1) * 8;
+    return p;
+}
+
+// The tensor-core form of a context whose key is on the device: key bytes, workspace pool.
+// Optional (digits of up to two bytes, room on the device): the scalar kernel takes the rest.
+cudaError_t lwe_mma_setup(tp_lwe_ks_ctx* c) {
+    const int planes = (ilog2(c->basis) + 7) / 8;
+    if (planes > 2 || !tensor_map_encoder()) return cudaSuccess;
+    const uint32_t kpad = (c->n_in * c->digits + tp::kMmaK - 1) / tp::kMmaK * tp::kMmaK;
+    cudaError_t e = cudaSuccess;
+    if (!c->kbytes) {
+        cudaMemPoolProps pp = {};
+        pp.allocType = cudaMemAllocationTypePinned;
+        pp.location.type = cudaMemLocationTypeDevice;
+        pp.location.id = c->device;
+        uint64_t keep = 512ull << 20;
+        e = planes == 1 ? cudaFuncSetAttribute(tp::lwe_mma_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)tp::mma_smem(1))
+                        : cudaFuncSetAttribute(tp::lwe_mma_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)tp::mma_smem(2));
+        if (e == cudaSuccess && !c->pool) e = cudaMemPoolCreate(&c->pool, &pp);
+        if (e == cudaSuccess) e = cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (e == cudaSuccess && !c->err) e = cudaHostAlloc(&c->err, sizeof(int), cudaHostAllocMapped);
+        if (e == cudaSuccess) e = cudaMalloc(&c->kbytes, 8ull * (c->n_out + 1) * kpad);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return cudaSuccess;
+        }
+        *c->err = 0;
+        c->planes = planes;
+        c->kpad = kpad;
+    }
+    const uint64_t threads = (uint64_t)(c->n_out + 1) * (kpad / 16);
+    tp::lwe_key_bytes_kernel<<<(unsigned)std::min<uint64_t>((threads + 255) / 256, 65535), 256>>>(
+        c->kbytes, c->key, c->n_in * c->digits, kpad, c->n_out + 1);
+    tp::note_launch();
+    return cudaGetLastError();
+}
+
+// Launches the key switch of `batch` rows described by kp. `ws`: lwe_mma_plan(batch).bytes()
+// for the tensor-core form, or null: it comes from the context's pool in stream order. A
+// stream that is being captured without a workspace, a digit above 16 bits, a context whose
+// bytes did not fit the device, or a failing allocation run the scalar kernel.
+tp_status lwe_ks_launch(const tp_lwe_ks_ctx* c, tp::LweKsParams kp, uint8_t* ws, cudaStream_t st) {
+    bool mma = c->planes > 0;
+    uint8_t* own = nullptr;
+    if (mma && *(volatile int*)c->err) return fail(TP_ERR_TIMEOUT, "a wait inside an earlier LWE key switch ran out");
+    LweMmaPlan plan{};
+    if (mma) {
+        plan = lwe_mma_plan(c, kp.batch);
+        if (!ws) {
+            cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+            mma = cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
+                  cudaMallocFromPoolAsync(&own, plan.bytes(), c->pool, st) == cudaSuccess;
+            if (!mma) cudaGetLastError();
+            ws = own;
+        }
+    }
+    if (!mma) {
+        dim3 grid((c->n_out + 1 + tp::kLweKsCols - 1) / tp::kLweKsCols,
+                  (unsigned)((kp.batch + tp::kLweKsRows - 1) / tp::kLweKsRows));
+        tp::lwe_ks_kernel<<<grid, tp::kLweKsCols, 0, st>>>(kp);
+        tp::note_launch();
+        TP_CUDA(cudaGetLastError());
+        return TP_OK;
+    }
+    CUtensorMap am, bm;
+    const uint32_t width = c->n_out + 1;
+    cudaError_t e = cudaSuccess;
+    if (!byte_map(&am, ws, c->kpad, (uint64_t)c->planes * plan.rows_pad, tp::kMmaRows) ||
+        !byte_map(&bm, c->kbytes, c->kpad, 8ull * width, tp::kMmaCols))
+        e = cudaErrorInvalidValue;
+    uint64_t* part = reinterpret_cast<uint64_t*>(ws + plan.plane_bytes);
+    for (uint64_t r0 = 0; r0 < kp.batch && e == cudaSuccess; r0 += plan.rows) {
+        const uint32_t rows = (uint32_t)std::min<uint64_t>(plan.rows, kp.batch - r0);
+        const unsigned db = (unsigned)std::min<uint64_t>(((uint64_t)rows * (c->kpad / 16) + 255) / 256, 65535);
+        const unsigned fb = (unsigned)std::min<uint64_t>(((uint64_t)rows * width + 255) / 256, 65535);
+        tp::LweMmaParams mp{part, rows, plan.rows_pad, width, c->kpad / tp::kMmaK, plan.splits, c->err};
+        const dim3 grid((rows + tp::kMmaRows - 1) / tp::kMmaRows, (width + tp::kMmaWords - 1) / tp::kMmaWords, plan.splits);
+        if (c->planes == 1) {
+            tp::lwe_digits_kernel<1><<<db, 256, 0, st>>>(ws, kp, r0, rows, plan.rows_pad, c->kpad);
+            tp::lwe_mma_kernel<1><<<grid, tp::kMmaThreads, tp::mma_smem(1), st>>>(am, bm, mp);
+        } else {
+            tp::lwe_digits_kernel<2><<<db, 256, 0, st>>>(ws, kp, r0, rows, plan.rows_pad, c->kpad);
+            tp::lwe_mma_kernel<2><<<grid, tp::kMmaThreads, tp::mma_smem(2), st>>>(am, bm, mp);
+        }
+        tp::lwe_mma_finish_kernel<<<fb, 256, 0, st>>>(kp, part, r0, rows, plan.splits);
+        for (int q = 0; q < 3; ++q) tp::note_launch();
+        e = cudaGetLastError();
+    }
+    if (own) {
+        const cudaError_t fe = cudaFreeAsync(own, st);
+        if (e == cudaSuccess) e = fe;
+    }
+    TP_CUDA(e);
+    return TP_OK;
+}
+
+}  // namespace
 
 tp_status tp_lwe_ks_create(uint64_t modulus, uint32_t n_in, uint32_t n_out, uint64_t basis, uint32_t digits,
                            int device, tp_lwe_ks_ctx** out) {
@@ -1683,6 +1850,9 @@ tp_status tp_lwe_ks_destroy(tp_lwe_ks_ctx* c) {
     cudaSetDevice(c->device);
     cudaFree(c->key);
     cudaFree(c->cterm);
+    cudaFree(c->kbytes);
+    if (c->pool) cudaMemPoolDestroy(c->pool);
+    cudaFreeHost(c->err);
     delete c;
     return TP_OK;
 }
@@ -1705,6 +1875,7 @@ tp_status tp_lwe_ks_upload_key(tp_lwe_ks_ctx* c, const uint64_t* ksk, uint64_t w
     tp::lwe_ks_cterm_kernel<<<blocks, dim3(32, tp::kCtermSlices)>>>(c->cterm, kp);
     tp::note_launch();
     TP_CUDA(cudaGetLastError());
+    TP_CUDA(lwe_mma_setup(c));
     TP_CUDA(cudaDeviceSynchronize());
     c->kp.cterm = c->cterm;
     c->key_ready = true;
@@ -1723,12 +1894,7 @@ tp_status tp_lwe_ks_batch(tp_lwe_ks_ctx* c, uint64_t batch, uint64_t* out, const
     kp.in = in;
     kp.out = out;
     kp.batch = batch;
-    dim3 grid((c->n_out + 1 + tp::kLweKsCols - 1) / tp::kLweKsCols,
-              (unsigned)((batch + tp::kLweKsRows - 1) / tp::kLweKsRows));
-    tp::lwe_ks_kernel<<<grid, tp::kLweKsCols, 0, (cudaStream_t)stream>>>(kp);
-    tp::note_launch();
-    TP_CUDA(cudaGetLastError());
-    return TP_OK;
+    return lwe_ks_launch(c, kp, nullptr, (cudaStream_t)stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -1755,8 +1921,8 @@ tp_status tp_modulus_switch_batch(uint64_t count, uint64_t* vec, uint64_t source
     return TP_OK;
 }
 
-tp_status tp_pbs_epilogue_batch(tp_lwe_ks_ctx* c, uint64_t batch, uint64_t* out_lwe, const uint64_t* rlwe_coef,
-                                uint64_t target_modulus, void* stream) {
+static tp_status pbs_epilogue(tp_lwe_ks_ctx* c, uint64_t batch, uint64_t* out_lwe, const uint64_t* rlwe_coef,
+                              uint64_t target_modulus, uint8_t* ws, void* stream) {
     if (!c) return fail(TP_ERR_PARAM, "null context");
     if (!c->key_ready) return fail(TP_ERR_STATE, "no key uploaded");
     if (c->n_in < 2 || (c->n_in & (c->n_in - 1)))
@@ -1774,12 +1940,12 @@ tp_status tp_pbs_epilogue_batch(tp_lwe_ks_ctx* c, uint64_t batch, uint64_t* out_
     kp.batch = batch;
     kp.rlwe_in = 1;
     kp.ms_log2 = (uint32_t)k;
-    dim3 grid((c->n_out + 1 + tp::kLweKsCols - 1) / tp::kLweKsCols,
-              (unsigned)((batch + tp::kLweKsRows - 1) / tp::kLweKsRows));
-    tp::lwe_ks_kernel<<<grid, tp::kLweKsCols, 0, (cudaStream_t)stream>>>(kp);
-    tp::note_launch();
-    TP_CUDA(cudaGetLastError());
-    return TP_OK;
+    return lwe_ks_launch(c, kp, ws, (cudaStream_t)stream);
+}
+
+tp_status tp_pbs_epilogue_batch(tp_lwe_ks_ctx* c, uint64_t batch, uint64_t* out_lwe, const uint64_t* rlwe_coef,
+                                uint64_t target_modulus, void* stream) {
+    return pbs_epilogue(c, batch, out_lwe, rlwe_coef, target_modulus, nullptr, stream);
 }
 
 tp_status tp_pbs_graph_create(tp_br_ctx* br, tp_lwe_ks_ctx* ks, uint64_t batch, uint64_t* rlwe_scratch,
@@ -1794,31 +1960,40 @@ tp_status tp_pbs_graph_create(tp_br_ctx* br, tp_lwe_ks_ctx* ks, uint64_t batch, 
     if (ks->device != br->device) return fail(TP_ERR_PARAM, "contexts live on different devices");
     TP_CUDA(cudaSetDevice(br->device));
     cudaStream_t s = nullptr;
-    TP_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
+    uint8_t* ws = nullptr;  // the graph's own: replays may run beside other calls on the context
+    if (ks->planes && cudaMalloc(&ws, lwe_mma_plan(ks, batch).bytes()) != cudaSuccess) cudaGetLastError();
+    cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) {
-        cudaStreamDestroy(s);
+        if (s) cudaStreamDestroy(s);
+        cudaFree(ws);
         return fail(TP_ERR_CUDA, "begin capture: %s", cudaGetErrorString(e));
     }
     ++tp::t_capturing;
     tp_status st = tp_br_blind_rotate_batch(br, batch, rlwe_scratch, lwes, (uint64_t)br->prm.lwe_dim + 1, accs,
                                             acc_stride, 1, s);
-    if (st == TP_OK) st = tp_pbs_epilogue_batch(ks, batch, out_lwe, rlwe_scratch, 2ull * br->prm.ring_dim, s);
+    if (st == TP_OK) st = pbs_epilogue(ks, batch, out_lwe, rlwe_scratch, 2ull * br->prm.ring_dim, ws, s);
     --tp::t_capturing;
     cudaGraph_t g = nullptr;
     e = cudaStreamEndCapture(s, &g);
     cudaStreamDestroy(s);
     if (st != TP_OK) {
         if (g) cudaGraphDestroy(g);
+        cudaFree(ws);
         return st;
     }
-    if (e != cudaSuccess) return fail(TP_ERR_CUDA, "end capture: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        cudaFree(ws);
+        return fail(TP_ERR_CUDA, "end capture: %s", cudaGetErrorString(e));
+    }
     auto* gr = new tp_graph();
+    gr->ws = ws;
     gr->device = br->device;
     gr->kernels = graph_kernel_nodes(g);
     e = cudaGraphInstantiate(&gr->exec, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) {
+        cudaFree(ws);
         delete gr;
         return fail(TP_ERR_CUDA, "instantiate: %s", cudaGetErrorString(e));
     }
