@@ -202,7 +202,7 @@ br_fft_kernel(const __grid_constant__ BrFftParams prm) {
 #pragma unroll
                 for (int i = 0; i < 16; ++i) pb[fft_pos(tg + i * TG)] = x[i];
                 F::group_sync(grp);
-                F::tail(pb, tab_f, tg, grp);
+                F::tail(pb, tab_f, tg, grp, [&](int e, double2 v) { pb[fft_pos(e)] = v; });
             }
 
             // ---- slot-wise products; this thread's slots lane + m LANES, one limb ----
@@ -351,6 +351,264 @@ br_fft_kernel(const __grid_constant__ BrFftParams prm) {
             uint64_t* r = res + (u >> LOGK) * N + (u & (n - 1));
             r[0] = v.x;
             r[n] = v.y;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// A few rotations: one rotation per cluster of CS blocks, for latency. One block alone reads
+// its key at a third of the rate that a full GPU's blocks get (they share lines on the way
+// from L2) and runs every transform itself. Here block c transforms the polynomials c PP ..
+// c PP + PP - 1 (PP = 1 at eight blocks), multiplies the slots [c n/CS, (c + 1) n/CS) and
+// recombines the same range of coefficients. Four exchanges an iteration through distributed
+// shared memory, each behind a cluster barrier: digit slots to their blocks, products to the
+// blocks of their limbs, rounded limbs to the blocks of their coefficients, words mod p to
+// the blocks whose digits need them. An area is written again only after a later barrier
+// than its last reads, so four barriers suffice.
+// ---------------------------------------------------------------------------
+__host__ __device__ constexpr int br_fft_cluster_polys(int dl, int limbs, int cs) {
+    return (2 * (dl > limbs ? dl : limbs) + cs - 1) / cs;
+}
+__host__ __device__ constexpr int br_fft_cluster_threads(int logn, int limbs) { return (1 << (logn - 4)) * limbs; }
+// Forward and backward buffers (PP polynomials each), digit slots (2l n/CS), limb and word
+// areas (2L n/CS, 2n), accumulator (2n), pass tables, monomial factors, LWE words.
+__host__ __device__ constexpr size_t br_fft_cluster_smem(int logn, int dl, int limbs, int cs, uint32_t n) {
+    const size_t k = (size_t)1 << (logn - 1);
+    return (2 * br_fft_cluster_polys(dl, limbs, cs) * k + (2 * dl + 2 * limbs) * (k / cs) + 4 * k +
+            2 * fft_table_len(logn - 1) + 8) * 16 + (((size_t)n + 4) / 4) * 16;
+}
+
+template <int LOGN, int VARIANT, int DL, int L, int CS>
+__global__ void __launch_bounds__(br_fft_cluster_threads(LOGN, L), 1)
+br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
+    static_assert(VARIANT == kCggiBinary || VARIANT == kCggiTernary, "CGGI only");
+    constexpr int LOGK = LOGN - 1;
+    using F = Fft<LOGK>;
+    constexpr int N = 1 << LOGN, n = F::n, TG = F::T;
+    constexpr int G = br_rgsw_per_group(VARIANT);
+    constexpr int C = 2 * G, R = 2 * DL;
+    constexpr int LANES = n / 8, T = LANES * L, M = 8 / CS, NS = n / CS;
+    constexpr int PP = br_fft_cluster_polys(DL, L, CS);
+    constexpr uint32_t MASK2N = 2u * N - 1u;
+    constexpr bool SIGNED = VARIANT != kCggiBinary;
+    static_assert(8 % CS == 0 && PP * TG <= T, "block shape");
+
+    extern __shared__ __align__(16) uint64_t smem[];
+    double2* work = reinterpret_cast<double2*>(smem);                  // PP n
+    double2* inv = work + PP * n;                                      // PP n
+    double2* dig = inv + PP * n;                                       // R NS
+    ulonglong2* lim = reinterpret_cast<ulonglong2*>(dig + R * NS);     // 2L NS
+    ulonglong2* gb = lim + 2 * L * NS;                                 // 2 n
+    ulonglong2* acc = gb + 2 * n;                                      // 2 n: plus corr (signed)
+    double2* tab_f = reinterpret_cast<double2*>(acc + 2 * n);
+    double2* tab_i = tab_f + fft_table_len(LOGK);
+    double2* mono_s = tab_i + fft_table_len(LOGK);
+    uint32_t* lwe_s = reinterpret_cast<uint32_t*>(mono_s + 8);
+
+    auto cluster = cooperative_groups::this_cluster();
+    const int c = (int)cluster.block_rank();
+    const int t = threadIdx.x;
+    const int grp = t / TG, tg = t % TG;
+    const int limb = t / LANES, lane = t % LANES;
+    for (int i = t; i < fft_table_len(LOGK); i += T) {
+        tab_f[i] = prm.tab_fwd[i];
+        tab_i[i] = prm.tab_inv[i];
+    }
+    // blocks whose forward polynomials are digits of half h
+    auto first_of = [](int h) { return h * DL / PP; };
+    auto last_of = [](int h) { return (h * DL + DL - 1) / PP; };
+    cluster.sync();  // every block of the cluster running before remote stores
+
+    const uint64_t clusters = gridDim.x / CS;
+    for (uint64_t b = blockIdx.x / CS; b < prm.batch; b += clusters) {
+        __syncthreads();
+        const uint64_t* lwe = prm.lwes + b * prm.lwe_stride;
+        bool bad = false;
+        for (uint32_t i = t; i <= prm.n; i += T) {
+            const uint64_t v = lwe[i];
+            bad |= v > MASK2N;
+            lwe_s[i] = (uint32_t)v & MASK2N;
+        }
+        if (bad) atomicOr(prm.err, 1u);
+        __syncthreads();
+        {
+            // acc = acc_in X^b, plus the signed digits' corrector
+            const uint64_t* ain = prm.accs + b * prm.acc_stride;
+            const uint32_t s = (2u * N - lwe_s[prm.n]) & MASK2N;
+            for (int u = t; u < 2 * n; u += T) {
+                const uint64_t* a = ain + (u >> LOGK) * N;
+                ulonglong2 v = rot_pair<LOGK>(
+                    [&](uint32_t j) { return make_ulonglong2(gl_canon(a[j]), gl_canon(a[j + n])); }, u & (n - 1), s);
+                if constexpr (SIGNED) v = make_ulonglong2(gl_add(v.x, prm.corr), gl_add(v.y, prm.corr));
+                acc[u] = v;
+            }
+        }
+        cluster.sync();  // every block has read the accumulator before one writes its result over it
+
+        auto prefetch = [&](uint32_t it) {  // this block's slots of an iteration's key, one thread per limb
+            constexpr uint32_t per = (uint32_t)R * C * LANES * 16;
+            if (it < prm.n && t < L)
+                l2_prefetch(reinterpret_cast<const char*>(prm.key) + (((uint64_t)it * L + t) * 8 + c * M) * per, M * per);
+        };
+        prefetch(0);
+        prefetch(1);
+#pragma unroll 1
+        for (uint32_t it = 0; it < prm.n; ++it) {
+            prefetch(it + 2);
+            const uint32_t a = lwe_s[it];
+            if (a == 0) continue;
+
+            // ---- digits and forward transforms, slots to their blocks ----
+            const int p = c * PP + grp;
+            if (grp < PP && p < R) {
+                const int h = p / DL, d = p - h * DL;
+                const uint32_t sh = prm.dshift[d];
+                const uint32_t mk = (uint32_t)prm.dmask[d];
+                const double off = 4503599627370496.0 + (SIGNED ? (double)prm.ddelta[d] : 0.0);
+                const ulonglong2* ah = acc + h * n;
+                double2 x[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const int j = tg + i * TG;
+                    ulonglong2 v = ah[j];
+                    if constexpr (!SIGNED) {
+                        const ulonglong2 w = rot_pair<LOGK>([&](uint32_t k) { return ah[k]; }, j, a);
+                        v = make_ulonglong2(gl_sub(w.x, v.x), gl_sub(w.y, v.y));
+                    }
+                    x[i] = make_double2(__hiloint2double(0x43300000, (int)((uint32_t)(v.x >> sh) & mk)) - off,
+                                        __hiloint2double(0x43300000, (int)((uint32_t)(v.y >> sh) & mk)) - off);
+                }
+                F::head(x, prm.head);
+                double2* pb = work + grp * n;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) pb[fft_pos(tg + i * TG)] = x[i];
+                F::group_sync(grp);
+                F::tail(pb, tab_f, tg, grp, [&](int e, double2 v) {
+                    cluster.map_shared_rank(dig, (unsigned)(e / NS))[p * NS + fft_pos(e % NS)] = v;
+                });
+            } else if (VARIANT == kCggiTernary && t >= T - M) {
+                const int mm = t - (T - M);
+                mono_s[mm] = __ldg(prm.roots + ((4u * a * (__brev((uint32_t)(c * M + mm)) >> 29)) & MASK2N));
+            }
+
+            // ---- slot-wise products; slots lane + (c M + mm) LANES, one limb ----
+            constexpr int BR = C == 4 ? (R % 3 == 0 ? 3 : 2) : (R % 4 == 0 ? 4 : R), NB = M * R / BR;
+            const double2* kp = prm.key + ((((uint64_t)it * L + limb) * 8 + c * M) * (R * C)) * LANES + lane;
+            double2 kv[2][BR][C];
+            auto load = [&](int q, double2 (&k)[BR][C]) {
+#pragma unroll
+                for (int r = 0; r < BR; ++r)
+#pragma unroll
+                    for (int cc = 0; cc < C; ++cc) k[r][cc] = key_ld(kp + ((q * BR + r) * C + cc) * LANES);
+            };
+            load(0, kv[0]);
+            double2 wb = make_double2(1.0, 0.0);
+            if constexpr (VARIANT == kCggiTernary)
+                wb = __ldg(prm.roots + ((a * (1u + 32u * (__brev((uint32_t)lane) >> (35 - LOGK)))) & MASK2N));
+            cluster.sync();
+            double2 s[C];
+#pragma unroll
+            for (int q = 0; q < NB; ++q) {
+                const int mm = q * BR / R, pos = fft_pos(lane + mm * LANES);
+                if (q + 1 < NB) load(q + 1, kv[(q + 1) & 1]);
+                if (q * BR % R == 0) {
+#pragma unroll
+                    for (int cc = 0; cc < C; ++cc) s[cc] = make_double2(0.0, 0.0);
+                }
+#pragma unroll
+                for (int r = 0; r < BR; ++r) {
+                    const double2 x = dig[(q * BR % R + r) * NS + pos];
+#pragma unroll
+                    for (int cc = 0; cc < C; ++cc) {
+                        const double2 k = kv[q & 1][r][cc];
+                        s[cc].x = fma(x.x, k.x, s[cc].x);
+                        s[cc].y = fma(x.x, k.y, s[cc].y);
+                        s[cc].x = fma(-x.y, k.y, s[cc].x);
+                        s[cc].y = fma(x.y, k.x, s[cc].y);
+                    }
+                }
+                if ((q + 1) * BR % R != 0) continue;
+                double2 v[2] = {s[0], s[1]};
+                if constexpr (VARIANT == kCggiTernary) {
+                    const double2 f = mono_s[mm];
+                    const double2 w = make_double2(fma(wb.x, f.x, -(wb.y * f.y)), fma(wb.x, f.y, wb.y * f.x));
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const double2 e = s[C - 2 + h];
+                        v[h] = make_double2(fma(w.y, e.y, fma(-w.x, e.x, s[h].x)),
+                                            fma(-w.y, e.x, fma(-w.x, e.y, s[h].y)));
+                    }
+                }
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int qo = h * L + limb;
+                    cluster.map_shared_rank(inv, (unsigned)(qo / PP))[(qo % PP) * n + fft_pos(c * NS + lane + mm * LANES)] = v[h];
+                }
+            }
+            cluster.sync();
+
+            // ---- backward transforms, rounded limbs to the blocks of their coefficients ----
+            if (grp < PP && p < 2 * L) {
+                double2* pb = inv + grp * n;
+                F::itail(pb, tab_i, tg, grp, [&](int e) { return pb + fft_pos(e); });
+                F::group_sync(grp);
+                double2 x[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) x[i] = pb[fft_pos(tg + i * TG)];
+                F::ihead(x, prm.head);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const int j = tg + i * TG;
+                    cluster.map_shared_rank(lim, (unsigned)(j / NS))[p * NS + j % NS] =
+                        make_ulonglong2(fft_round(x[i].x), fft_round(x[i].y));
+                }
+            }
+            cluster.sync();
+
+            // ---- words mod p to the blocks that need their half ----
+            for (int u = t; u < 2 * NS; u += T) {
+                const int h = u / NS, j = u % NS;
+                uint64_t cx[L], cy[L];
+#pragma unroll
+                for (int l = 0; l < L; ++l) {
+                    const ulonglong2 v = lim[(h * L + l) * NS + j];
+                    cx[l] = v.x;
+                    cy[l] = v.y;
+                }
+                const ulonglong2 g = make_ulonglong2(fft_recombine<L>(cx), fft_recombine<L>(cy));
+                for (int q = first_of(h); q <= last_of(h); ++q)
+                    cluster.map_shared_rank(gb, (unsigned)q)[h * n + c * NS + j] = g;
+            }
+            cluster.sync();
+
+            // ---- accumulator halves of this block ----
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (c < first_of(h) || c > last_of(h)) continue;
+                const ulonglong2* gh = gb + h * n;
+                for (int u = t; u < n; u += T) {
+                    const ulonglong2 v = acc[h * n + u], g = gh[u];
+                    if constexpr (VARIANT == kCggiBinary) {
+                        acc[h * n + u] = make_ulonglong2(gl_add(v.x, g.x), gl_add(v.y, g.y));
+                    } else {
+                        const ulonglong2 w = rot_pair<LOGK>([&](uint32_t j) { return gh[j]; }, u, a);
+                        acc[h * n + u] = make_ulonglong2(gl_add(v.x, gl_sub(w.x, g.x)), gl_add(v.y, gl_sub(w.y, g.y)));
+                    }
+                }
+            }
+            __syncthreads();
+        }
+
+        uint64_t* res = prm.out + b * (2ull * N);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (c != last_of(h)) continue;
+            for (int u = t; u < n; u += T) {
+                ulonglong2 v = acc[h * n + u];
+                if constexpr (SIGNED) v = make_ulonglong2(gl_sub(v.x, prm.corr), gl_sub(v.y, prm.corr));
+                res[h * N + u] = v.x;
+                res[h * N + u + n] = v.y;
+            }
         }
     }
 }

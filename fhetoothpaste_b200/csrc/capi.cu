@@ -241,6 +241,9 @@ struct tp_br_ctx {
     const void* fft_kernel = nullptr;
     int fft_limbs = 0, fft_cap = 0;
     size_t fft_smem = 0;
+    const void* fftc_kernel = nullptr;  // one rotation on a cluster of kFftCluster blocks
+    int fftc_cap = 0;                   // resident clusters (0: unavailable)
+    size_t fftc_smem = 0;
     const tp::FftTables* fft_tab = nullptr;
     double2* fft_key = nullptr;
     bool fft_ready = false;       // the key is resident and exact in this form
@@ -318,6 +321,22 @@ static bool br_fft_key_exact(const tp_br_ctx* c, double norm2) {
     return tp::fft_exact(c->logn - 1, 2 * c->prm.digits, dmax, norm2, c->fft_limbs, c->G);
 }
 
+// Launch of `clusters` rotations at a time in the cluster form.
+static cudaLaunchConfig_t br_fftc_config(const tp_br_ctx* c, unsigned clusters, cudaStream_t st, cudaLaunchAttribute* attr) {
+    cudaLaunchConfig_t cfg = {};
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = tp::kFftCluster;
+    attr->val.clusterDim.y = 1;
+    attr->val.clusterDim.z = 1;
+    cfg.gridDim = dim3(clusters * tp::kFftCluster);
+    cfg.blockDim = dim3(tp::br_fft_cluster_threads(c->logn, c->fft_limbs));
+    cfg.dynamicSmemBytes = c->fftc_smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
 // Picks the double-precision kernel of a parameter set: the fewest limbs whose error bound
 // holds for keys of random words (fewer limbs: less key to read and fewer transforms). The
 // key itself is checked at upload. Without a kernel the modular forms run.
@@ -343,15 +362,28 @@ static void br_setup_fft(tp_br_ctx* c) {
         c->fft_kernel = k;
         c->fft_smem = smem;
         c->fft_cap = per_sm * sm_count(c->device);
+        const void* kc = tp::br_fft_cluster_ptr(c->logn, c->prm.variant, c->prm.digits, limbs);
+        c->fftc_smem = tp::br_fft_cluster_smem(c->logn, (int)c->prm.digits, limbs, tp::kFftCluster, c->prm.lwe_dim);
+        cudaLaunchAttribute attr;
+        cudaLaunchConfig_t cfg = br_fftc_config(c, 1, nullptr, &attr);
+        e = c->fftc_smem <= 227u * 1024u
+                ? cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->fftc_smem)
+                : cudaErrorInvalidValue;
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&c->fftc_cap, kc, &cfg);
+        if (e == cudaSuccess && c->fftc_cap > 0) c->fftc_kernel = kc;
+        else cudaGetLastError();
         return;
     }
 }
 
-// A launch of a few rotations at N = 2048 leaves each of them to stream a key three times the
-// modular one (1.2 MB an iteration) through one SM, from HBM: one rotation measured 18.4 ms
-// against 17.0 in the modular form, eight 11.8.
-static bool br_uses_fft(const tp_br_ctx* c, uint64_t batch) {
-    return c->fft_ready && c->fft_on && (c->logn < 11 || batch >= 8);
+static bool br_uses_fft(const tp_br_ctx* c) { return c->fft_ready && c->fft_on; }
+
+// Few rotations run on eight blocks each (15 clusters are resident), two waves of them at N =
+// 2048, one at N = 1024. Milliseconds for n = 60, clusters against one block per rotation:
+// ternary N = 2048 (l = 3) 0.47 / 1.13 at batch 15, 0.94 / 1.10 at 30, 1.40 / 1.09 at 45; binary
+// N = 1024 (l = 4) 0.40 / 0.62 at 15, 0.80 / 0.62 at 30.
+static bool br_fft_cluster(const tp_br_ctx* c, uint64_t batch) {
+    return batch <= (uint64_t)c->fftc_cap * (c->logn >= 11 ? 2 : 1);
 }
 
 extern "C" {
@@ -2751,11 +2783,17 @@ static tp_br_ctx::Form br_one_block(const tp_br_ctx* c) {
 
 int br_cluster_ctas(const tp_br_ctx* c) { return c ? 1 << c->logs : 1; }
 
+uint64_t br_fft_blocks(const tp_br_ctx* c, uint64_t batch) {
+    if (!c || !br_uses_fft(c)) return 0;
+    return br_fft_cluster(c, batch) ? std::min<uint64_t>(batch, c->fftc_cap) * tp::kFftCluster
+                                    : std::min<uint64_t>(batch, c->fft_cap);
+}
+
 uint64_t br_concurrency(const tp_br_ctx* c, int split) {
     if (!c) return 0;
     if (split == 2) return c->loge == 2 ? (uint64_t)c->pair_cap : 0;
     if (split == 4) return c->loge == 2 ? (uint64_t)c->quad_cap : 0;
-    return c->fft_ready && c->fft_on ? (uint64_t)c->fft_cap : (uint64_t)br_one_block(c).cap;
+    return br_uses_fft(c) ? (uint64_t)c->fft_cap : (uint64_t)br_one_block(c).cap;
 }
 
 tp_status br_batch_launch(tp_br_ctx* c, uint64_t batch, uint64_t* results, const uint64_t* lwes,
@@ -2769,7 +2807,7 @@ tp_status br_batch_launch(tp_br_ctx* c, uint64_t batch, uint64_t* results, const
     if (acc_stride != 0 && acc_stride < 2ull * c->prm.ring_dim) return fail(TP_ERR_PARAM, "acc_stride below 2N");
     if (((uintptr_t)results & 15) || ((uintptr_t)accs & 7) || ((uintptr_t)lwes & 7))
         return fail(TP_ERR_PARAM, "results must be 16-byte aligned, lwes/accs 8-byte aligned");
-    if (br_uses_fft(c, batch)) {
+    if (br_uses_fft(c)) {
         TP_CUDA(cudaSetDevice(c->device));
         tp::BrFftParams fp{};
         fp.key = c->fft_key;
@@ -2790,9 +2828,16 @@ tp_status br_batch_launch(tp_br_ctx* c, uint64_t batch, uint64_t* results, const
         fp.err = c->err;
         fp.head = c->fft_tab->head;
         void* fargs[] = {&fp};
-        TP_CUDA(cudaLaunchKernel(c->fft_kernel, dim3((unsigned)std::min<uint64_t>(batch, c->fft_cap)),
-                                 dim3(tp::br_fft_threads(c->logn, (int)c->prm.digits, c->fft_limbs)), fargs,
-                                 c->fft_smem, (cudaStream_t)stream));
+        if (br_fft_cluster(c, batch)) {
+            cudaLaunchAttribute attr;
+            const cudaLaunchConfig_t cfg =
+                br_fftc_config(c, (unsigned)std::min<uint64_t>(batch, c->fftc_cap), (cudaStream_t)stream, &attr);
+            TP_CUDA(cudaLaunchKernelExC(&cfg, c->fftc_kernel, fargs));
+        } else {
+            TP_CUDA(cudaLaunchKernel(c->fft_kernel, dim3((unsigned)std::min<uint64_t>(batch, c->fft_cap)),
+                                     dim3(tp::br_fft_threads(c->logn, (int)c->prm.digits, c->fft_limbs)), fargs,
+                                     c->fft_smem, (cudaStream_t)stream));
+        }
         tp::note_launch();
         return out_coef ? TP_OK : ntt_launch(c->prm.ring_dim, 2 * batch, results, results, stream, true);
     }

@@ -151,8 +151,10 @@ struct Fft {
         for (int q = 0; q < 4; ++q) w[q] = tab[q * blocks + b];
     }
 
-    // The levels after the first pass, in place on `buf`; tab = pass 2 then pass 3 entries.
-    static __device__ __forceinline__ void tail(double2* buf, const double2* tab, int t, int g) {
+    // The levels after the first pass, in place on `buf` but for the output: slot e goes to
+    // put(e, value). tab = pass 2 then pass 3 entries.
+    template <typename Put>
+    static __device__ __forceinline__ void tail(double2* buf, const double2* tab, int t, int g, Put&& put) {
         constexpr int B2 = 1 << HEAD, B3 = n / 8;
         double2 x[8], w[4];
         load_tw(w, tab, B2, t >> 2);
@@ -174,7 +176,7 @@ struct Fft {
             for (int k = 0; k < 8; ++k) x[k] = buf[fft_pos(8 * b + k)];
             fft_radix8(x, w);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) buf[fft_pos(8 * b + k)] = x[k];
+            for (int k = 0; k < 8; ++k) put(8 * b + k, x[k]);
         }
     }
     // The inverse of tail, in place but for its input: slot e is read at *at(e). Ends before the

@@ -32,11 +32,11 @@ def inputs(rng, N, n, batch):
     return lwes, accs
 
 
-@pytest.mark.parametrize("coef", [True, False])
+@pytest.mark.parametrize("batch,coef", [(1, True), (9, False), (37, True)])  # clusters of blocks, then one block each
 @pytest.mark.parametrize("variant,N,beta,digits", SETS)
-def test_equals_oracle(native, oracle, variant, N, beta, digits, coef):
+def test_equals_oracle(native, oracle, variant, N, beta, digits, batch, coef):
     rng = np.random.default_rng(N + 10 * beta + digits)
-    n, batch = 4, 9
+    n = 4
     rot, key = rotator(variant, N, beta, digits, n, rng)
     lwes, accs = inputs(rng, N, n, batch)
     before = native.tp_kernel_launches()
@@ -47,11 +47,12 @@ def test_equals_oracle(native, oracle, variant, N, beta, digits, coef):
 
 
 @pytest.mark.parametrize("variant,N,beta,digits", SETS[:2] + SETS[5:7])
-def test_equals_modular_kernel_over_forms(native, variant, N, beta, digits):
+@pytest.mark.parametrize("batch", [2 * 148 * 2 + 3, 15])
+def test_equals_modular_kernel_over_forms(native, variant, N, beta, digits, batch):
     """Strides, a shared accumulator, results in place, more rotations than resident blocks."""
     import torch
     rng = np.random.default_rng(7)
-    n, batch = 3, 2 * 148 * 2 + 3
+    n = 3
     rot, _ = rotator(variant, N, beta, digits, n, rng)
     lwes, accs = inputs(rng, N, n, batch)
     wide = np.zeros((batch, n + 6), np.uint64)
