@@ -241,9 +241,11 @@ struct tp_br_ctx {
     const void* fft_kernel = nullptr;
     int fft_limbs = 0, fft_cap = 0;
     size_t fft_smem = 0;
-    const void* fftc_kernel = nullptr;  // one rotation on a cluster of kFftCluster blocks
-    int fftc_cap = 0;                   // resident clusters (0: unavailable)
-    size_t fftc_smem = 0;
+    struct FftCluster {                 // one rotation on a cluster of 2^(i + 1) blocks, i < 3
+        const void* k = nullptr;
+        int cap = 0;                    // resident clusters (0: unavailable)
+        size_t smem = 0;
+    } fftc[3];
     const tp::FftTables* fft_tab = nullptr;
     double2* fft_key = nullptr;
     bool fft_ready = false;       // the key is resident and exact in this form
@@ -321,16 +323,17 @@ static bool br_fft_key_exact(const tp_br_ctx* c, double norm2) {
     return tp::fft_exact(c->logn - 1, 2 * c->prm.digits, dmax, norm2, c->fft_limbs, c->G);
 }
 
-// Launch of `clusters` rotations at a time in the cluster form.
-static cudaLaunchConfig_t br_fftc_config(const tp_br_ctx* c, unsigned clusters, cudaStream_t st, cudaLaunchAttribute* attr) {
+// Launch of `clusters` rotations at a time on clusters of 2^(i + 1) blocks.
+static cudaLaunchConfig_t br_fftc_config(const tp_br_ctx* c, int i, unsigned clusters, cudaStream_t st,
+                                         cudaLaunchAttribute* attr) {
     cudaLaunchConfig_t cfg = {};
     attr->id = cudaLaunchAttributeClusterDimension;
-    attr->val.clusterDim.x = tp::kFftCluster;
+    attr->val.clusterDim.x = 2u << i;
     attr->val.clusterDim.y = 1;
     attr->val.clusterDim.z = 1;
-    cfg.gridDim = dim3(clusters * tp::kFftCluster);
+    cfg.gridDim = dim3(clusters * (2u << i));
     cfg.blockDim = dim3(tp::br_fft_cluster_threads(c->logn, c->fft_limbs));
-    cfg.dynamicSmemBytes = c->fftc_smem;
+    cfg.dynamicSmemBytes = c->fftc[i].smem;
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
@@ -362,28 +365,43 @@ static void br_setup_fft(tp_br_ctx* c) {
         c->fft_kernel = k;
         c->fft_smem = smem;
         c->fft_cap = per_sm * sm_count(c->device);
-        const void* kc = tp::br_fft_cluster_ptr(c->logn, c->prm.variant, c->prm.digits, limbs);
-        c->fftc_smem = tp::br_fft_cluster_smem(c->logn, (int)c->prm.digits, limbs, tp::kFftCluster, c->prm.lwe_dim);
-        cudaLaunchAttribute attr;
-        cudaLaunchConfig_t cfg = br_fftc_config(c, 1, nullptr, &attr);
-        e = c->fftc_smem <= 227u * 1024u
-                ? cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->fftc_smem)
-                : cudaErrorInvalidValue;
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&c->fftc_cap, kc, &cfg);
-        if (e == cudaSuccess && c->fftc_cap > 0) c->fftc_kernel = kc;
-        else cudaGetLastError();
+        for (int i = 0; i < 3; ++i) {
+            auto& f = c->fftc[i];
+            const void* kc = tp::br_fft_cluster_ptr(c->logn, c->prm.variant, c->prm.digits, limbs, 2 << i);
+            f.smem = tp::br_fft_cluster_smem(c->logn, (int)c->prm.digits, limbs, 2 << i, c->prm.lwe_dim);
+            if (!kc || f.smem > 227u * 1024u) continue;
+            cudaLaunchAttribute attr;
+            const cudaLaunchConfig_t cfg = br_fftc_config(c, i, 1, nullptr, &attr);
+            e = cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem);
+            if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&f.cap, kc, &cfg);
+            if (e == cudaSuccess && f.cap > 0) f.k = kc;
+            else cudaGetLastError();
+        }
         return;
     }
 }
 
-static bool br_uses_fft(const tp_br_ctx* c) { return c->fft_ready && c->fft_on; }
-
-// Few rotations run on eight blocks each (15 clusters are resident), two waves of them at N =
-// 2048, one at N = 1024. Milliseconds for n = 60, clusters against one block per rotation:
-// ternary N = 2048 (l = 3) 0.47 / 1.13 at batch 15, 0.94 / 1.10 at 30, 1.40 / 1.09 at 45; binary
-// N = 1024 (l = 4) 0.40 / 0.62 at 15, 0.80 / 0.62 at 30.
-static bool br_fft_cluster(const tp_br_ctx* c, uint64_t batch) {
-    return batch <= (uint64_t)c->fftc_cap * (c->logn >= 11 ? 2 : 1);
+// The form of a launch of `batch` rotations whose context left the choice open: clusters of
+// 2^(i + 1) blocks per rotation in double precision (i = 0 .. 2), one block in double
+// precision (kFftOneBlock), or the modular kernels (kModular, kModularPair: two blocks per
+// rotation). Milliseconds at n = 60 (clusters of 8 / 4 / 2, one block, modular, modular pair),
+// one wave each; 15, 30, 74 clusters are resident:
+//   ternary N = 2048, l = 3:       0.48 / 0.62 / -    1.09  1.53  1.09
+//   binary N = 2048, l = 4:        0.54 / 0.65 / -    1.28  1.72  1.04
+//   ternary N = 2048, l = 4 (2^16) 0.59 / 0.84 / -    2.07  2.06  1.31
+//   binary N = 1024, l = 4:        0.40 / 0.48 / 0.57 0.63  0.98  -
+//   ternary N = 1024, l = 4 (2^16) 0.37 / 0.49 / 0.68 1.46  1.24  -
+// So the widest cluster that takes the batch in one wave, then (N = 2048) the modular pair in
+// its one wave, then one block. Where a block reads 64 or more key polynomials an iteration
+// (ternary, four digits, four limbs) its key stream leaves one block no faster than modular.
+enum { kFftOneBlock = 3, kModularPair = 4, kModular = 5 };
+static int br_form(const tp_br_ctx* c, uint64_t batch) {
+    if (!c->fft_ready || !c->fft_on) return kModular;
+    for (int i = 2; i >= 0; --i)
+        if (batch <= (uint64_t)c->fftc[i].cap) return i;
+    const bool wide = c->G * 2 * (int)c->prm.digits * c->fft_limbs >= 64;
+    if ((c->logn >= 11 || wide) && c->loge == 2 && batch <= (uint64_t)c->pair_cap) return kModularPair;
+    return wide ? kModular : kFftOneBlock;
 }
 
 extern "C" {
@@ -2784,16 +2802,16 @@ static tp_br_ctx::Form br_one_block(const tp_br_ctx* c) {
 int br_cluster_ctas(const tp_br_ctx* c) { return c ? 1 << c->logs : 1; }
 
 uint64_t br_fft_blocks(const tp_br_ctx* c, uint64_t batch) {
-    if (!c || !br_uses_fft(c)) return 0;
-    return br_fft_cluster(c, batch) ? std::min<uint64_t>(batch, c->fftc_cap) * tp::kFftCluster
-                                    : std::min<uint64_t>(batch, c->fft_cap);
+    const int i = c ? br_form(c, batch) : kModular;
+    if (i > kFftOneBlock) return 0;
+    return i < kFftOneBlock ? batch << (i + 1) : std::min<uint64_t>(batch, c->fft_cap);
 }
 
 uint64_t br_concurrency(const tp_br_ctx* c, int split) {
     if (!c) return 0;
     if (split == 2) return c->loge == 2 ? (uint64_t)c->pair_cap : 0;
     if (split == 4) return c->loge == 2 ? (uint64_t)c->quad_cap : 0;
-    return br_uses_fft(c) ? (uint64_t)c->fft_cap : (uint64_t)br_one_block(c).cap;
+    return (uint64_t)br_one_block(c).cap;
 }
 
 tp_status br_batch_launch(tp_br_ctx* c, uint64_t batch, uint64_t* results, const uint64_t* lwes,
@@ -2807,7 +2825,8 @@ tp_status br_batch_launch(tp_br_ctx* c, uint64_t batch, uint64_t* results, const
     if (acc_stride != 0 && acc_stride < 2ull * c->prm.ring_dim) return fail(TP_ERR_PARAM, "acc_stride below 2N");
     if (((uintptr_t)results & 15) || ((uintptr_t)accs & 7) || ((uintptr_t)lwes & 7))
         return fail(TP_ERR_PARAM, "results must be 16-byte aligned, lwes/accs 8-byte aligned");
-    if (br_uses_fft(c)) {
+    const int form = br_form(c, batch);
+    if (form <= kFftOneBlock) {
         TP_CUDA(cudaSetDevice(c->device));
         tp::BrFftParams fp{};
         fp.key = c->fft_key;
@@ -2828,11 +2847,11 @@ tp_status br_batch_launch(tp_br_ctx* c, uint64_t batch, uint64_t* results, const
         fp.err = c->err;
         fp.head = c->fft_tab->head;
         void* fargs[] = {&fp};
-        if (br_fft_cluster(c, batch)) {
+        if (const int i = form; i < kFftOneBlock) {
             cudaLaunchAttribute attr;
             const cudaLaunchConfig_t cfg =
-                br_fftc_config(c, (unsigned)std::min<uint64_t>(batch, c->fftc_cap), (cudaStream_t)stream, &attr);
-            TP_CUDA(cudaLaunchKernelExC(&cfg, c->fftc_kernel, fargs));
+                br_fftc_config(c, i, (unsigned)std::min<uint64_t>(batch, c->fftc[i].cap), (cudaStream_t)stream, &attr);
+            TP_CUDA(cudaLaunchKernelExC(&cfg, c->fftc[i].k, fargs));
         } else {
             TP_CUDA(cudaLaunchKernel(c->fft_kernel, dim3((unsigned)std::min<uint64_t>(batch, c->fft_cap)),
                                      dim3(tp::br_fft_threads(c->logn, (int)c->prm.digits, c->fft_limbs)), fargs,
@@ -2841,7 +2860,7 @@ tp_status br_batch_launch(tp_br_ctx* c, uint64_t batch, uint64_t* results, const
         tp::note_launch();
         return out_coef ? TP_OK : ntt_launch(c->prm.ring_dim, 2 * batch, results, results, stream, true);
     }
-    if (split == 0) split = c->split;
+    if (split == 0) split = form == kModularPair ? 2 : c->split;
     if (split == 4 && br_concurrency(c, 4) == 0) split = 2;
     if (split == 2 && br_concurrency(c, 2) == 0) split = 1;
     TP_CUDA(cudaSetDevice(c->device));

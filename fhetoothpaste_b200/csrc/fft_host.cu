@@ -118,17 +118,27 @@ __global__ void __launch_bounds__(256) fft_key_kernel(double2* __restrict__ dst,
     }
 }
 
-template <int LOGN, int VARIANT>
+template <int LOGN, int VARIANT, int CS>
 const void* pick_cluster(uint32_t digits, int limbs) {
     switch (digits * 10 + limbs) {
-        case 23: return (const void*)br_fft_cluster_kernel<LOGN, VARIANT, 2, 3, kFftCluster>;
-        case 24: return (const void*)br_fft_cluster_kernel<LOGN, VARIANT, 2, 4, kFftCluster>;
-        case 33: return (const void*)br_fft_cluster_kernel<LOGN, VARIANT, 3, 3, kFftCluster>;
-        case 34: return (const void*)br_fft_cluster_kernel<LOGN, VARIANT, 3, 4, kFftCluster>;
-        case 43: return (const void*)br_fft_cluster_kernel<LOGN, VARIANT, 4, 3, kFftCluster>;
-        case 44: return (const void*)br_fft_cluster_kernel<LOGN, VARIANT, 4, 4, kFftCluster>;
+        case 23: return (const void*)br_fft_cluster_kernel<LOGN, VARIANT, 2, 3, CS>;
+        case 24: return (const void*)br_fft_cluster_kernel<LOGN, VARIANT, 2, 4, CS>;
+        case 33: return (const void*)br_fft_cluster_kernel<LOGN, VARIANT, 3, 3, CS>;
+        case 34: return (const void*)br_fft_cluster_kernel<LOGN, VARIANT, 3, 4, CS>;
+        case 43: return (const void*)br_fft_cluster_kernel<LOGN, VARIANT, 4, 3, CS>;
+        case 44: return (const void*)br_fft_cluster_kernel<LOGN, VARIANT, 4, 4, CS>;
         default: return nullptr;
     }
+}
+template <int VARIANT>
+const void* pick_cluster(int logn, uint32_t digits, int limbs, int cs) {
+    if (logn == 10)
+        return cs == 2   ? pick_cluster<10, VARIANT, 2>(digits, limbs)
+               : cs == 4 ? pick_cluster<10, VARIANT, 4>(digits, limbs)
+                         : pick_cluster<10, VARIANT, 8>(digits, limbs);
+    if (logn == 11 && cs >= 4)
+        return cs == 4 ? pick_cluster<11, VARIANT, 4>(digits, limbs) : pick_cluster<11, VARIANT, 8>(digits, limbs);
+    return nullptr;
 }
 
 template <int LOGN, int VARIANT>
@@ -154,13 +164,9 @@ const void* br_fft_kernel_ptr(int logn, int variant, uint32_t digits, int limbs)
     return nullptr;
 }
 
-const void* br_fft_cluster_ptr(int logn, int variant, uint32_t digits, int limbs) {
-    if (variant == kCggiBinary)
-        return logn == 10 ? pick_cluster<10, kCggiBinary>(digits, limbs)
-                          : logn == 11 ? pick_cluster<11, kCggiBinary>(digits, limbs) : nullptr;
-    if (variant == kCggiTernary)
-        return logn == 10 ? pick_cluster<10, kCggiTernary>(digits, limbs)
-                          : logn == 11 ? pick_cluster<11, kCggiTernary>(digits, limbs) : nullptr;
+const void* br_fft_cluster_ptr(int logn, int variant, uint32_t digits, int limbs, int cs) {
+    if (variant == kCggiBinary) return pick_cluster<kCggiBinary>(logn, digits, limbs, cs);
+    if (variant == kCggiTernary) return pick_cluster<kCggiTernary>(logn, digits, limbs, cs);
     return nullptr;
 }
 
