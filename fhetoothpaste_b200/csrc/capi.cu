@@ -17,6 +17,7 @@
 #include "br_launch.h"
 #include "br_fft_kernel.cuh"
 #include "fft_host.h"
+#include "ks_fft_kernel.cuh"
 #include "misc_kernels.cuh"
 #include "util_kernels.cuh"
 #include "ks_kernels.cuh"
@@ -1111,8 +1112,43 @@ struct tp_ks_ctx {
     std::vector<uint64_t> consec_off;  // per level: offset into the plan (words)
     std::vector<uint32_t> consec_cnt;  // per level: nodes of one pack
     uint64_t* zero = nullptr;          // 2N zero words
+    // double-precision form of the modes with coefficient results (packing contexts, N = 1024 and
+    // 2048), where one is built and every key passes its exactness bound; off once a tile is set
+    const void* fft_kernel = nullptr;
+    int fft_limbs = 0, fft_cap = 0;
+    const tp::FftTables* fft_tab = nullptr;
+    double2* fft_key = nullptr;
+    bool fft_ready = false, fft_on = true;
     std::mutex mu;
 };
+
+// Whether the digits' products with limb polynomials of squared norm `norm2` are exact.
+static bool ks_fft_key_exact(const tp_ks_ctx* c, double norm2) {
+    double dmax = 0;
+    for (uint32_t d = 0; d < c->digits; ++d) dmax = std::max(dmax, (double)c->kp.ddelta[d]);
+    return tp::fft_exact(c->logn - 1, c->digits, dmax, norm2, c->fft_limbs, 1);
+}
+
+static void ks_setup_fft(tp_ks_ctx* c) {
+    if (c->kind != 2) return;
+    for (int limbs = 3; limbs <= 4; ++limbs) {
+        const void* k = tp::ks_fft_kernel_ptr(c->logn, c->digits, limbs);
+        c->fft_limbs = limbs;
+        if (!k || !ks_fft_key_exact(c, tp::fft_typical_norm2(c->logn - 1, limbs))) continue;
+        const size_t smem = tp::ks_fft_smem(c->logn, limbs);
+        int per_sm = 0;
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess)
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, tp::ks_fft_threads(c->logn, limbs), smem);
+        if (e == cudaSuccess && per_sm > 0) e = tp::fft_tables(c->device, c->logn - 1, &c->fft_tab);
+        if (e == cudaSuccess && per_sm > 0) {
+            c->fft_kernel = k;
+            c->fft_cap = per_sm * sm_count(c->device);
+            return;
+        }
+        cudaGetLastError();
+    }
+}
 
 static tp_status ks_create(int kind, uint32_t ring_dim, uint64_t basis, uint32_t digits, uint32_t index, int device,
                            tp_ks_ctx** out) {
@@ -1203,6 +1239,7 @@ static tp_status ks_create(int kind, uint32_t ring_dim, uint64_t basis, uint32_t
             }
         }
     }
+    ks_setup_fft(c);
     *out = c;
     return TP_OK;
 }
@@ -1224,6 +1261,7 @@ tp_status tp_ks_destroy(tp_ks_ctx* c) {
     if (!c) return TP_OK;
     cudaSetDevice(c->device);
     cudaFree(c->key);
+    cudaFree(c->fft_key);
     cudaFree(c->work);
     cudaFree(c->consec_plan);
     cudaFree(c->zero);
@@ -1232,6 +1270,33 @@ tp_status tp_ks_destroy(tp_ks_ctx* c) {
 }
 
 uint64_t tp_ks_key_words(const tp_ks_ctx* c) { return c ? c->key_words : 0; }
+
+// The limbs' transforms of the keys in `stage` (reference layout, overwritten), where there is
+// room for them and they pass the bound; without them the modular kernel runs.
+static cudaError_t ks_upload_fft(tp_ks_ctx* c, uint64_t* stage) {
+    c->fft_ready = false;
+    unsigned long long* norm2 = nullptr;
+    unsigned long long v = 0;
+    const uint64_t polys = c->key_words / c->N;
+    cudaError_t e = cudaMalloc(&norm2, sizeof *norm2);
+    if (e == cudaSuccess && !c->fft_key) e = cudaMalloc(&c->fft_key, c->key_words * 8 * c->fft_limbs);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(norm2);
+        return cudaSuccess;
+    }
+    e = cudaMemset(norm2, 0, sizeof *norm2);
+    tp::scale_kernel<<<(unsigned)std::min<uint64_t>((c->key_words + 255) / 256, 65535), 256>>>(stage, stage, c->key_words, 1);
+    tp::note_launch();
+    if (e == cudaSuccess && ntt_launch(c->N, polys, stage, stage, nullptr, false) != TP_OK) e = cudaErrorLaunchFailure;
+    tp::fft_key_launch(c->fft_key, stage, polys, 0, 1, c->digits, c->fft_limbs, *c->fft_tab, norm2, nullptr);
+    tp::note_launch();
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpy(&v, norm2, sizeof v, cudaMemcpyDeviceToHost);
+    cudaFree(norm2);
+    if (e == cudaSuccess) c->fft_ready = ks_fft_key_exact(c, (double)v);
+    return e;
+}
 
 tp_status tp_ks_upload_key(tp_ks_ctx* c, const uint64_t* ksk, uint64_t words) {
     if (!c || !ksk) return fail(TP_ERR_PARAM, "null argument");
@@ -1253,6 +1318,7 @@ tp_status tp_ks_upload_key(tp_ks_ctx* c, const uint64_t* ksk, uint64_t words) {
         tp::note_launch();
         e = cudaGetLastError();
     }
+    if (e == cudaSuccess && c->fft_kernel) e = ks_upload_fft(c, stage);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     cudaFree(stage);
     if (e != cudaSuccess) return fail(TP_ERR_CUDA, "key upload: %s", cudaGetErrorString(e));
@@ -1263,6 +1329,21 @@ tp_status tp_ks_upload_key(tp_ks_ctx* c, const uint64_t* ksk, uint64_t words) {
 static tp_status ks_launch(tp_ks_ctx* c, int mode, const tp::KsKernelParams& kp, cudaStream_t st) {
     tp::KsKernelParams p = kp;
     void* args[] = {&p};
+    if (c->fft_ready && c->fft_on && mode >= tp::kKsMerge) {
+        tp::KsFftParams fp{};
+        fp.ks = kp;
+        fp.key = c->fft_key + (uint64_t)(kp.key - c->key) / 2 * c->fft_limbs;  // kp.key: one of the context's keys
+        fp.tab_fwd = c->fft_tab->pass_fwd;
+        fp.tab_inv = c->fft_tab->pass_inv;
+        fp.mode = mode;
+        fp.head = c->fft_tab->head;
+        void* fargs[] = {&fp};
+        TP_CUDA(cudaLaunchKernel(c->fft_kernel, dim3((unsigned)std::min<uint64_t>(kp.items, c->fft_cap)),
+                                 dim3(tp::ks_fft_threads(c->logn, c->fft_limbs)), fargs,
+                                 tp::ks_fft_smem(c->logn, c->fft_limbs), st));
+        tp::note_launch();
+        return TP_OK;
+    }
     if (c->logs > 0) {
         // one item per cluster of 2^logs CTAs
         const uint64_t clusters = std::min<uint64_t>(kp.items, (uint64_t)c->cluster_cap[mode]);
@@ -1295,6 +1376,7 @@ tp_status tp_ks_set_tile(tp_ks_ctx* c, uint32_t coef_per_thread) {
     if (coef_per_thread != 4 && coef_per_thread != 8) return fail(TP_ERR_PARAM, "tile must be 4 or 8");
     const int loge = coef_per_thread == 4 ? 2 : 3;
     std::lock_guard<std::mutex> lk(c->mu);
+    c->fft_on = false;  // a tile set by name runs the modular kernels
     if (loge == c->loge) return TP_OK;
     if (c->logs > 0) return fail(TP_ERR_PARAM, "ring sizes above 4096 run on clusters with 4 coefficients per thread");
     TP_CUDA(cudaSetDevice(c->device));
@@ -1534,8 +1616,9 @@ tp_status tp_pack_consecutive_batch(tp_ks_ctx* c, uint64_t packs, uint64_t len, 
 // key 2^L + 1, shift N >> L), leaving each region's root at its first node. The
 // merge at a level depends on that level only, never on the node's place in the
 // whole tree, so a subtree runs exactly like the bottom of a smaller tree.
+// `leaf`: the regions' LWE inputs when the first level sets its leaves up itself (level0 = 0).
 static tp_status pack_merge_levels(tp_ks_ctx* c, uint64_t packs, uint64_t count, int level0, uint64_t* work,
-                                   cudaStream_t st) {
+                                   const uint64_t* leaf, cudaStream_t st) {
     const uint64_t N = c->N;
     const uint64_t kw = (uint64_t)c->digits * 2 * N;
     tp::KsKernelParams kp = c->kp;
@@ -1551,10 +1634,25 @@ static tp_status pack_merge_levels(tp_ks_ctx* c, uint64_t packs, uint64_t count,
         kp.auto_index = (1u << L) + 1;
         kp.auto_index_inv = inv_mod_2n(kp.auto_index, 2 * (uint32_t)N);
         kp.shift = (uint32_t)(N >> L);
+        kp.leaf = k == 1 ? leaf : nullptr;
+        kp.leaf_log = (uint32_t)levels;
         tp_status s = ks_launch(c, tp::kKsMerge, kp, st);
         if (s != TP_OK) return s;
     }
     return TP_OK;
+}
+
+// Leaves and merges of `packs` regions of `len` LWE inputs in `work` (L0Setup and the tree,
+// lwe_to_rlwe_packing.cpp:129-224). The double-precision kernel's first level reads the LWE rows
+// itself, which saves a pass over nodes twice their size.
+static tp_status pack_tree(tp_ks_ctx* c, uint64_t packs, uint64_t len, uint64_t* work, const uint64_t* in, cudaStream_t st) {
+    if (len > 1 && c->fft_ready && c->fft_on) return pack_merge_levels(c, packs, len, 0, work, in, st);
+    const uint64_t need = packs * len * 2 * c->N;
+    tp::pack_l0_kernel<<<(unsigned)std::min<uint64_t>((need + 255) / 256, 65535), 256, 0, st>>>(
+        work, in, packs, (uint32_t)len, (uint32_t)ilog2(len), (uint32_t)c->logn, c->tab->n_inv);
+    tp::note_launch();
+    TP_CUDA(cudaGetLastError());
+    return pack_merge_levels(c, packs, len, 0, work, nullptr, st);
 }
 
 // The context's work area holds at least `words` words.
@@ -1589,14 +1687,7 @@ tp_status tp_pack_batch(tp_ks_ctx* c, uint64_t packs, uint64_t len, uint64_t* ou
     cudaStream_t st = (cudaStream_t)stream;
     const int log_len = ilog2(len);
     {
-        const uint64_t blocks = std::min<uint64_t>((need + 255) / 256, 65535 * 4ull);
-        tp::pack_l0_kernel<<<(unsigned)std::min<uint64_t>(blocks, 65535), 256, 0, st>>>(
-            c->work, in, packs, (uint32_t)len, (uint32_t)log_len, (uint32_t)c->logn, c->tab->n_inv);
-        tp::note_launch();
-        TP_CUDA(cudaGetLastError());
-    }
-    {
-        tp_status s = pack_merge_levels(c, packs, len, 0, c->work, st);
+        tp_status s = pack_tree(c, packs, len, c->work, in, st);
         if (s != TP_OK) return s;
     }
     // trailing traces when len < N (lwe_to_rlwe_packing.cpp:228-234)
@@ -1628,11 +1719,7 @@ tp_status tp_pack_subtree_batch(tp_ks_ctx* c, uint64_t packs, uint64_t len, uint
     tp_status s = pack_work(c, need);
     if (s != TP_OK) return s;
     cudaStream_t st = (cudaStream_t)stream;
-    tp::pack_l0_kernel<<<(unsigned)std::min<uint64_t>((need + 255) / 256, 65535), 256, 0, st>>>(
-        c->work, in, packs, (uint32_t)len, (uint32_t)ilog2(len), (uint32_t)c->logn, c->tab->n_inv);
-    tp::note_launch();
-    TP_CUDA(cudaGetLastError());
-    s = pack_merge_levels(c, packs, len, 0, c->work, st);
+    s = pack_tree(c, packs, len, c->work, in, st);
     if (s != TP_OK) return s;
     TP_CUDA(cudaMemcpy2DAsync(out, 2 * N * 8, c->work, len * 2 * N * 8, 2 * N * 8, packs, cudaMemcpyDeviceToDevice, st));
     return TP_OK;
@@ -1661,7 +1748,7 @@ tp_status tp_pack_merge_batch(tp_ks_ctx* c, uint64_t packs, uint64_t count, uint
     if (s != TP_OK) return s;
     cudaStream_t st = (cudaStream_t)stream;
     TP_CUDA(cudaMemcpyAsync(c->work, nodes, need * 8, cudaMemcpyDeviceToDevice, st));
-    s = pack_merge_levels(c, packs, count, (int)level0, c->work, st);
+    s = pack_merge_levels(c, packs, count, (int)level0, c->work, nullptr, st);
     if (s != TP_OK) return s;
     if (finish) {
         s = ks_trace_steps(c, packs, c->work, count * 2 * N, c->logn, top + 1, st);
@@ -2743,19 +2830,12 @@ extern "C" tp_status tp_pack_batch_noalloc(tp_ks_ctx* c, uint64_t packs, uint64_
         }
         work = g_pack_scratch_addr[c->device];
     }
-    // Every word of the nodes in use is written by the set-up kernel below
+    // Every word of the nodes in use is written by the set-up (or the first merges)
     // before any merge reads it, so nothing left by an earlier call is read.
     cudaStream_t st = (cudaStream_t)stream;
     const int log_len = ilog2(len);
     {
-        const uint64_t blocks = std::min<uint64_t>((need + 255) / 256, 65535);
-        tp::pack_l0_kernel<<<(unsigned)blocks, 256, 0, st>>>(work, in, packs, (uint32_t)len, (uint32_t)log_len,
-                                                            (uint32_t)c->logn, c->tab->n_inv);
-        tp::note_launch();
-        TP_CUDA(cudaGetLastError());
-    }
-    {
-        tp_status s = pack_merge_levels(c, packs, len, 0, work, st);  // the merges of tp_pack_batch
+        tp_status s = pack_tree(c, packs, len, work, in, st);  // as in tp_pack_batch
         if (s != TP_OK) return s;
     }
     {

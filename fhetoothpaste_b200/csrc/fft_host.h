@@ -50,4 +50,7 @@ const void* br_fft_kernel_ptr(int logn, int variant, uint32_t digits, int limbs)
 // One rotation on a cluster of cs blocks (2, 4 or 8; nullptr where not built).
 const void* br_fft_cluster_ptr(int logn, int variant, uint32_t digits, int limbs, int cs);
 
+// Key switches with coefficient results (ks_fft_kernel.cuh).
+const void* ks_fft_kernel_ptr(int logn, uint32_t digits, int limbs);
+
 }  // namespace tp

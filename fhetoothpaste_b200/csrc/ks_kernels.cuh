@@ -51,6 +51,11 @@ struct KsKernelParams {
     const uint64_t* zero;
     uint32_t pair_count;
     uint32_t prev_count;
+    // kKsMerge of a tree's first level straight from its inputs (the double-precision kernel
+    // only): merge it joins leaves 2q and 2q + 1 of pack p, it = p 2^(leaf_log - 1) + q, each set
+    // up from its LWE row as pack_l0_kernel does
+    const uint64_t* leaf;
+    uint32_t leaf_log;
     uint64_t corr;
     uint32_t dshift[8];
     uint64_t dmask[8];
