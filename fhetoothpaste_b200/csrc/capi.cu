@@ -101,12 +101,15 @@ struct Tables {
     uint64_t* tw_inv = nullptr;
     uint64_t* psi_pow = nullptr;
     uint64_t n_inv = 0;
+    // transform kernels of this size, [forward]: resident blocks (clusters above N = 4096) once
+    // the kernel's attributes are set, 0 before
+    std::atomic<int> ntt_cap[2] = {};
 };
 
 std::mutex g_tab_mu;
 std::vector<Tables*> g_tables;
 
-tp_status get_tables(int device, int logn, const Tables** out) {
+tp_status get_tables(int device, int logn, Tables** out) {
     std::lock_guard<std::mutex> lk(g_tab_mu);
     for (auto* t : g_tables)
         if (t->device == device && t->logn == logn) {
@@ -209,7 +212,7 @@ struct tp_br_ctx {
     int G = 1;                    // RGSWs per iteration group
     uint64_t groups = 0;          // iteration groups (n, or n/2 for BMMP)
     uint64_t key_words = 0;
-    const Tables* tab = nullptr;
+    Tables* tab = nullptr;
     uint64_t* key = nullptr;      // device layout
     bool key_ready = false;
     unsigned int* err = nullptr;  // device error word
@@ -1095,7 +1098,7 @@ struct tp_ks_ctx {
     uint64_t basis = 0;
     int nkeys = 1;                // packing: logN keys, index 2^j + 1, j = 1..logN
     uint64_t key_words = 0;
-    const Tables* tab = nullptr;
+    Tables* tab = nullptr;
     uint64_t* key = nullptr;
     bool key_ready = false;
     tp::KsKernelParams kp{};
@@ -2216,52 +2219,48 @@ static tp_status ntt_launch(uint32_t ring_dim, uint64_t count, uint64_t* out, co
     int device = 0;
     TP_CUDA(cudaGetDevice(&device));
     const int logn = ilog2(ring_dim);
-    const Tables* tab = nullptr;
+    Tables* tab = nullptr;
     tp_status s = get_tables(device, logn, &tab);
     if (s != TP_OK) return s;
     const void* k = tp::ntt_kernel_lookup(logn, fwd);
     if (!in_stride) in_stride = ring_dim;
     if (!out_stride) out_stride = ring_dim;
+    // one block of N/4 threads per polynomial, 3N words of shared memory; above N = 4096 a
+    // cluster of 2^logs blocks with 5 NL words each (NL = N / 2^logs)
     const int logs = tp::br_cluster_logs(logn);
-    if (logs > 0) {
-        // one polynomial per cluster of 2^logs CTAs of N / 2^(logs+2) threads; shared
-        // memory: 5 NL words (NL = N / 2^logs)
-        const unsigned S = 1u << logs;
-        const size_t smem = 5ull * (ring_dim >> logs) * 8;
-        TP_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const unsigned S = 1u << logs;
+    cudaLaunchAttribute attr[2] = {};
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see pdl_wait
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = S;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(ring_dim >> (logs + 2));
+    cfg.dynamicSmemBytes = (size_t)(logs ? 5 : 3) * (ring_dim >> logs) * 8;
+    cfg.stream = (cudaStream_t)stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = logs ? 2 : 1;
+    int cap = tab->ntt_cap[fwd].load(std::memory_order_acquire);
+    if (cap == 0) {  // once per size, direction and device: these calls cost as much as the launch
+        TP_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes));
         if (S > 8) TP_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr = {};
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = S;
-        attr.val.clusterDim.y = 1;
-        attr.val.clusterDim.z = 1;
-        cfg.gridDim = dim3(S * (unsigned)sm_count(device));
-        cfg.blockDim = dim3(ring_dim >> (logs + 2));
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = (cudaStream_t)stream;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
-        int clusters = 0;
-        TP_CUDA(cudaOccupancyMaxActiveClusters(&clusters, k, &cfg));
-        if (clusters < 1) return fail(TP_ERR_CUDA, "NTT cluster kernel (N=%u): no resident cluster", ring_dim);
-        cfg.gridDim = dim3((unsigned)(std::min<uint64_t>(count, (uint64_t)clusters) << logs));
-        const uint64_t* tw = fwd ? tab->tw_fwd : tab->tw_inv;
-        uint64_t n_inv = tab->n_inv;
-        void* args[] = {&out, &in, &count, &tw, &n_inv, &in_stride, &out_stride};
-        TP_CUDA(cudaLaunchKernelExC(&cfg, k, args));
-        tp::note_launch();
-        return TP_OK;
+        if (logs) {
+            cfg.gridDim = dim3(S * (unsigned)sm_count(device));
+            TP_CUDA(cudaOccupancyMaxActiveClusters(&cap, k, &cfg));
+            if (cap < 1) return fail(TP_ERR_CUDA, "NTT cluster kernel (N=%u): no resident cluster", ring_dim);
+        } else {
+            TP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cap, k, (int)cfg.blockDim.x, cfg.dynamicSmemBytes));
+            cap = std::max(1, cap) * sm_count(device);
+        }
+        tab->ntt_cap[fwd].store(cap, std::memory_order_release);
     }
-    const size_t smem = 3ull * ring_dim * 8;
-    TP_CUDA(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int per_sm = 0;
-    TP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k, ring_dim / 8, smem));
-    const uint64_t grid = std::min<uint64_t>(count, (uint64_t)std::max(1, per_sm) * sm_count(device));
+    cfg.gridDim = dim3((unsigned)(std::min<uint64_t>(count, (uint64_t)cap) << logs));
     const uint64_t* tw = fwd ? tab->tw_fwd : tab->tw_inv;
     uint64_t n_inv = tab->n_inv;
     void* args[] = {&out, &in, &count, &tw, &n_inv, &in_stride, &out_stride};
-    TP_CUDA(cudaLaunchKernel(k, dim3((unsigned)grid), dim3(ring_dim / 8), args, smem, (cudaStream_t)stream));
+    TP_CUDA(cudaLaunchKernelExC(&cfg, k, args));
     tp::note_launch();
     return TP_OK;
 }
@@ -2811,7 +2810,6 @@ extern "C" tp_status tp_pack_batch_noalloc(tp_ks_ctx* c, uint64_t packs, uint64_
                     "packs * len * 2N (%llu packs of %llu words) exceeds the fixed scratch of %llu words (16 MiB); "
                     "use fewer packs per call or tp_pack_batch",
                     (unsigned long long)packs, (unsigned long long)per_pack, (unsigned long long)kPackScratchWords);
-    const uint64_t need = packs * per_pack;
     if (c->device < 0 || c->device >= kMaxDevices) return fail(TP_ERR_PARAM, "device index out of range");
     // The context's key, tile and tables are read under its lock, as in tp_pack_batch:
     // tp_ks_set_tile or tp_ks_upload_key on another thread cannot swap them mid-call.
