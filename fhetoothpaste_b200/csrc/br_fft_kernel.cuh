@@ -24,6 +24,7 @@
 
 #include "br_kernels.cuh"
 #include "fft_block.cuh"
+#include "mbar.cuh"
 
 namespace tp {
 
@@ -93,6 +94,85 @@ __device__ __forceinline__ ulonglong2 rot_pair(Load&& at, uint32_t j, uint32_t s
     const uint32_t q = (idx >> LOGK) & 3u;
     const uint64_t a = (q & 1u) ? v.y : v.x, b = (q & 1u) ? v.x : v.y;
     return make_ulonglong2((q & 2u) ? gl_neg(a) : a, (q == 1u || q == 2u) ? gl_neg(b) : b);
+}
+
+// This thread's 16 points (pairs j = tg + i TG) of one digit of an accumulator half: (v >> sh) &
+// mk - off (off carries 2^52). Signed digits of v itself; unsigned ones of (X^-a - 1) v.
+template <int LOGK, bool SIGNED>
+__device__ __forceinline__ void digit_points(double2 (&x)[16], const ulonglong2* ah, int tg, uint32_t a, uint32_t sh,
+                                             uint32_t mk, double off) {
+    constexpr int TG = Fft<LOGK>::T;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const int j = tg + i * TG;
+        ulonglong2 v = ah[j];
+        if constexpr (!SIGNED) {
+            const ulonglong2 w = rot_pair<LOGK>([&](uint32_t k) { return ah[k]; }, j, a);
+            v = make_ulonglong2(gl_sub(w.x, v.x), gl_sub(w.y, v.y));
+        }
+        x[i] = make_double2(__hiloint2double(0x43300000, (int)((uint32_t)(v.x >> sh) & mk)) - off,
+                            __hiloint2double(0x43300000, (int)((uint32_t)(v.y >> sh) & mk)) - off);
+    }
+}
+// s += x k
+__device__ __forceinline__ void cmac(double2& s, double2 x, double2 k) {
+    s.x = fma(x.x, k.x, s.x);
+    s.y = fma(x.x, k.y, s.y);
+    s.x = fma(-x.y, k.y, s.x);
+    s.y = fma(x.y, k.x, s.y);
+}
+__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
+    return make_double2(fma(a.x, b.x, -(a.y * b.y)), fma(a.x, b.y, a.y * b.x));
+}
+// lo - w hi
+__device__ __forceinline__ double2 csubmul(double2 lo, double2 w, double2 hi) {
+    return make_double2(fma(w.y, hi.y, fma(-w.x, hi.x, lo.x)), fma(-w.y, hi.x, fma(-w.x, hi.y, lo.y)));
+}
+// Rounded limbs (in place of the products in buf) to words G mod p; acc += G (binary) or
+// (X^-a - 1) G (ternary). All T threads; ends with a barrier.
+template <int LOGK, int VARIANT, int L, int T>
+__device__ __forceinline__ void recombine_update(double2* buf, ulonglong2* acc, int t, uint32_t a) {
+    constexpr int n = 1 << LOGK;
+    const ulonglong2* wb = reinterpret_cast<const ulonglong2*>(buf);
+    ulonglong2* gb = reinterpret_cast<ulonglong2*>(buf);
+    constexpr int U = (2 * n + T - 1) / T;
+    ulonglong2 gv[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+        const int u = t + k * T;
+        if ((2 * n) % T == 0 || u < 2 * n) {
+            const int h = u >> LOGK, pos = fft_pos(u & (n - 1));
+            uint64_t cx[L], cy[L];
+#pragma unroll
+            for (int l = 0; l < L; ++l) {
+                const ulonglong2 v = wb[(h * L + l) * n + pos];
+                cx[l] = v.x;
+                cy[l] = v.y;
+            }
+            gv[k] = make_ulonglong2(fft_recombine<L>(cx), fft_recombine<L>(cy));
+            if constexpr (VARIANT == kCggiBinary) {
+                // acc += ExtProd (mux_operator.cpp:151)
+                const ulonglong2 v = acc[u];
+                acc[u] = make_ulonglong2(gl_add(v.x, gv[k].x), gl_add(v.y, gv[k].y));
+            } else {
+                gb[(h * L) * n + pos] = gv[k];
+            }
+        }
+    }
+    __syncthreads();
+    if constexpr (VARIANT == kCggiTernary) {
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+            const int u = t + k * T;
+            if ((2 * n) % T == 0 || u < 2 * n) {
+                const ulonglong2* gh = gb + (u >> LOGK) * (L * n);
+                const ulonglong2 w = rot_pair<LOGK>([&](uint32_t j) { return gh[fft_pos((int)j)]; }, u & (n - 1), a);
+                const ulonglong2 v = acc[u];
+                acc[u] = make_ulonglong2(gl_add(v.x, gl_sub(w.x, gv[k].x)), gl_add(v.y, gl_sub(w.y, gv[k].y)));
+            }
+        }
+        __syncthreads();
+    }
 }
 
 template <int LOGN, int VARIANT, int DL, int L>
@@ -186,17 +266,7 @@ br_fft_kernel(const __grid_constant__ BrFftParams prm) {
                 const double off = 4503599627370496.0 + (SIGNED ? (double)prm.ddelta[d] : 0.0);
                 const ulonglong2* ah = acc + h * n;
                 double2 x[16];
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const int j = tg + i * TG;
-                    ulonglong2 v = ah[j];
-                    if constexpr (!SIGNED) {
-                        const ulonglong2 w = rot_pair<LOGK>([&](uint32_t k) { return ah[k]; }, j, a);
-                        v = make_ulonglong2(gl_sub(w.x, v.x), gl_sub(w.y, v.y));
-                    }
-                    x[i] = make_double2(__hiloint2double(0x43300000, (int)((uint32_t)(v.x >> sh) & mk)) - off,
-                                        __hiloint2double(0x43300000, (int)((uint32_t)(v.y >> sh) & mk)) - off);
-                }
+                digit_points<LOGK, SIGNED>(x, ah, tg, a, sh, mk, off);
                 F::head(x, prm.head);
                 double2* pb = buf + grp * n;
 #pragma unroll
@@ -242,25 +312,14 @@ br_fft_kernel(const __grid_constant__ BrFftParams prm) {
                         for (int r = 0; r < BR; ++r) {
                             const double2 x = buf[(q * BR % R + r) * n + pos];
 #pragma unroll
-                            for (int c = 0; c < C; ++c) {
-                                const double2 k = kv[q & 1][r][c];
-                                s[c].x = fma(x.x, k.x, s[c].x);
-                                s[c].y = fma(x.x, k.y, s[c].y);
-                                s[c].x = fma(-x.y, k.y, s[c].x);
-                                s[c].y = fma(x.y, k.x, s[c].y);
-                            }
+                            for (int c = 0; c < C; ++c) cmac(s[c], x, kv[q & 1][r][c]);
                         }
                         if ((q + 1) * BR % R != 0) continue;
                         double2 v[2] = {s[0], s[1]};
                         if constexpr (VARIANT == kCggiTernary) {
-                            const double2 f = mono_s[m];
-                            const double2 w = make_double2(fma(wb.x, f.x, -(wb.y * f.y)), fma(wb.x, f.y, wb.y * f.x));
+                            const double2 w = cmul(wb, mono_s[m]);
 #pragma unroll
-                            for (int h = 0; h < 2; ++h) {
-                                const double2 e = s[C - 2 + h];
-                                v[h] = make_double2(fma(w.y, e.y, fma(-w.x, e.x, s[h].x)),
-                                                    fma(-w.y, e.x, fma(-w.x, e.y, s[h].y)));
-                            }
+                            for (int h = 0; h < 2; ++h) v[h] = csubmul(s[h], w, s[C - 2 + h]);
                         }
 #pragma unroll
                         for (int h = 0; h < 2; ++h) {
@@ -300,48 +359,7 @@ br_fft_kernel(const __grid_constant__ BrFftParams prm) {
             __syncthreads();
 
             // ---- limbs to words mod p; accumulator ----
-            const ulonglong2* wb = reinterpret_cast<const ulonglong2*>(buf);
-            ulonglong2* gb = reinterpret_cast<ulonglong2*>(buf);
-            constexpr int U = (2 * n + T - 1) / T;
-            ulonglong2 gv[U];
-#pragma unroll
-            for (int k = 0; k < U; ++k) {
-                const int u = t + k * T;
-                if ((2 * n) % T == 0 || u < 2 * n) {
-                    const int h = u >> LOGK, pos = fft_pos(u & (n - 1));
-                    uint64_t cx[L], cy[L];
-#pragma unroll
-                    for (int l = 0; l < L; ++l) {
-                        const ulonglong2 v = wb[(h * L + l) * n + pos];
-                        cx[l] = v.x;
-                        cy[l] = v.y;
-                    }
-                    gv[k] = make_ulonglong2(fft_recombine<L>(cx), fft_recombine<L>(cy));
-                    if constexpr (VARIANT == kCggiBinary) {
-                        // acc += ExtProd (mux_operator.cpp:151)
-                        const ulonglong2 v = acc[u];
-                        acc[u] = make_ulonglong2(gl_add(v.x, gv[k].x), gl_add(v.y, gv[k].y));
-                    } else {
-                        gb[(h * L) * n + pos] = gv[k];
-                    }
-                }
-            }
-            __syncthreads();
-            if constexpr (VARIANT == kCggiTernary) {
-#pragma unroll
-                for (int k = 0; k < U; ++k) {
-                    const int u = t + k * T;
-                    if ((2 * n) % T == 0 || u < 2 * n) {
-                        const ulonglong2* gh = gb + (u >> LOGK) * (L * n);
-                        const ulonglong2 w = rot_pair<LOGK>([&](uint32_t j) { return gh[fft_pos((int)j)]; },
-                                                            u & (n - 1), a);
-                        const ulonglong2 v = acc[u];
-                        acc[u] = make_ulonglong2(gl_add(v.x, gl_sub(w.x, gv[k].x)),
-                                                 gl_add(v.y, gl_sub(w.y, gv[k].y)));
-                    }
-                }
-                __syncthreads();
-            }
+            recombine_update<LOGK, VARIANT, L, T>(buf, acc, t, a);
         }
 
         uint64_t* res = prm.out + b * (2ull * N);
@@ -353,6 +371,279 @@ br_fft_kernel(const __grid_constant__ BrFftParams prm) {
             r[n] = v.y;
         }
     }
+}
+
+// ---------------------------------------------------------------------------
+// Two rotations on a cluster of two blocks, for throughput: block c rotates ciphertext c of the
+// pair and multiplies the slots of half c of both, so that each block reads half the key (the
+// key stream from L2 takes 45% of an iteration of the one-block form). Per iteration the blocks
+// exchange half of their digits' slots and half of their products through distributed shared
+// memory, 48 KB each at ternary N = 2048, with two cluster barriers: the digits of the other
+// block's half go to its receive area, free since the barrier after the last products; products
+// go where their block's digits of that half have been sent away from. Digits travel as bulk
+// copies (the transform's own stores, a 128-byte line apart from lane to lane, took 4.7k clocks for 48 KB).
+// Ternary N = 2048, n = 630, 4096 rotations: 317 -> 298 ms over the one-block form.
+// ---------------------------------------------------------------------------
+__host__ __device__ constexpr size_t br_fft_pair_base_bytes(int logn, int dl, int limbs) {
+    const size_t k = (size_t)1 << (logn - 1);
+    return ((2 * (dl > limbs ? dl : limbs)) * k + dl * k + 2 * k + 9) * 16;  // buffers, receive area, accumulator, factors, barrier
+}
+__host__ __device__ constexpr size_t br_fft_pair_limit(int logn) { return logn >= 11 ? 227u * 1024u : 113u * 1024u; }
+__host__ __device__ constexpr bool br_fft_pair_tabs(int logn, int dl, int limbs) {  // pass tables in shared memory
+    return br_fft_pair_base_bytes(logn, dl, limbs) + 2 * fft_table_len(logn - 1) * 16 + 4096 <= br_fft_pair_limit(logn);
+}
+// Eighths of the slots whose own products go to a spare area (see br_fft_spare).
+__host__ __device__ constexpr int br_fft_pair_spare(int logn, int dl, int limbs) {
+    if (!br_fft_pair_tabs(logn, dl, limbs)) return 0;
+    const size_t room = br_fft_pair_limit(logn) - 4096 - br_fft_pair_base_bytes(logn, dl, limbs) -
+                        2 * fft_table_len(logn - 1) * 16;
+    const int m = (int)(room / ((size_t)2 * limbs * (1 << (logn - 4)) * 16));
+    return m > 4 ? 4 : m;
+}
+__host__ __device__ constexpr size_t br_fft_pair_smem(int logn, int dl, int limbs, uint32_t n) {
+    return br_fft_pair_base_bytes(logn, dl, limbs) +
+           (br_fft_pair_tabs(logn, dl, limbs) ? 2 * fft_table_len(logn - 1) * 16 : 0) +
+           (size_t)2 * limbs * br_fft_pair_spare(logn, dl, limbs) * (1 << (logn - 4)) * 16 + ((2 * (size_t)(n + 1) + 7) / 8) * 16;
+}
+
+template <int LOGN, int VARIANT, int DL, int L>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(br_fft_threads(LOGN, DL, L), LOGN <= 10 ? 2 : 1)
+br_fft_pair_kernel(const __grid_constant__ BrFftParams prm) {
+    static_assert(VARIANT == kCggiBinary || VARIANT == kCggiTernary, "CGGI only");
+    constexpr int LOGK = LOGN - 1;
+    using F = Fft<LOGK>;
+    constexpr int N = 1 << LOGN, n = F::n, TG = F::T;
+    constexpr int G = br_rgsw_per_group(VARIANT);
+    constexpr int C = 2 * G, R = 2 * DL;
+    constexpr int T = br_fft_threads(LOGN, DL, L);
+    constexpr int P = 2 * (DL > L ? DL : L);
+    constexpr int LANES = n / 8, M = 4;        // slots of this block per thread
+    constexpr int SPARE = br_fft_pair_spare(LOGN, DL, L);
+    constexpr bool TABS = br_fft_pair_tabs(LOGN, DL, L);
+    constexpr uint32_t MASK2N = 2u * N - 1u;
+    constexpr bool SIGNED = VARIANT != kCggiBinary;
+
+    extern __shared__ __align__(16) uint64_t smem[];
+    double2* buf = reinterpret_cast<double2*>(smem);                   // P n
+    double2* recv = buf + P * n;                                       // R n/2: the other rotation's digits
+    ulonglong2* acc = reinterpret_cast<ulonglong2*>(recv + R * (n / 2));  // 2 n: plus corr (signed)
+    double2* mono_s = reinterpret_cast<double2*>(acc + 2 * n);         // [rotation][m < 4]
+    uint64_t* bar = reinterpret_cast<uint64_t*>(mono_s + 8);           // the other block's digits have come
+    double2* spare = mono_s + 9;
+    double2* tabs = spare + 2 * L * SPARE * LANES;
+    uint16_t* lwe_s = reinterpret_cast<uint16_t*>(tabs + (TABS ? 2 * fft_table_len(LOGK) : 0));  // [rotation][n + 1]
+
+    auto cluster = cooperative_groups::this_cluster();
+    const int c = (int)cluster.block_rank();
+    const int t = threadIdx.x;
+    const int grp = t / TG, tg = t % TG;
+    const int limb = t / LANES, lane = t % LANES;
+    const double2* tab_f = prm.tab_fwd;
+    const double2* tab_i = prm.tab_inv;
+    if constexpr (TABS) {
+        for (int i = t; i < fft_table_len(LOGK); i += T) {
+            tabs[i] = prm.tab_fwd[i];
+            tabs[fft_table_len(LOGK) + i] = prm.tab_inv[i];
+        }
+        tab_f = tabs;
+        tab_i = tabs + fft_table_len(LOGK);
+    }
+    uint32_t phase = 0;
+    bool ok = true;  // a wait for the other block's digits ran out
+    if (t == 0) {
+        mbar_init(bar, 1);
+        mbar_init_fence();
+    }
+    double2* buf_peer = cluster.map_shared_rank(buf, (unsigned)(c ^ 1));
+    cluster.sync();  // both blocks running, their barriers set, before remote stores
+
+    for (uint64_t b0 = blockIdx.x & ~1ull; b0 < prm.batch; b0 += gridDim.x) {
+        const uint64_t b = b0 + c;
+        __syncthreads();
+        bool bad = false;
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {  // both rotations' words; a missing one is all zeros and written nowhere
+            const uint64_t* lwe = prm.lwes + (b0 + r) * prm.lwe_stride;
+            const bool have = b0 + r < prm.batch;
+            for (uint32_t i = t; i <= prm.n; i += T) {
+                const uint64_t v = have ? lwe[i] : 0;
+                bad |= v > MASK2N;
+                lwe_s[r * (prm.n + 1) + i] = (uint16_t)(v & MASK2N);
+            }
+        }
+        if (bad && c == 0) atomicOr(prm.err, 1u);
+        __syncthreads();
+        {
+            const uint64_t* ain = prm.accs + b * prm.acc_stride;
+            const uint32_t s = (2u * N - lwe_s[c * (prm.n + 1) + prm.n]) & MASK2N;
+            for (int u = t; u < 2 * n; u += T) {
+                ulonglong2 v = make_ulonglong2(0, 0);
+                if (b < prm.batch) {
+                    const uint64_t* a = ain + (u >> LOGK) * N;
+                    v = rot_pair<LOGK>([&](uint32_t j) { return make_ulonglong2(gl_canon(a[j]), gl_canon(a[j + n])); },
+                                       u & (n - 1), s);
+                }
+                if constexpr (SIGNED) v = make_ulonglong2(gl_add(v.x, prm.corr), gl_add(v.y, prm.corr));
+                acc[u] = v;
+            }
+        }
+        __syncthreads();
+
+        auto prefetch = [&](uint32_t it) {  // this block's share of an iteration's key, as in the one-block form
+            constexpr uint32_t bytes = (uint32_t)L * 8 * R * C * LANES * 16;
+            const uint32_t share = ((bytes + gridDim.x - 1) / gridDim.x + 127u) & ~127u;
+            const uint32_t off = blockIdx.x * share;
+            if (it < prm.n && off < bytes) l2_prefetch(reinterpret_cast<const char*>(prm.key) + (uint64_t)it * bytes + off,
+                                                       min(share, bytes - off));
+        };
+        if (t == 0) {
+            prefetch(0);
+            prefetch(1);
+        }
+#pragma unroll 1
+        for (uint32_t it = 0; it < prm.n; ++it) {
+            if (t == 0) prefetch(it + 2);
+            const uint32_t ar[2] = {lwe_s[it], lwe_s[prm.n + 1 + it]};
+            if (ar[0] == 0 && ar[1] == 0) continue;  // one rotation alone at 0 adds (X^0 - 1) G = 0
+            const uint32_t a = c ? ar[1] : ar[0];
+            if (t == 0) mbar_expect(bar, R * (n / 2) * 16);
+
+            if constexpr (VARIANT == kCggiTernary) {
+                // factors of this block's m (see br_fft_kernel), both rotations
+                if (t < 8)
+                    mono_s[t] = __ldg(prm.roots + ((4u * (t < 4 ? ar[0] : ar[1]) *
+                                                    (__brev((uint32_t)(c * M + (t & 3))) >> 29)) & MASK2N));
+            }
+
+            // ---- digits and forward transforms; the other half's slots to the other block ----
+            if (grp < R) {
+                const int h = grp / DL, d = grp - h * DL;
+                double2 x[16];
+                digit_points<LOGK, SIGNED>(x, acc + h * n, tg, a, prm.dshift[d], (uint32_t)prm.dmask[d],
+                                           4503599627370496.0 + (SIGNED ? (double)prm.ddelta[d] : 0.0));
+                F::head(x, prm.head);
+                double2* pb = buf + grp * n;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) pb[fft_pos(tg + i * TG)] = x[i];
+                F::group_sync(grp);
+                F::tail(pb, tab_f, tg, grp, [&](int e, double2 v) { pb[fft_pos(e)] = v; });
+                bulk_fence();
+                F::group_sync(grp);
+                if (tg == 0)
+                    bulk_to_block(recv + grp * (n / 2), pb + (c ^ 1) * (n / 2), n / 2 * 16, bar, (uint32_t)(c ^ 1));
+            }
+
+            // ---- slot-wise products, slots lane + (4 c + m) LANES of both rotations, one limb ----
+            double2 o[2][M - SPARE + 1];
+            {
+                constexpr int BR = 2, NB = M * R / BR;
+                const double2* kp = prm.key + ((((uint64_t)it * L + limb) * 8 + c * M) * (R * C)) * LANES + lane;
+                double2 kv[2][BR][C];
+                auto load = [&](int q, double2 (&k)[BR][C]) {
+#pragma unroll
+                    for (int r = 0; r < BR; ++r)
+#pragma unroll
+                        for (int cc = 0; cc < C; ++cc) k[r][cc] = key_ld(kp + ((q * BR + r) * C + cc) * LANES);
+                };
+                double2 wb[2];
+                const bool on = limb < L;
+                if (on) {
+                    load(0, kv[0]);
+                    if constexpr (VARIANT == kCggiTernary) {
+                        const uint32_t e = 1u + 32u * (__brev((uint32_t)lane) >> (35 - LOGK));
+                        wb[0] = __ldg(prm.roots + ((ar[0] * e) & MASK2N));
+                        wb[1] = __ldg(prm.roots + ((ar[1] * e) & MASK2N));
+                    }
+                }
+                __syncthreads();
+                ok = ok && mbar_wait(bar, phase);
+                phase ^= 1;
+                if (on) {
+                    double2 s[2][C];
+#pragma unroll
+                    for (int q = 0; q < NB; ++q) {
+                        const int m = q * BR / R, pos = fft_pos(lane + (c * M + m) * LANES),
+                                  rpos = fft_pos(lane + m * LANES);
+                        if (q + 1 < NB) load(q + 1, kv[(q + 1) & 1]);
+                        if (q * BR % R == 0) {
+#pragma unroll
+                            for (int cc = 0; cc < C; ++cc) s[0][cc] = s[1][cc] = make_double2(0.0, 0.0);
+                        }
+#pragma unroll
+                        for (int r = 0; r < BR; ++r) {
+                            const double2 x0 = buf[(q * BR % R + r) * n + pos];
+                            const double2 x1 = recv[(q * BR % R + r) * (n / 2) + rpos];
+#pragma unroll
+                            for (int cc = 0; cc < C; ++cc) {
+                                cmac(s[0][cc], x0, kv[q & 1][r][cc]);
+                                cmac(s[1][cc], x1, kv[q & 1][r][cc]);
+                            }
+                        }
+                        if ((q + 1) * BR % R != 0) continue;
+                        if constexpr (VARIANT == kCggiTernary) {
+                            // rotation of s[0] is c, of s[1] the other
+                            const double2 w0 = cmul(c ? wb[1] : wb[0], mono_s[c * 4 + m]);
+                            const double2 w1 = cmul(c ? wb[0] : wb[1], mono_s[(c ^ 1) * 4 + m]);
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                s[0][h] = csubmul(s[0][h], w0, s[0][C - 2 + h]);
+                                s[1][h] = csubmul(s[1][h], w1, s[1][C - 2 + h]);
+                            }
+                        }
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            buf_peer[(h * L + limb) * n + pos] = s[1][h];
+                            if (m < SPARE) spare[(h * L + limb) * (SPARE * LANES) + rpos] = s[0][h];
+                            else o[h][m - SPARE] = s[0][h];
+                        }
+                    }
+                }
+                cluster.sync();  // both blocks' reads of the digits done, products of the other half here
+                if (on) {
+#pragma unroll
+                    for (int m = SPARE; m < M; ++m)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+                            buf[(h * L + limb) * n + fft_pos(lane + (c * M + m) * LANES)] = o[h][m - SPARE];
+                }
+                __syncthreads();
+            }
+
+            // ---- backward transforms, rounded coefficients back in place ----
+            if (grp < 2 * L) {
+                double2* pb = buf + grp * n;
+                F::itail(pb, tab_i, tg, grp, [&](int e) {
+                    const int el = e - c * (n / 2);
+                    return el >= 0 && el < SPARE * LANES ? spare + grp * (SPARE * LANES) + fft_pos(el) : pb + fft_pos(e);
+                });
+                F::group_sync(grp);
+                double2 x[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) x[i] = pb[fft_pos(tg + i * TG)];
+                F::ihead(x, prm.head);
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    *reinterpret_cast<ulonglong2*>(pb + fft_pos(tg + i * TG)) =
+                        make_ulonglong2(fft_round(x[i].x), fft_round(x[i].y));
+            }
+            __syncthreads();
+
+            recombine_update<LOGK, VARIANT, L, T>(buf, acc, t, a);
+        }
+
+        if (b < prm.batch) {
+            uint64_t* res = prm.out + b * (2ull * N);
+            for (int u = t; u < 2 * n; u += T) {
+                ulonglong2 v = acc[u];
+                if constexpr (SIGNED) v = make_ulonglong2(gl_sub(v.x, prm.corr), gl_sub(v.y, prm.corr));
+                uint64_t* r = res + (u >> LOGK) * N + (u & (n - 1));
+                r[0] = v.x;
+                r[n] = v.y;
+            }
+        }
+    }
+    if (!ok) atomicOr(prm.err, 2u);
+    cluster.sync();  // no block leaves while the other may still store to it
 }
 
 // ---------------------------------------------------------------------------
@@ -371,11 +662,11 @@ __host__ __device__ constexpr int br_fft_cluster_polys(int dl, int limbs, int cs
 }
 __host__ __device__ constexpr int br_fft_cluster_threads(int logn, int limbs) { return (1 << (logn - 4)) * limbs; }
 // Forward and backward buffers (PP polynomials each), digit slots (2l n/CS), limb and word
-// areas (2L n/CS, 2n), accumulator (2n), pass tables, monomial factors, LWE words.
+// areas (2L n/CS, 2n), accumulator (2n), pass tables, monomial factors, barrier, LWE words.
 __host__ __device__ constexpr size_t br_fft_cluster_smem(int logn, int dl, int limbs, int cs, uint32_t n) {
     const size_t k = (size_t)1 << (logn - 1);
     return (2 * br_fft_cluster_polys(dl, limbs, cs) * k + (2 * dl + 2 * limbs) * (k / cs) + 4 * k +
-            2 * fft_table_len(logn - 1) + 8) * 16 + (((size_t)n + 4) / 4) * 16;
+            2 * fft_table_len(logn - 1) + 9) * 16 + (((size_t)n + 4) / 4) * 16;
 }
 
 template <int LOGN, int VARIANT, int DL, int L, int CS>
@@ -403,7 +694,8 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
     double2* tab_f = reinterpret_cast<double2*>(acc + 2 * n);
     double2* tab_i = tab_f + fft_table_len(LOGK);
     double2* mono_s = tab_i + fft_table_len(LOGK);
-    uint32_t* lwe_s = reinterpret_cast<uint32_t*>(mono_s + 8);
+    uint64_t* bar = reinterpret_cast<uint64_t*>(mono_s + 8);           // every block's digits have come
+    uint32_t* lwe_s = reinterpret_cast<uint32_t*>(mono_s + 9);
 
     auto cluster = cooperative_groups::this_cluster();
     const int c = (int)cluster.block_rank();
@@ -417,7 +709,13 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
     // blocks whose forward polynomials are digits of half h
     auto first_of = [](int h) { return h * DL / PP; };
     auto last_of = [](int h) { return (h * DL + DL - 1) / PP; };
-    cluster.sync();  // every block of the cluster running before remote stores
+    uint32_t phase = 0;
+    bool ok = true;  // a wait for the blocks' digits ran out
+    if (t == 0) {
+        mbar_init(bar, 1);
+        mbar_init_fence();
+    }
+    cluster.sync();  // every block of the cluster running, its barrier set, before remote stores
 
     const uint64_t clusters = gridDim.x / CS;
     for (uint64_t b = blockIdx.x / CS; b < prm.batch; b += clusters) {
@@ -457,6 +755,7 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
             prefetch(it + 2);
             const uint32_t a = lwe_s[it];
             if (a == 0) continue;
+            if (t == 0) mbar_expect(bar, R * NS * 16);
 
             // ---- digits and forward transforms, slots to their blocks ----
             const int p = c * PP + grp;
@@ -467,25 +766,16 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
                 const double off = 4503599627370496.0 + (SIGNED ? (double)prm.ddelta[d] : 0.0);
                 const ulonglong2* ah = acc + h * n;
                 double2 x[16];
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const int j = tg + i * TG;
-                    ulonglong2 v = ah[j];
-                    if constexpr (!SIGNED) {
-                        const ulonglong2 w = rot_pair<LOGK>([&](uint32_t k) { return ah[k]; }, j, a);
-                        v = make_ulonglong2(gl_sub(w.x, v.x), gl_sub(w.y, v.y));
-                    }
-                    x[i] = make_double2(__hiloint2double(0x43300000, (int)((uint32_t)(v.x >> sh) & mk)) - off,
-                                        __hiloint2double(0x43300000, (int)((uint32_t)(v.y >> sh) & mk)) - off);
-                }
+                digit_points<LOGK, SIGNED>(x, ah, tg, a, sh, mk, off);
                 F::head(x, prm.head);
                 double2* pb = work + grp * n;
 #pragma unroll
                 for (int i = 0; i < 16; ++i) pb[fft_pos(tg + i * TG)] = x[i];
                 F::group_sync(grp);
-                F::tail(pb, tab_f, tg, grp, [&](int e, double2 v) {
-                    cluster.map_shared_rank(dig, (unsigned)(e / NS))[p * NS + fft_pos(e % NS)] = v;
-                });
+                F::tail(pb, tab_f, tg, grp, [&](int e, double2 v) { pb[fft_pos(e)] = v; });
+                bulk_fence();
+                F::group_sync(grp);
+                if (tg < CS) bulk_to_block(dig + p * NS, pb + tg * NS, NS * 16, bar, (uint32_t)tg);
             } else if (VARIANT == kCggiTernary && t >= T - M) {
                 const int mm = t - (T - M);
                 mono_s[mm] = __ldg(prm.roots + ((4u * a * (__brev((uint32_t)(c * M + mm)) >> 29)) & MASK2N));
@@ -505,11 +795,13 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
             double2 wb = make_double2(1.0, 0.0);
             if constexpr (VARIANT == kCggiTernary)
                 wb = __ldg(prm.roots + ((a * (1u + 32u * (__brev((uint32_t)lane) >> (35 - LOGK)))) & MASK2N));
-            cluster.sync();
+            __syncthreads();
+            ok = ok && mbar_wait(bar, phase);
+            phase ^= 1;
             double2 s[C];
 #pragma unroll
             for (int q = 0; q < NB; ++q) {
-                const int mm = q * BR / R, pos = fft_pos(lane + mm * LANES);
+                const int mm = q * BR / R, pos = fft_pos(c * NS + lane + mm * LANES) - c * NS;
                 if (q + 1 < NB) load(q + 1, kv[(q + 1) & 1]);
                 if (q * BR % R == 0) {
 #pragma unroll
@@ -519,25 +811,14 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
                 for (int r = 0; r < BR; ++r) {
                     const double2 x = dig[(q * BR % R + r) * NS + pos];
 #pragma unroll
-                    for (int cc = 0; cc < C; ++cc) {
-                        const double2 k = kv[q & 1][r][cc];
-                        s[cc].x = fma(x.x, k.x, s[cc].x);
-                        s[cc].y = fma(x.x, k.y, s[cc].y);
-                        s[cc].x = fma(-x.y, k.y, s[cc].x);
-                        s[cc].y = fma(x.y, k.x, s[cc].y);
-                    }
+                    for (int cc = 0; cc < C; ++cc) cmac(s[cc], x, kv[q & 1][r][cc]);
                 }
                 if ((q + 1) * BR % R != 0) continue;
                 double2 v[2] = {s[0], s[1]};
                 if constexpr (VARIANT == kCggiTernary) {
-                    const double2 f = mono_s[mm];
-                    const double2 w = make_double2(fma(wb.x, f.x, -(wb.y * f.y)), fma(wb.x, f.y, wb.y * f.x));
+                    const double2 w = cmul(wb, mono_s[mm]);
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const double2 e = s[C - 2 + h];
-                        v[h] = make_double2(fma(w.y, e.y, fma(-w.x, e.x, s[h].x)),
-                                            fma(-w.y, e.x, fma(-w.x, e.y, s[h].y)));
-                    }
+                    for (int h = 0; h < 2; ++h) v[h] = csubmul(s[h], w, s[C - 2 + h]);
                 }
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
@@ -611,6 +892,7 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
             }
         }
     }
+    if (!ok) atomicOr(prm.err, 2u);
 }
 
 }  // namespace tp

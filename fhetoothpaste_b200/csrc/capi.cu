@@ -249,7 +249,7 @@ struct tp_br_ctx {
         const void* k = nullptr;
         int cap = 0;                    // resident clusters (0: unavailable)
         size_t smem = 0;
-    } fftc[3];
+    } fftc[3], fftp;                    // fftp: two rotations on a cluster of two blocks
     const tp::FftTables* fft_tab = nullptr;
     double2* fft_key = nullptr;
     bool fft_ready = false;       // the key is resident and exact in this form
@@ -369,6 +369,21 @@ static void br_setup_fft(tp_br_ctx* c) {
         c->fft_kernel = k;
         c->fft_smem = smem;
         c->fft_cap = per_sm * sm_count(c->device);
+        {
+            auto& f = c->fftp;
+            const void* kp = tp::br_fft_pair_ptr(c->logn, c->prm.variant, c->prm.digits, limbs);
+            f.smem = tp::br_fft_pair_smem(c->logn, (int)c->prm.digits, limbs, c->prm.lwe_dim);
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(2 * (unsigned)sm_count(c->device));
+            cfg.blockDim = dim3(tp::br_fft_threads(c->logn, (int)c->prm.digits, limbs));
+            cfg.dynamicSmemBytes = f.smem;
+            e = kp && f.smem <= 227u * 1024u
+                    ? cudaFuncSetAttribute(kp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem)
+                    : cudaErrorInvalidValue;
+            if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&f.cap, kp, &cfg);
+            if (e == cudaSuccess && f.cap > 0) f.k = kp;
+            else if (kp) cudaGetLastError();
+        }
         for (int i = 0; i < 3; ++i) {
             auto& f = c->fftc[i];
             const void* kc = tp::br_fft_cluster_ptr(c->logn, c->prm.variant, c->prm.digits, limbs, 2 << i);
@@ -386,26 +401,30 @@ static void br_setup_fft(tp_br_ctx* c) {
 }
 
 // The form of a launch of `batch` rotations whose context left the choice open: clusters of
-// 2^(i + 1) blocks per rotation in double precision (i = 0 .. 2), one block in double
-// precision (kFftOneBlock), or the modular kernels (kModular, kModularPair: two blocks per
-// rotation). Milliseconds at n = 60 (clusters of 8 / 4 / 2, one block, modular, modular pair),
-// one wave each; 15, 30, 74 clusters are resident:
-//   ternary N = 2048, l = 3:       0.48 / 0.62 / -    1.09  1.53  1.09
-//   binary N = 2048, l = 4:        0.54 / 0.65 / -    1.28  1.72  1.04
-//   ternary N = 2048, l = 4 (2^16) 0.59 / 0.84 / -    2.07  2.06  1.31
-//   binary N = 1024, l = 4:        0.40 / 0.48 / 0.57 0.63  0.98  -
-//   ternary N = 1024, l = 4 (2^16) 0.37 / 0.49 / 0.68 1.46  1.24  -
-// So the widest cluster that takes the batch in one wave, then (N = 2048) the modular pair in
-// its one wave, then one block. Where a block reads 64 or more key polynomials an iteration
-// (ternary, four digits, four limbs) its key stream leaves one block no faster than modular.
-enum { kFftOneBlock = 3, kModularPair = 4, kModular = 5 };
+// 2^(i + 1) blocks per rotation in double precision (i = 0 .. 2), one block (kFftOneBlock) or two
+// rotations on two blocks (kFftPair) in double precision, or the modular kernels (kModular,
+// kModularPair: two blocks per rotation). Milliseconds at n = 60, one wave each (15, 30, 74
+// clusters, 148 rotations) and 600 rotations:
+//                                  clusters 8 / 4 / 2    one block   pair        modular, pair
+//   ternary N = 2048, l = 3        0.43 / 0.56 / -       1.10 5.66   1.04 5.19   1.53  1.09
+//   binary N = 2048, l = 4         0.49 / 0.60 / -       1.32 6.58   1.22 5.99   1.72  1.04
+//   binary N = 2048, l = 3 (2^12)  0.44 / 0.54 / -       0.86 4.27   0.91 4.42   1.40  -
+//   ternary N = 2048, l = 4 (2^16) 0.49 / 0.76 / -       2.08 11.4   1.46 7.65   2.06  1.31
+//   binary N = 1024, l = 4         0.37 / 0.43 / 0.57    0.63 2.65   0.66 2.54   0.98  -
+//   ternary N = 1024, l = 4 (2^16) 0.36 / 0.43 / 0.68    1.56 5.54   1.01 3.60   1.24  -
+// So: the widest cluster that takes the batch in one wave; then, at N = 2048, the modular pair in
+// its one wave; then one block, or the pair where the key polynomials read per slot and iteration
+// (2 G rows limbs) reach 64 and halving them pays for the exchanges (at N = 1024, where two
+// blocks share an SM, from the second block per SM on, or from 128).
+enum { kFftOneBlock = 3, kFftPair = 4, kModularPair = 5, kModular = 6 };
 static int br_form(const tp_br_ctx* c, uint64_t batch) {
     if (!c->fft_ready || !c->fft_on) return kModular;
     for (int i = 2; i >= 0; --i)
         if (batch <= (uint64_t)c->fftc[i].cap) return i;
-    const bool wide = c->G * 2 * (int)c->prm.digits * c->fft_limbs >= 64;
-    if ((c->logn >= 11 || wide) && c->loge == 2 && batch <= (uint64_t)c->pair_cap) return kModularPair;
-    return wide ? kModular : kFftOneBlock;
+    if (c->logn >= 11 && c->loge == 2 && batch <= (uint64_t)c->pair_cap) return kModularPair;
+    const int polys = 2 * c->G * 2 * (int)c->prm.digits * c->fft_limbs;
+    const bool full = c->logn >= 11 || batch > (uint64_t)c->fft_cap / 2;
+    return c->fftp.k && (polys >= 128 || (polys >= 64 && full)) ? kFftPair : kFftOneBlock;
 }
 
 extern "C" {
@@ -894,6 +913,7 @@ tp_status tp_br_check(tp_br_ctx* c, void* stream) {
     unsigned int flags = 0;
     TP_CUDA(cudaMemcpy(&flags, c->err, sizeof flags, cudaMemcpyDeviceToHost));
     TP_CUDA(cudaMemset(c->err, 0, sizeof flags));
+    if (flags & 2u) return fail(TP_ERR_TIMEOUT, "a wait between the blocks of a rotation ran out; its results are not valid");
     if (flags & 1u) return fail(TP_ERR_PARAM, "an LWE word was outside [0, 2N); it was reduced mod 2N");
     return TP_OK;
 }
@@ -2881,7 +2901,8 @@ int br_cluster_ctas(const tp_br_ctx* c) { return c ? 1 << c->logs : 1; }
 
 uint64_t br_fft_blocks(const tp_br_ctx* c, uint64_t batch) {
     const int i = c ? br_form(c, batch) : kModular;
-    if (i > kFftOneBlock) return 0;
+    if (i > kFftPair) return 0;
+    if (i == kFftPair) return 2 * std::min<uint64_t>((batch + 1) / 2, c->fftp.cap);
     return i < kFftOneBlock ? batch << (i + 1) : std::min<uint64_t>(batch, c->fft_cap);
 }
 
@@ -2904,7 +2925,7 @@ tp_status br_batch_launch(tp_br_ctx* c, uint64_t batch, uint64_t* results, const
     if (((uintptr_t)results & 15) || ((uintptr_t)accs & 7) || ((uintptr_t)lwes & 7))
         return fail(TP_ERR_PARAM, "results must be 16-byte aligned, lwes/accs 8-byte aligned");
     const int form = br_form(c, batch);
-    if (form <= kFftOneBlock) {
+    if (form <= kFftPair) {
         TP_CUDA(cudaSetDevice(c->device));
         tp::BrFftParams fp{};
         fp.key = c->fft_key;
@@ -2930,6 +2951,10 @@ tp_status br_batch_launch(tp_br_ctx* c, uint64_t batch, uint64_t* results, const
             const cudaLaunchConfig_t cfg =
                 br_fftc_config(c, i, (unsigned)std::min<uint64_t>(batch, c->fftc[i].cap), (cudaStream_t)stream, &attr);
             TP_CUDA(cudaLaunchKernelExC(&cfg, c->fftc[i].k, fargs));
+        } else if (form == kFftPair) {
+            TP_CUDA(cudaLaunchKernel(c->fftp.k, dim3(2 * (unsigned)std::min<uint64_t>((batch + 1) / 2, c->fftp.cap)),
+                                     dim3(tp::br_fft_threads(c->logn, (int)c->prm.digits, c->fft_limbs)), fargs,
+                                     c->fftp.smem, (cudaStream_t)stream));
         } else {
             TP_CUDA(cudaLaunchKernel(c->fft_kernel, dim3((unsigned)std::min<uint64_t>(batch, c->fft_cap)),
                                      dim3(tp::br_fft_threads(c->logn, (int)c->prm.digits, c->fft_limbs)), fargs,

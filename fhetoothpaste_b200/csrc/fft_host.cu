@@ -118,6 +118,19 @@ __global__ void __launch_bounds__(256) fft_key_kernel(double2* __restrict__ dst,
     }
 }
 
+template <int LOGN, int VARIANT>
+const void* pick_pair(uint32_t digits, int limbs) {
+    switch (digits * 10 + limbs) {
+        case 23: return (const void*)br_fft_pair_kernel<LOGN, VARIANT, 2, 3>;
+        case 24: return (const void*)br_fft_pair_kernel<LOGN, VARIANT, 2, 4>;
+        case 33: return (const void*)br_fft_pair_kernel<LOGN, VARIANT, 3, 3>;
+        case 34: return (const void*)br_fft_pair_kernel<LOGN, VARIANT, 3, 4>;
+        case 43: return (const void*)br_fft_pair_kernel<LOGN, VARIANT, 4, 3>;
+        case 44: return (const void*)br_fft_pair_kernel<LOGN, VARIANT, 4, 4>;
+        default: return nullptr;
+    }
+}
+
 template <int LOGN, int VARIANT, int CS>
 const void* pick_cluster(uint32_t digits, int limbs) {
     switch (digits * 10 + limbs) {
@@ -161,6 +174,14 @@ const void* br_fft_kernel_ptr(int logn, int variant, uint32_t digits, int limbs)
         return logn == 10 ? pick<10, kCggiBinary>(digits, limbs) : logn == 11 ? pick<11, kCggiBinary>(digits, limbs) : nullptr;
     if (variant == kCggiTernary)
         return logn == 10 ? pick<10, kCggiTernary>(digits, limbs) : logn == 11 ? pick<11, kCggiTernary>(digits, limbs) : nullptr;
+    return nullptr;
+}
+
+const void* br_fft_pair_ptr(int logn, int variant, uint32_t digits, int limbs) {
+    if (variant == kCggiBinary)
+        return logn == 10 ? pick_pair<10, kCggiBinary>(digits, limbs) : logn == 11 ? pick_pair<11, kCggiBinary>(digits, limbs) : nullptr;
+    if (variant == kCggiTernary)
+        return logn == 10 ? pick_pair<10, kCggiTernary>(digits, limbs) : logn == 11 ? pick_pair<11, kCggiTernary>(digits, limbs) : nullptr;
     return nullptr;
 }
 

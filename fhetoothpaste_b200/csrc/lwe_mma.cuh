@@ -24,6 +24,7 @@
 
 #include "gl_arith.cuh"
 #include "ks_util_kernels.cuh"
+#include "mbar.cuh"
 
 namespace tp {
 
@@ -41,28 +42,6 @@ struct LweMmaParams {
     int* err;             // host-mapped: set when a wait ran out
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t* b, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect(uint64_t* b, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
-}
-// Waits for the phase of parity `ph`; gives up (false) after a few seconds.
-__device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t ph) {
-    for (uint32_t i = 0; i < (1u << 22); ++i) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(smem_u32(b)), "r"(ph)
-            : "memory");
-        if (ok) return true;
-    }
-    return false;
-}
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
@@ -122,7 +101,7 @@ lwe_mma_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__
             mbar_init(empty + s, 1);
         }
         mbar_init(done, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        mbar_init_fence();
     }
     if (warp == 5)
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_s)),
