@@ -96,23 +96,27 @@ __device__ __forceinline__ ulonglong2 rot_pair(Load&& at, uint32_t j, uint32_t s
     return make_ulonglong2((q & 2u) ? gl_neg(a) : a, (q == 1u || q == 2u) ? gl_neg(b) : b);
 }
 
-// This thread's 16 points (pairs j = tg + i TG) of one digit of an accumulator half: (v >> sh) &
-// mk - off (off carries 2^52). Signed digits of v itself; unsigned ones of (X^-a - 1) v.
-template <int LOGK, bool SIGNED>
-__device__ __forceinline__ void digit_points(double2 (&x)[16], const ulonglong2* ah, int tg, uint32_t a, uint32_t sh,
-                                             uint32_t mk, double off) {
+// This thread's 16 points (pairs j = tg + i TG) of one digit of the pairs at v: (v >> sh) & mk -
+// off (off carries 2^52).
+template <int LOGK>
+__device__ __forceinline__ void digit_points(double2 (&x)[16], const ulonglong2* v, int tg, uint32_t sh, uint32_t mk,
+                                             double off) {
     constexpr int TG = Fft<LOGK>::T;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-        const int j = tg + i * TG;
-        ulonglong2 v = ah[j];
-        if constexpr (!SIGNED) {
-            const ulonglong2 w = rot_pair<LOGK>([&](uint32_t k) { return ah[k]; }, j, a);
-            v = make_ulonglong2(gl_sub(w.x, v.x), gl_sub(w.y, v.y));
-        }
-        x[i] = make_double2(__hiloint2double(0x43300000, (int)((uint32_t)(v.x >> sh) & mk)) - off,
-                            __hiloint2double(0x43300000, (int)((uint32_t)(v.y >> sh) & mk)) - off);
+        const ulonglong2 p = v[tg + i * TG];
+        x[i] = make_double2(__hiloint2double(0x43300000, (int)((uint32_t)(p.x >> sh) & mk)) - off,
+                            __hiloint2double(0x43300000, (int)((uint32_t)(p.y >> sh) & mk)) - off);
     }
+}
+// Pair u of (X^-a - 1) acc, half u / n: what binary CGGI decomposes (mux_operator.cpp:144-150).
+// Every digit of a half needs it, so the block forms it once (each digit for itself took a third
+// of the forward phase: binary N = 2048, l = 4, 11.7k clocks against 8.7k).
+template <int LOGK>
+__device__ __forceinline__ ulonglong2 rotated_difference(const ulonglong2* acc, uint32_t u, uint32_t a) {
+    const ulonglong2* ah = acc + (u & (1u << LOGK));
+    const ulonglong2 v = acc[u], w = rot_pair<LOGK>([&](uint32_t k) { return ah[k]; }, u & ((1u << LOGK) - 1u), a);
+    return make_ulonglong2(gl_sub(w.x, v.x), gl_sub(w.y, v.y));
 }
 // s += x k
 __device__ __forceinline__ void cmac(double2& s, double2 x, double2 k) {
@@ -259,14 +263,21 @@ br_fft_kernel(const __grid_constant__ BrFftParams prm) {
             }
 
             // ---- digits and forward transforms: group grp takes digit grp % DL of half grp / DL ----
+            const ulonglong2* src = acc;
+            if constexpr (!SIGNED) {
+                ulonglong2* d = reinterpret_cast<ulonglong2*>(buf);
+                for (int u = t; u < 2 * n; u += T) d[u] = rotated_difference<LOGK>(acc, u, a);
+                src = d;
+                __syncthreads();
+            }
+            double2 x[16];
             if (grp < R) {
                 const int h = grp / DL, d = grp - h * DL;
-                const uint32_t sh = prm.dshift[d];
-                const uint32_t mk = (uint32_t)prm.dmask[d];
-                const double off = 4503599627370496.0 + (SIGNED ? (double)prm.ddelta[d] : 0.0);
-                const ulonglong2* ah = acc + h * n;
-                double2 x[16];
-                digit_points<LOGK, SIGNED>(x, ah, tg, a, sh, mk, off);
+                digit_points<LOGK>(x, src + h * n, tg, prm.dshift[d], (uint32_t)prm.dmask[d],
+                                   4503599627370496.0 + (SIGNED ? (double)prm.ddelta[d] : 0.0));
+            }
+            if constexpr (!SIGNED) __syncthreads();  // the differences are read before the transforms overwrite them
+            if (grp < R) {
                 F::head(x, prm.head);
                 double2* pb = buf + grp * n;
 #pragma unroll
@@ -516,11 +527,21 @@ br_fft_pair_kernel(const __grid_constant__ BrFftParams prm) {
             }
 
             // ---- digits and forward transforms; the other half's slots to the other block ----
+            const ulonglong2* src = acc;
+            if constexpr (!SIGNED) {
+                ulonglong2* d = reinterpret_cast<ulonglong2*>(buf);
+                for (int u = t; u < 2 * n; u += T) d[u] = rotated_difference<LOGK>(acc, u, a);
+                src = d;
+                __syncthreads();
+            }
+            double2 x[16];
             if (grp < R) {
                 const int h = grp / DL, d = grp - h * DL;
-                double2 x[16];
-                digit_points<LOGK, SIGNED>(x, acc + h * n, tg, a, prm.dshift[d], (uint32_t)prm.dmask[d],
-                                           4503599627370496.0 + (SIGNED ? (double)prm.ddelta[d] : 0.0));
+                digit_points<LOGK>(x, src + h * n, tg, prm.dshift[d], (uint32_t)prm.dmask[d],
+                                   4503599627370496.0 + (SIGNED ? (double)prm.ddelta[d] : 0.0));
+            }
+            if constexpr (!SIGNED) __syncthreads();  // the differences are read before the transforms overwrite them
+            if (grp < R) {
                 F::head(x, prm.head);
                 double2* pb = buf + grp * n;
 #pragma unroll
@@ -682,7 +703,7 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
     constexpr int PP = br_fft_cluster_polys(DL, L, CS);
     constexpr uint32_t MASK2N = 2u * N - 1u;
     constexpr bool SIGNED = VARIANT != kCggiBinary;
-    static_assert(8 % CS == 0 && PP * TG <= T, "block shape");
+    static_assert(8 % CS == 0 && PP * TG <= T - 32, "block shape");
 
     extern __shared__ __align__(16) uint64_t smem[];
     double2* work = reinterpret_cast<double2*>(smem);                  // PP n
@@ -745,8 +766,9 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
 
         auto prefetch = [&](uint32_t it) {  // this block's slots of an iteration's key, one thread per limb
             constexpr uint32_t per = (uint32_t)R * C * LANES * 16;
-            if (it < prm.n && t < L)
-                l2_prefetch(reinterpret_cast<const char*>(prm.key) + (((uint64_t)it * L + t) * 8 + c * M) * per, M * per);
+            const uint32_t l = (uint32_t)(t - (T - 32));  // of a warp that has no transform
+            if (it < prm.n && l < L)
+                l2_prefetch(reinterpret_cast<const char*>(prm.key) + (((uint64_t)it * L + l) * 8 + c * M) * per, M * per);
         };
         prefetch(0);
         prefetch(1);
@@ -755,18 +777,25 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
             prefetch(it + 2);
             const uint32_t a = lwe_s[it];
             if (a == 0) continue;
-            if (t == 0) mbar_expect(bar, R * NS * 16);
+            if (t == T - 1) mbar_expect(bar, R * NS * 16);
 
             // ---- digits and forward transforms, slots to their blocks ----
             const int p = c * PP + grp;
+            const ulonglong2* src = acc;
+            if constexpr (!SIGNED) {
+                // in the words' area, which is written again only after this block's digits have gone
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    if (c >= first_of(h) && c <= last_of(h))
+                        for (int u = t; u < n; u += T) gb[h * n + u] = rotated_difference<LOGK>(acc, h * n + u, a);
+                src = gb;
+                __syncthreads();
+            }
             if (grp < PP && p < R) {
                 const int h = p / DL, d = p - h * DL;
-                const uint32_t sh = prm.dshift[d];
-                const uint32_t mk = (uint32_t)prm.dmask[d];
-                const double off = 4503599627370496.0 + (SIGNED ? (double)prm.ddelta[d] : 0.0);
-                const ulonglong2* ah = acc + h * n;
                 double2 x[16];
-                digit_points<LOGK, SIGNED>(x, ah, tg, a, sh, mk, off);
+                digit_points<LOGK>(x, src + h * n, tg, prm.dshift[d], (uint32_t)prm.dmask[d],
+                                   4503599627370496.0 + (SIGNED ? (double)prm.ddelta[d] : 0.0));
                 F::head(x, prm.head);
                 double2* pb = work + grp * n;
 #pragma unroll
