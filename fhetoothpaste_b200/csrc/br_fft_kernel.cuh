@@ -133,18 +133,18 @@ __device__ __forceinline__ double2 csubmul(double2 lo, double2 w, double2 hi) {
     return make_double2(fma(w.y, hi.y, fma(-w.x, hi.x, lo.x)), fma(-w.y, hi.x, fma(-w.x, hi.y, lo.y)));
 }
 // Rounded limbs (in place of the products in buf) to words G mod p; acc += G (binary) or
-// (X^-a - 1) G (ternary). All T threads; ends with a barrier.
-template <int LOGK, int VARIANT, int L, int T>
+// (X^-a - 1) G (ternary), over H halves. All T threads; ends with a barrier.
+template <int LOGK, int VARIANT, int L, int T, int H = 2>
 __device__ __forceinline__ void recombine_update(double2* buf, ulonglong2* acc, int t, uint32_t a) {
     constexpr int n = 1 << LOGK;
     const ulonglong2* wb = reinterpret_cast<const ulonglong2*>(buf);
     ulonglong2* gb = reinterpret_cast<ulonglong2*>(buf);
-    constexpr int U = (2 * n + T - 1) / T;
+    constexpr int U = (H * n + T - 1) / T;
     ulonglong2 gv[U];
 #pragma unroll
     for (int k = 0; k < U; ++k) {
         const int u = t + k * T;
-        if ((2 * n) % T == 0 || u < 2 * n) {
+        if ((H * n) % T == 0 || u < H * n) {
             const int h = u >> LOGK, pos = fft_pos(u & (n - 1));
             uint64_t cx[L], cy[L];
 #pragma unroll
@@ -168,7 +168,7 @@ __device__ __forceinline__ void recombine_update(double2* buf, ulonglong2* acc, 
 #pragma unroll
         for (int k = 0; k < U; ++k) {
             const int u = t + k * T;
-            if ((2 * n) % T == 0 || u < 2 * n) {
+            if ((H * n) % T == 0 || u < H * n) {
                 const ulonglong2* gh = gb + (u >> LOGK) * (L * n);
                 const ulonglong2 w = rot_pair<LOGK>([&](uint32_t j) { return gh[fft_pos((int)j)]; }, u & (n - 1), a);
                 const ulonglong2 v = acc[u];
@@ -922,6 +922,223 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
         }
     }
     if (!ok) atomicOr(prm.err, 2u);
+}
+
+// ---------------------------------------------------------------------------
+// N = 4096: one rotation on a cluster of two blocks, block c holding accumulator half c (both
+// halves with their digits' transforms, 6 x 32 KB at l = 3, do not fit one SM). Block c transforms
+// the l digits of its half, multiplies slot half c of all 2l digits for both halves and all limbs,
+// and transforms, rounds and recombines the L limb polynomials of its half, so that only slots
+// cross: half of the digits' as bulk copies, half of the products as stores. The pass tables are
+// read through L1 (no shared memory is left for them). 74 clusters are resident; ternary, l = 3, n
+// = 60: 74 rotations 4.01 -> 1.58 ms, 148 4.02 -> 3.2, one 3.96 -> 2.49 (modular -> here). Key
+// batches 1 / 2 / 3 ahead: 1.70 / 1.66 / 1.58 ms.
+// ---------------------------------------------------------------------------
+__host__ __device__ constexpr int br_fft_halves_threads(int logn, int limbs) { return (1 << (logn - 5)) * limbs; }
+// Transform buffers (L polynomials), receive area (l half polynomials), accumulator half, monomial
+// factors, barrier, LWE words (16-bit).
+__host__ __device__ constexpr size_t br_fft_halves_smem(int logn, int dl, int limbs, uint32_t n) {
+    const size_t k = (size_t)1 << (logn - 1);
+    return (limbs * k + dl * (k / 2) + k + 5) * 16 + ((size_t)(n + 1 + 7) / 8) * 16;
+}
+
+template <int LOGN, int VARIANT, int DL, int L>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(br_fft_halves_threads(LOGN, L), 1)
+br_fft_halves_kernel(const __grid_constant__ BrFftParams prm) {
+    static_assert(VARIANT == kCggiBinary || VARIANT == kCggiTernary, "CGGI only");
+    constexpr int LOGK = LOGN - 1;
+    using F = Fft<LOGK>;
+    constexpr int N = 1 << LOGN, n = F::n, TG = F::T;
+    constexpr int G = br_rgsw_per_group(VARIANT);
+    constexpr int C = 2 * G, R = 2 * DL;
+    constexpr int T = br_fft_halves_threads(LOGN, L);
+    constexpr int LANES = n / 16, M = 8;       // slots c n/2 + lane + m LANES of this thread, one limb
+    constexpr uint32_t MASK2N = 2u * N - 1u;
+    constexpr bool SIGNED = VARIANT != kCggiBinary;
+    static_assert(DL <= L && TG * L == T && LANES * L == T, "block shape");
+
+    extern __shared__ __align__(16) uint64_t smem[];
+    double2* buf = reinterpret_cast<double2*>(smem);                     // L n
+    double2* recv = buf + L * n;                                         // DL n/2: the other half's digits
+    ulonglong2* acc = reinterpret_cast<ulonglong2*>(recv + DL * (n / 2));  // n: plus corr (signed)
+    double2* mono_s = reinterpret_cast<double2*>(acc + n);               // 4: factors of the key's m = 4 c + q
+    uint64_t* bar = reinterpret_cast<uint64_t*>(mono_s + 4);
+    uint16_t* lwe_s = reinterpret_cast<uint16_t*>(mono_s + 5);
+
+    auto cluster = cooperative_groups::this_cluster();
+    const int c = (int)cluster.block_rank();
+    const int t = threadIdx.x;
+    const int grp = t / TG, tg = t % TG;
+    const int limb = t / LANES, lane = t % LANES;
+    uint32_t phase = 0;
+    bool ok = true;  // a wait for the other block's digits ran out
+    if (t == 0) {
+        mbar_init(bar, 1);
+        mbar_init_fence();
+    }
+    double2* buf_peer = cluster.map_shared_rank(buf, (unsigned)(c ^ 1));
+    cluster.sync();  // both blocks running, their barriers set, before remote stores
+
+    for (uint64_t b = blockIdx.x >> 1; b < prm.batch; b += gridDim.x >> 1) {
+        __syncthreads();
+        const uint64_t* lwe = prm.lwes + b * prm.lwe_stride;
+        bool bad = false;
+        for (uint32_t i = t; i <= prm.n; i += T) {
+            const uint64_t v = lwe[i];
+            bad |= v > MASK2N;
+            lwe_s[i] = (uint16_t)(v & MASK2N);
+        }
+        if (bad && c == 0) atomicOr(prm.err, 1u);
+        __syncthreads();
+        {
+            // acc = half c of acc_in X^b, plus the signed digits' corrector
+            const uint64_t* a = prm.accs + b * prm.acc_stride + (uint64_t)c * N;
+            const uint32_t s = (2u * N - lwe_s[prm.n]) & MASK2N;
+            for (int u = t; u < n; u += T) {
+                ulonglong2 v = rot_pair<LOGK>(
+                    [&](uint32_t j) { return make_ulonglong2(gl_canon(a[j]), gl_canon(a[j + n])); }, u, s);
+                if constexpr (SIGNED) v = make_ulonglong2(gl_add(v.x, prm.corr), gl_add(v.y, prm.corr));
+                acc[u] = v;
+            }
+        }
+        __syncthreads();
+
+        auto prefetch = [&](uint32_t it) {  // this block's share of an iteration's key, as in the one-block form
+            constexpr uint32_t bytes = (uint32_t)L * 8 * R * C * (n / 8) * 16;
+            const uint32_t share = ((bytes + gridDim.x - 1) / gridDim.x + 127u) & ~127u;
+            const uint32_t off = blockIdx.x * share;
+            if (it < prm.n && off < bytes) l2_prefetch(reinterpret_cast<const char*>(prm.key) + (uint64_t)it * bytes + off,
+                                                       min(share, bytes - off));
+        };
+        if (t == 0) {
+            prefetch(0);
+            prefetch(1);
+        }
+#pragma unroll 1
+        for (uint32_t it = 0; it < prm.n; ++it) {
+            if (t == 0) prefetch(it + 2);
+            const uint32_t a = lwe_s[it];
+            if (a == 0) continue;
+            if (t == 0) mbar_expect(bar, DL * (n / 2) * 16);
+            if constexpr (VARIANT == kCggiTernary) {
+                if (t < 4) mono_s[t] = __ldg(prm.roots + ((4u * a * (__brev((uint32_t)(4 * c + t)) >> 29)) & MASK2N));
+            }
+
+            // ---- digits and forward transforms; the other half's slots to the other block ----
+            const ulonglong2* src = acc;
+            if constexpr (!SIGNED) {
+                ulonglong2* d = reinterpret_cast<ulonglong2*>(buf);
+                for (int u = t; u < n; u += T) d[u] = rotated_difference<LOGK>(acc, u, a);
+                src = d;
+                __syncthreads();
+            }
+            double2 x[16];
+            if (grp < DL)
+                digit_points<LOGK>(x, src, tg, prm.dshift[grp], (uint32_t)prm.dmask[grp],
+                                   4503599627370496.0 + (SIGNED ? (double)prm.ddelta[grp] : 0.0));
+            if constexpr (!SIGNED) __syncthreads();
+            if (grp < DL) {
+                F::head(x, prm.head);
+                double2* pb = buf + grp * n;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) pb[fft_pos(tg + i * TG)] = x[i];
+                F::group_sync(grp);
+                F::tail(pb, prm.tab_fwd, tg, grp, [&](int e, double2 v) { pb[fft_pos(e)] = v; });
+                bulk_fence();
+                F::group_sync(grp);
+                if (tg == 0)
+                    bulk_to_block(recv + grp * (n / 2), pb + (c ^ 1) * (n / 2), n / 2 * 16, bar, (uint32_t)(c ^ 1));
+            }
+
+            // ---- slot-wise products, one limb; rows of half c from buf, of the other from recv ----
+            double2 o[M];
+            {
+                // slot lane + m LANES of this half is lane' = lane + (m & 1) LANES of the key's 4 c + m / 2
+                const double2* kp = prm.key + (((uint64_t)it * L + limb) * 8 + 4 * c) * (R * C) * (n / 8) + lane;
+                constexpr int BR = C == 4 ? 1 : 2, NB = M * R / BR;  // four loads a batch, AH batches ahead
+                constexpr int AH = 3;
+                static_assert(R % BR == 0, "a batch lies in one slot");
+                double2 kv[AH + 1][BR][C];
+                auto load = [&](int q, double2 (&k)[BR][C]) {
+                    const int m = q * BR / R, r0 = q * BR % R;
+#pragma unroll
+                    for (int r = 0; r < BR; ++r)
+#pragma unroll
+                        for (int cc = 0; cc < C; ++cc)
+                            k[r][cc] = key_ld(kp + (((m >> 1) * R + r0 + r) * C + cc) * (n / 8) + (m & 1) * LANES);
+                };
+#pragma unroll
+                for (int q = 0; q < AH; ++q) load(q, kv[q]);
+                double2 wb[2];
+                if constexpr (VARIANT == kCggiTernary) {
+#pragma unroll
+                    for (int q = 0; q < 2; ++q)
+                        wb[q] = __ldg(prm.roots + ((a * (1u + 32u * (__brev((uint32_t)(lane + q * LANES)) >> (35 - LOGK)))) & MASK2N));
+                }
+                __syncthreads();
+                ok = ok && mbar_wait(bar, phase);
+                phase ^= 1;
+                double2 s[C];
+#pragma unroll
+                for (int q = 0; q < NB; ++q) {
+                    const int m = q * BR / R, r0 = q * BR % R;
+                    const int el = lane + m * LANES, e = c * (n / 2) + el;
+                    if (q + AH < NB) load(q + AH, kv[(q + AH) % (AH + 1)]);
+                    if (r0 == 0) {
+#pragma unroll
+                        for (int cc = 0; cc < C; ++cc) s[cc] = make_double2(0.0, 0.0);
+                    }
+#pragma unroll
+                    for (int k = 0; k < BR; ++k) {
+                        const int r = r0 + k;
+                        const double2 xv = (r / DL) == c ? buf[(r % DL) * n + fft_pos(e)]
+                                                         : recv[(r % DL) * (n / 2) + fft_pos(el)];
+#pragma unroll
+                        for (int cc = 0; cc < C; ++cc) cmac(s[cc], xv, kv[q % (AH + 1)][k][cc]);
+                    }
+                    if (r0 + BR != R) continue;
+                    double2 v[2] = {s[0], s[1]};
+                    if constexpr (VARIANT == kCggiTernary) {
+                        const double2 w = cmul(wb[m & 1], mono_s[m >> 1]);
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) v[h] = csubmul(s[h], w, s[C - 2 + h]);
+                    }
+                    buf_peer[limb * n + fft_pos(e)] = c ? v[0] : v[1];
+                    o[m] = c ? v[1] : v[0];
+                }
+                cluster.sync();  // both blocks' reads of the digits done, products of the other half's slots here
+#pragma unroll
+                for (int m = 0; m < M; ++m) buf[limb * n + fft_pos(c * (n / 2) + lane + m * LANES)] = o[m];
+                __syncthreads();
+            }
+
+            // ---- backward transforms, rounded coefficients back in place ----
+            {
+                double2* pb = buf + grp * n;
+                F::itail(pb, prm.tab_inv, tg, grp, [&](int e) { return pb + fft_pos(e); });
+                F::group_sync(grp);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) x[i] = pb[fft_pos(tg + i * TG)];
+                F::ihead(x, prm.head);
+#pragma unroll
+                for (int i = 0; i < 16; ++i)
+                    *reinterpret_cast<ulonglong2*>(pb + fft_pos(tg + i * TG)) =
+                        make_ulonglong2(fft_round(x[i].x), fft_round(x[i].y));
+            }
+            __syncthreads();
+            recombine_update<LOGK, VARIANT, L, T, 1>(buf, acc, t, a);
+        }
+
+        uint64_t* res = prm.out + b * (2ull * N) + (uint64_t)c * N;
+        for (int u = t; u < n; u += T) {
+            ulonglong2 v = acc[u];
+            if constexpr (SIGNED) v = make_ulonglong2(gl_sub(v.x, prm.corr), gl_sub(v.y, prm.corr));
+            res[u] = v.x;
+            res[u + n] = v.y;
+        }
+    }
+    if (!ok) atomicOr(prm.err, 2u);
+    cluster.sync();  // no block leaves while the other may still store to it
 }
 
 }  // namespace tp

@@ -350,17 +350,27 @@ static cudaLaunchConfig_t br_fftc_config(const tp_br_ctx* c, int i, unsigned clu
 static void br_setup_fft(tp_br_ctx* c) {
     if (c->prm.variant == TP_BR_BMMP_BINARY) return;
     for (int limbs = 3; limbs <= 4; ++limbs) {
-        const void* k = tp::br_fft_kernel_ptr(c->logn, c->prm.variant, c->prm.digits, limbs);
+        const bool halves = c->logn == 12;
+        const void* k = halves ? tp::br_fft_halves_ptr(c->logn, c->prm.variant, c->prm.digits, limbs)
+                               : tp::br_fft_kernel_ptr(c->logn, c->prm.variant, c->prm.digits, limbs);
         c->fft_limbs = limbs;
         if (!k || !br_fft_key_exact(c, tp::fft_typical_norm2(c->logn - 1, limbs))) continue;
-        const size_t smem = tp::br_fft_smem(c->logn, (int)c->prm.digits, limbs, c->prm.lwe_dim);
+        const size_t smem = halves ? tp::br_fft_halves_smem(c->logn, (int)c->prm.digits, limbs, c->prm.lwe_dim)
+                                   : tp::br_fft_smem(c->logn, (int)c->prm.digits, limbs, c->prm.lwe_dim);
         int per_sm = 0;
         cudaError_t e = smem <= 227u * 1024u
                             ? cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
                             : cudaErrorInvalidValue;
-        if (e == cudaSuccess)
+        if (e == cudaSuccess && halves) {  // clusters of two blocks
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(2 * (unsigned)sm_count(c->device));
+            cfg.blockDim = dim3(tp::br_fft_halves_threads(c->logn, limbs));
+            cfg.dynamicSmemBytes = smem;
+            e = cudaOccupancyMaxActiveClusters(&per_sm, k, &cfg);
+        } else if (e == cudaSuccess) {
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k,
                                                               tp::br_fft_threads(c->logn, (int)c->prm.digits, limbs), smem);
+        }
         if (e == cudaSuccess && per_sm > 0) e = tp::fft_tables(c->device, c->logn - 1, &c->fft_tab);
         if (e != cudaSuccess || per_sm < 1) {
             cudaGetLastError();  // clear the optional probe's error
@@ -368,7 +378,8 @@ static void br_setup_fft(tp_br_ctx* c) {
         }
         c->fft_kernel = k;
         c->fft_smem = smem;
-        c->fft_cap = per_sm * sm_count(c->device);
+        c->fft_cap = halves ? per_sm : per_sm * sm_count(c->device);
+        if (halves) return;
         {
             auto& f = c->fftp;
             const void* kp = tp::br_fft_pair_ptr(c->logn, c->prm.variant, c->prm.digits, limbs);
@@ -402,7 +413,8 @@ static void br_setup_fft(tp_br_ctx* c) {
 
 // The form of a launch of `batch` rotations whose context left the choice open: clusters of
 // 2^(i + 1) blocks per rotation in double precision (i = 0 .. 2), one block (kFftOneBlock) or two
-// rotations on two blocks (kFftPair) in double precision, or the modular kernels (kModular,
+// rotations on two blocks (kFftPair) in double precision (at N = 4096 always one rotation on two
+// blocks, kFftHalves), or the modular kernels (kModular,
 // kModularPair: two blocks per rotation). Milliseconds at n = 60, one wave each (15, 30, 74
 // clusters, 148 rotations) and 600 rotations:
 //                                  clusters 8 / 4 / 2    one block   pair        modular, pair
@@ -416,9 +428,10 @@ static void br_setup_fft(tp_br_ctx* c) {
 // its one wave; then one block, or the pair where the key polynomials read per slot and iteration
 // (2 G rows limbs) reach 64 and halving them pays for the exchanges (at N = 1024, where two
 // blocks share an SM, from the second block per SM on, or from 128).
-enum { kFftOneBlock = 3, kFftPair = 4, kModularPair = 5, kModular = 6 };
+enum { kFftOneBlock = 3, kFftPair = 4, kFftHalves = 5, kModularPair = 6, kModular = 7 };
 static int br_form(const tp_br_ctx* c, uint64_t batch) {
     if (!c->fft_ready || !c->fft_on) return kModular;
+    if (c->logn == 12) return kFftHalves;
     for (int i = 2; i >= 0; --i)
         if (batch <= (uint64_t)c->fftc[i].cap) return i;
     if (c->logn >= 11 && c->loge == 2 && batch <= (uint64_t)c->pair_cap) return kModularPair;
@@ -2901,7 +2914,8 @@ int br_cluster_ctas(const tp_br_ctx* c) { return c ? 1 << c->logs : 1; }
 
 uint64_t br_fft_blocks(const tp_br_ctx* c, uint64_t batch) {
     const int i = c ? br_form(c, batch) : kModular;
-    if (i > kFftPair) return 0;
+    if (i > kFftHalves) return 0;
+    if (i == kFftHalves) return 2 * std::min<uint64_t>(batch, c->fft_cap);
     if (i == kFftPair) return 2 * std::min<uint64_t>((batch + 1) / 2, c->fftp.cap);
     return i < kFftOneBlock ? batch << (i + 1) : std::min<uint64_t>(batch, c->fft_cap);
 }
@@ -2925,7 +2939,7 @@ tp_status br_batch_launch(tp_br_ctx* c, uint64_t batch, uint64_t* results, const
     if (((uintptr_t)results & 15) || ((uintptr_t)accs & 7) || ((uintptr_t)lwes & 7))
         return fail(TP_ERR_PARAM, "results must be 16-byte aligned, lwes/accs 8-byte aligned");
     const int form = br_form(c, batch);
-    if (form <= kFftPair) {
+    if (form <= kFftHalves) {
         TP_CUDA(cudaSetDevice(c->device));
         tp::BrFftParams fp{};
         fp.key = c->fft_key;
@@ -2951,6 +2965,10 @@ tp_status br_batch_launch(tp_br_ctx* c, uint64_t batch, uint64_t* results, const
             const cudaLaunchConfig_t cfg =
                 br_fftc_config(c, i, (unsigned)std::min<uint64_t>(batch, c->fftc[i].cap), (cudaStream_t)stream, &attr);
             TP_CUDA(cudaLaunchKernelExC(&cfg, c->fftc[i].k, fargs));
+        } else if (form == kFftHalves) {
+            TP_CUDA(cudaLaunchKernel(c->fft_kernel, dim3(2 * (unsigned)std::min<uint64_t>(batch, c->fft_cap)),
+                                     dim3(tp::br_fft_halves_threads(c->logn, c->fft_limbs)), fargs, c->fft_smem,
+                                     (cudaStream_t)stream));
         } else if (form == kFftPair) {
             TP_CUDA(cudaLaunchKernel(c->fftp.k, dim3(2 * (unsigned)std::min<uint64_t>((batch + 1) / 2, c->fftp.cap)),
                                      dim3(tp::br_fft_threads(c->logn, (int)c->prm.digits, c->fft_limbs)), fargs,

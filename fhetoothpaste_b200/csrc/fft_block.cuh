@@ -15,8 +15,9 @@
 // with one twiddle per block of a level, tw[m + b] for block b of the level with m blocks.
 //
 // One polynomial is transformed by n/16 threads, 16 complex points (64 registers) each,
-// in three passes over an in-place shared-memory buffer: the first log2(n) - 6 levels on
-// elements t + i n/16, then 3 levels inside blocks of 64 and 3 levels inside blocks of 8.
+// in three passes over an in-place shared-memory buffer: the first levels (3 or 4) on
+// elements t + i n/16, then 3 levels inside blocks of 64 (4 inside blocks of 128 at n = 2048)
+// and 3 levels inside blocks of 8.
 // Twiddles of odd blocks are i times their even neighbour's and need no table entry.
 #pragma once
 
@@ -33,9 +34,14 @@ struct FftHead {
     double2 inv[16];  // (cos, sin) of tw[k]
 };
 
-// Words (double2) of the later passes' tables for n points: pass 2 has 2^(k-6) blocks,
-// pass 3 n/8, four entries each (first level, second, third for the two even children).
-__host__ __device__ constexpr int fft_table_len(int logk) { return 4 * (1 << (logk - 6)) + 4 * (1 << (logk - 3)); }
+// The later passes' tables (double2): pass 2 has 2^min(k-6, 4) blocks, pass 3 n/8, with four
+// entries each (first level, second, third for the two even children) or, for a pass 2 of four
+// levels, eight (and the four even grandchildren).
+__host__ __device__ constexpr int fft_blocks2(int logk) { return 1 << (logk < 10 ? logk - 6 : 4); }
+__host__ __device__ constexpr int fft_entries2(int logk) { return logk > 10 ? 8 : 4; }
+__host__ __device__ constexpr int fft_table_len(int logk) {
+    return fft_entries2(logk) * fft_blocks2(logk) + 4 * (1 << (logk - 3));
+}
 
 // Position of element e in a polynomial's buffer, in 16-byte units: the unit inside each
 // 128-byte line is permuted so that every pass and the slot-wise reads are conflict-free.
@@ -100,13 +106,67 @@ __device__ __forceinline__ void fft_iradix8(double2 (&x)[8], const double2 (&w)[
     for (int k = 0; k < 4; ++k) fft_ibfly(x[k], x[k + 4], w[0]);
 }
 
-// LOGK = log2 n (9 or 10), 16 points per thread.
+// Four levels on sixteen points (distances 8, 4, 2, 1) inside one block, twiddles as above and
+// w[4] .. w[7] for the fourth level's blocks 8b, 8b + 2, 8b + 4, 8b + 6.
+__device__ __forceinline__ void fft_radix16(double2 (&x)[16], const double2* w, int stride) {
+    const double2 w0 = w[0], w1 = w[stride];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) fft_bfly(x[k], x[k + 8], w0);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        fft_bfly(x[k], x[k + 4], w1);
+        fft_bfly_i(x[k + 8], x[k + 12], w1);
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const double2 w2 = w[(2 + q) * stride];
+#pragma unroll
+        for (int k = 8 * q; k < 8 * q + 2; ++k) {
+            fft_bfly(x[k], x[k + 2], w2);
+            fft_bfly_i(x[k + 4], x[k + 6], w2);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const double2 w3 = w[(4 + q) * stride];
+        fft_bfly(x[4 * q], x[4 * q + 1], w3);
+        fft_bfly_i(x[4 * q + 2], x[4 * q + 3], w3);
+    }
+}
+__device__ __forceinline__ void fft_iradix16(double2 (&x)[16], const double2* w, int stride) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const double2 w3 = w[(4 + q) * stride];
+        fft_ibfly(x[4 * q], x[4 * q + 1], w3);
+        fft_ibfly_i(x[4 * q + 2], x[4 * q + 3], w3);
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const double2 w2 = w[(2 + q) * stride];
+#pragma unroll
+        for (int k = 8 * q; k < 8 * q + 2; ++k) {
+            fft_ibfly(x[k], x[k + 2], w2);
+            fft_ibfly_i(x[k + 4], x[k + 6], w2);
+        }
+    }
+    const double2 w0 = w[0], w1 = w[stride];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        fft_ibfly(x[k], x[k + 4], w1);
+        fft_ibfly_i(x[k + 8], x[k + 12], w1);
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) fft_ibfly(x[k], x[k + 8], w0);
+}
+
+// LOGK = log2 n (9, 10 or 11), 16 points per thread.
 template <int LOGK>
 struct Fft {
     static constexpr int n = 1 << LOGK;
     static constexpr int T = n / 16;          // threads per polynomial
-    static constexpr int HEAD = LOGK - 6;     // levels of the first pass
-    static_assert(HEAD == 3 || HEAD == 4, "built for 512 and 1024 points");
+    static constexpr int HEAD = LOGK < 10 ? LOGK - 6 : 4;  // levels of the first pass
+    static constexpr bool MID16 = LOGK > 10;  // the second pass has four levels
+    static_assert(LOGK >= 9 && LOGK <= 11, "built for 512, 1024 and 2048 points");
 
     // Barrier of one polynomial's threads (group g of the block).
     static __device__ __forceinline__ void group_sync(int g) {
@@ -155,23 +215,33 @@ struct Fft {
     // put(e, value). tab = pass 2 then pass 3 entries.
     template <typename Put>
     static __device__ __forceinline__ void tail(double2* buf, const double2* tab, int t, int g, Put&& put) {
-        constexpr int B2 = 1 << HEAD, B3 = n / 8;
+        constexpr int B2 = fft_blocks2(LOGK), B3 = n / 8;
         double2 x[8], w[4];
-        load_tw(w, tab, B2, t >> 2);
+        if constexpr (MID16) {
+            double2 y[16];
+            const int e0 = ((t >> 3) << 7) + (t & 7);
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const int e0 = ((t >> 2) << 6) + (t & 3) + 4 * q;
+            for (int k = 0; k < 16; ++k) y[k] = buf[fft_pos(e0 + 8 * k)];
+            fft_radix16(y, tab + (t >> 3), B2);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) x[k] = buf[fft_pos(e0 + 8 * k)];
-            fft_radix8(x, w);
+            for (int k = 0; k < 16; ++k) buf[fft_pos(e0 + 8 * k)] = y[k];
+        } else {
+            load_tw(w, tab, B2, t >> 2);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) buf[fft_pos(e0 + 8 * k)] = x[k];
+            for (int q = 0; q < 2; ++q) {
+                const int e0 = ((t >> 2) << 6) + (t & 3) + 4 * q;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) x[k] = buf[fft_pos(e0 + 8 * k)];
+                fft_radix8(x, w);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) buf[fft_pos(e0 + 8 * k)] = x[k];
+            }
         }
         group_sync(g);
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             const int b = t + q * T;
-            load_tw(w, tab + 4 * B2, B3, b);
+            load_tw(w, tab + fft_entries2(LOGK) * B2, B3, b);
 #pragma unroll
             for (int k = 0; k < 8; ++k) x[k] = buf[fft_pos(8 * b + k)];
             fft_radix8(x, w);
@@ -183,12 +253,12 @@ struct Fft {
     // barrier that ihead's reads need.
     template <typename At>
     static __device__ __forceinline__ void itail(double2* buf, const double2* tab, int t, int g, At&& at) {
-        constexpr int B2 = 1 << HEAD, B3 = n / 8;
+        constexpr int B2 = fft_blocks2(LOGK), B3 = n / 8;
         double2 x[8], w[4];
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             const int b = t + q * T;
-            load_tw(w, tab + 4 * B2, B3, b);
+            load_tw(w, tab + fft_entries2(LOGK) * B2, B3, b);
 #pragma unroll
             for (int k = 0; k < 8; ++k) x[k] = *at(8 * b + k);
             fft_iradix8(x, w);
@@ -196,15 +266,25 @@ struct Fft {
             for (int k = 0; k < 8; ++k) buf[fft_pos(8 * b + k)] = x[k];
         }
         group_sync(g);
-        load_tw(w, tab, B2, t >> 2);
+        if constexpr (MID16) {
+            double2 y[16];
+            const int e0 = ((t >> 3) << 7) + (t & 7);
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const int e0 = ((t >> 2) << 6) + (t & 3) + 4 * q;
+            for (int k = 0; k < 16; ++k) y[k] = buf[fft_pos(e0 + 8 * k)];
+            fft_iradix16(y, tab + (t >> 3), B2);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) x[k] = buf[fft_pos(e0 + 8 * k)];
-            fft_iradix8(x, w);
+            for (int k = 0; k < 16; ++k) buf[fft_pos(e0 + 8 * k)] = y[k];
+        } else {
+            load_tw(w, tab, B2, t >> 2);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) buf[fft_pos(e0 + 8 * k)] = x[k];
+            for (int q = 0; q < 2; ++q) {
+                const int e0 = ((t >> 2) << 6) + (t & 3) + 4 * q;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) x[k] = buf[fft_pos(e0 + 8 * k)];
+                fft_iradix8(x, w);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) buf[fft_pos(e0 + 8 * k)] = x[k];
+            }
         }
     }
 };

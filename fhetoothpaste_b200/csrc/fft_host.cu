@@ -177,6 +177,19 @@ const void* br_fft_kernel_ptr(int logn, int variant, uint32_t digits, int limbs)
     return nullptr;
 }
 
+const void* br_fft_halves_ptr(int logn, int variant, uint32_t digits, int limbs) {
+    if (logn != 12 || limbs != 4 || digits < 2 || digits > 4) return nullptr;
+    if (variant == kCggiBinary)
+        return digits == 2   ? (const void*)br_fft_halves_kernel<12, kCggiBinary, 2, 4>
+               : digits == 3 ? (const void*)br_fft_halves_kernel<12, kCggiBinary, 3, 4>
+                             : (const void*)br_fft_halves_kernel<12, kCggiBinary, 4, 4>;
+    if (variant == kCggiTernary)
+        return digits == 2   ? (const void*)br_fft_halves_kernel<12, kCggiTernary, 2, 4>
+               : digits == 3 ? (const void*)br_fft_halves_kernel<12, kCggiTernary, 3, 4>
+                             : (const void*)br_fft_halves_kernel<12, kCggiTernary, 4, 4>;
+    return nullptr;
+}
+
 const void* br_fft_pair_ptr(int logn, int variant, uint32_t digits, int limbs) {
     if (variant == kCggiBinary)
         return logn == 10 ? pick_pair<10, kCggiBinary>(digits, limbs) : logn == 11 ? pick_pair<11, kCggiBinary>(digits, limbs) : nullptr;
@@ -198,7 +211,7 @@ cudaError_t fft_tables(int device, int logk, const FftTables** out) {
             *out = t;
             return cudaSuccess;
         }
-    const uint32_t n = 1u << logk, B2 = 1u << (logk - 6), B3 = n / 8, len = (uint32_t)fft_table_len(logk);
+    const uint32_t n = 1u << logk, B2 = (uint32_t)fft_blocks2(logk), B3 = n / 8, len = (uint32_t)fft_table_len(logk);
     auto ratio = [](uint32_t k) {
         const long double a = tw_angle(k);
         return make_double2((double)cosl(a), (double)(sinl(a) / cosl(a)));
@@ -209,17 +222,18 @@ cudaError_t fft_tables(int device, int logk, const FftTables** out) {
     };
     std::vector<double2> f(len), v(len), roots(4 * n);
     std::vector<double4> dd(n);
-    auto fill = [&](uint32_t off, uint32_t blocks) {
+    auto fill = [&](uint32_t off, uint32_t blocks, int entries) {
         for (uint32_t b = 0; b < blocks; ++b) {
-            const uint32_t k[4] = {blocks + b, 2 * blocks + 2 * b, 4 * blocks + 4 * b, 4 * blocks + 4 * b + 2};
-            for (int q = 0; q < 4; ++q) {
+            const uint32_t k[8] = {blocks + b,             2 * blocks + 2 * b,     4 * blocks + 4 * b,     4 * blocks + 4 * b + 2,
+                                   8 * blocks + 8 * b,     8 * blocks + 8 * b + 2, 8 * blocks + 8 * b + 4, 8 * blocks + 8 * b + 6};
+            for (int q = 0; q < entries; ++q) {
                 f[off + q * blocks + b] = ratio(k[q]);
                 v[off + q * blocks + b] = plain(k[q]);
             }
         }
     };
-    fill(0, B2);
-    fill(4 * B2, B3);
+    fill(0, B2, fft_entries2(logk));
+    fill(fft_entries2(logk) * B2, B3, 4);
     for (uint32_t k = 0; k < 4 * n; ++k) {
         const long double a = acosl(-1.0L) * (long double)k / (long double)(2 * n);
         roots[k] = make_double2((double)cosl(a), (double)sinl(a));
@@ -276,6 +290,8 @@ double fft_typical_norm2(int logk, int limbs) {
 void fft_key_launch(double2* dst, const uint64_t* src, uint64_t polys, uint64_t first, uint32_t G, uint32_t rows,
                     int limbs, const FftTables& tab, unsigned long long* norm2, cudaStream_t st) {
     const size_t smem = sizeof(double4) << tab.logk;  // 32 KB at 1024 points
+    if (smem > 48u * 1024u)
+        cudaFuncSetAttribute(fft_key_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const unsigned blocks = (unsigned)(polys < 4096 ? polys : 4096);
     fft_key_kernel<<<blocks, 256, smem, st>>>(dst, src, polys, first, G, rows, tab.logk, limbs, tab.dd, norm2);
 }

@@ -47,6 +47,8 @@ void fft_key_launch(double2* dst, const uint64_t* src, uint64_t polys, uint64_t 
                     int limbs, const FftTables& tab, unsigned long long* norm2, cudaStream_t st);
 
 const void* br_fft_kernel_ptr(int logn, int variant, uint32_t digits, int limbs);
+// One rotation on a cluster of two blocks, an accumulator half each (N = 4096).
+const void* br_fft_halves_ptr(int logn, int variant, uint32_t digits, int limbs);
 // Two rotations on a cluster of two blocks.
 const void* br_fft_pair_ptr(int logn, int variant, uint32_t digits, int limbs);
 // One rotation on a cluster of cs blocks (2, 4 or 8; nullptr where not built).

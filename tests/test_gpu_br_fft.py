@@ -1,4 +1,4 @@
-"""The double-precision rotation kernel (N = 1024, 2048) against the C oracle and the modular kernels.
+"""The double-precision rotation kernels (N = 1024, 2048, 4096) against the C oracle and the modular kernels.
 
 Every word has to be equal: the kernel runs only where its error bound proves that each
 product coefficient rounds to the exact integer.
@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 P = 0xFFFFFFFF00000001
 # (variant, N, log2 base, digits): three and four limbs, two to four digits, the largest digits of each limb count
 SETS = [(1, 2048, 12, 3), (0, 2048, 14, 4), (1, 2048, 16, 4), (1, 2048, 8, 4), (0, 2048, 12, 3), (1, 1024, 12, 3),
-        (0, 1024, 16, 4), (1, 1024, 16, 2), (0, 1024, 8, 2)]
+        (0, 1024, 16, 4), (1, 1024, 16, 2), (0, 1024, 8, 2), (1, 4096, 12, 3), (0, 4096, 14, 4), (1, 4096, 8, 2)]
 EXTREMES = [0, 1, P - 1, P - 2, P // 2, P // 2 + 1, 1 << 63, (1 << 63) - 1, (1 << 32) - 1]
 
 
@@ -41,14 +41,15 @@ def test_equals_oracle(native, oracle, variant, N, beta, digits, batch, coef):
     lwes, accs = inputs(rng, N, n, batch)
     before = native.tp_kernel_launches()
     got = rot.blind_rotate_batch_host(lwes, accs, out_coef=coef)
-    # clusters of eight, four and (odd batch) pairs or one block each; evaluation-domain results
+    # clusters of eight, four and (odd batch) pairs or one block each, halves on two blocks at N =
+    # 4096; evaluation-domain results
     # are transformed in a second launch
     assert native.tp_kernel_launches() - before == (1 if coef else 2)
     want = oracle.blind_rotate_many(variant, N, n, beta, digits, key, lwes, accs, coef, 4)
     np.testing.assert_array_equal(got, want)
 
 
-@pytest.mark.parametrize("variant,N,beta,digits", SETS[:2] + SETS[5:7])
+@pytest.mark.parametrize("variant,N,beta,digits", SETS[:2] + SETS[5:7] + SETS[9:11])
 @pytest.mark.parametrize("batch", [2 * 148 * 2 + 3, 60, 15])
 def test_equals_modular_kernel_over_forms(native, variant, N, beta, digits, batch):
     """Strides, a shared accumulator, results in place, more rotations than resident blocks."""
