@@ -656,12 +656,13 @@ tp_status tp_br_upload_key(tp_br_ctx* c, const uint64_t* brk, uint64_t words) {
     if (!c->key) TP_CUDA(cudaMalloc(&c->key, c->key_words * 8));
     const uint64_t N = c->prm.ring_dim;
     const uint64_t per_group = (uint64_t)c->G * 4 * N * c->prm.digits;
-    // stage at most ~128 MB of the reference layout at a time
-    uint64_t chunk = (128ull << 20) / (per_group * 8);
+    // two stages of ~8 MB of the reference layout: one is copied while the other is laid out (the
+    // copy from pageable memory takes several times as long as the kernels)
+    uint64_t chunk = (8ull << 20) / (per_group * 8);
     if (chunk < 1) chunk = 1;
     if (chunk > c->groups) chunk = c->groups;
     uint64_t* stage = nullptr;
-    TP_CUDA(cudaMalloc(&stage, chunk * per_group * 8));
+    TP_CUDA(cudaMalloc(&stage, 2 * chunk * per_group * 8));
     tp_status st = TP_OK;
     // the limbs' transforms (one double2 per two words and limb), where there is room for them
     unsigned long long* norm2 = nullptr;
@@ -676,43 +677,54 @@ tp_status tp_br_upload_key(tp_br_ctx* c, const uint64_t* brk, uint64_t words) {
             fft = false;
         }
     }
-    for (uint64_t g0 = 0; g0 < c->groups && st == TP_OK; g0 += chunk) {
-        const uint64_t ng = std::min(chunk, c->groups - g0);
-        cudaError_t e = cudaMemcpy(stage, brk + g0 * per_group, ng * per_group * 8, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) {
-            const uint64_t total = ng * per_group;
-            const int threads = 256;
-            const uint64_t blocks = std::min<uint64_t>((total + threads - 1) / threads, 65535);
-            tp::key_relayout_kernel<<<(unsigned)blocks, threads>>>(c->key + g0 * per_group, stage, ng, c->G,
-                                                                    2 * c->prm.digits, c->logn, c->loge, c->logs);
+    cudaStream_t copy = nullptr, work = nullptr;  // ordered with the legacy stream, not with each other
+    cudaEvent_t copied[2] = {}, done[2] = {};
+    cudaError_t e = cudaStreamCreate(&copy);
+    if (e == cudaSuccess) e = cudaStreamCreate(&work);
+    for (int q = 0; q < 2 && e == cudaSuccess; ++q) {
+        e = cudaEventCreateWithFlags(&copied[q], cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&done[q], cudaEventDisableTiming);
+    }
+    int q = 0;
+    for (uint64_t g0 = 0; g0 < c->groups && e == cudaSuccess && st == TP_OK; g0 += chunk, q ^= 1) {
+        const uint64_t ng = std::min(chunk, c->groups - g0), total = ng * per_group;
+        uint64_t* sg = stage + q * chunk * per_group;
+        if (g0 >= 2 * chunk) e = cudaStreamWaitEvent(copy, done[q], 0);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(sg, brk + g0 * per_group, total * 8, cudaMemcpyHostToDevice, copy);
+        if (e == cudaSuccess) e = cudaEventRecord(copied[q], copy);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(work, copied[q], 0);
+        if (e != cudaSuccess) break;
+        const int threads = 256;
+        const unsigned blocks = (unsigned)std::min<uint64_t>((total + threads - 1) / threads, 65535);
+        tp::key_relayout_kernel<<<blocks, threads, 0, work>>>(c->key + g0 * per_group, sg, ng, c->G, 2 * c->prm.digits,
+                                                              c->logn, c->loge, c->logs);
+        tp::note_launch();
+        if (fft) {
+            // canonical words, coefficients, limb transforms
+            tp::scale_kernel<<<blocks, threads, 0, work>>>(sg, sg, total, 1);
             tp::note_launch();
-            e = cudaGetLastError();
-            if (e == cudaSuccess && fft) {
-                // canonical words, coefficients, limb transforms
-                tp::scale_kernel<<<(unsigned)blocks, threads>>>(stage, stage, total, 1);
-                tp::note_launch();
-                st = ntt_launch((uint32_t)N, total / N, stage, stage, nullptr, false);
-                tp::fft_key_launch(c->fft_key, stage, total / N, g0 * c->G * 4 * c->prm.digits, c->G,
-                                   2 * c->prm.digits, c->fft_limbs, *c->fft_tab, norm2, nullptr);
-                tp::note_launch();
-                e = cudaGetLastError();
-            }
+            st = ntt_launch((uint32_t)N, total / N, sg, sg, work, false);
+            tp::fft_key_launch(c->fft_key, sg, total / N, g0 * c->G * 4 * c->prm.digits, c->G, 2 * c->prm.digits,
+                               c->fft_limbs, *c->fft_tab, norm2, work);
+            tp::note_launch();
         }
-        if (e == cudaSuccess) e = cudaDeviceSynchronize();
-        if (e != cudaSuccess) st = fail(TP_ERR_CUDA, "key upload: %s", cudaGetErrorString(e));
+        e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaEventRecord(done[q], work);
     }
-    cudaFree(stage);
-    if (st == TP_OK && fft) {
-        unsigned long long v = 0;
-        cudaError_t e = cudaMemcpy(&v, norm2, sizeof v, cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) st = fail(TP_ERR_CUDA, "key upload: %s", cudaGetErrorString(e));
-        else c->fft_ready = br_fft_key_exact(c, (double)v);
+    unsigned long long v = 0;
+    if (e == cudaSuccess) e = cudaStreamSynchronize(work);
+    if (e == cudaSuccess && fft) e = cudaMemcpy(&v, norm2, sizeof v, cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) st = fail(TP_ERR_CUDA, "key upload: %s", cudaGetErrorString(e));
+    for (int i = 0; i < 2; ++i) {
+        if (copied[i]) cudaEventDestroy(copied[i]);
+        if (done[i]) cudaEventDestroy(done[i]);
     }
+    if (copy) cudaStreamDestroy(copy);
+    if (work) cudaStreamDestroy(work);
+    cudaFree(stage);  // waits for what an error left in flight
     cudaFree(norm2);
-    if (!c->fft_ready) {  // the modular forms run
-        cudaFree(c->fft_key);
-        c->fft_key = nullptr;
-    }
+    // without it the modular forms run; the buffer stays, a recorded graph may still name it
+    c->fft_ready = st == TP_OK && fft && br_fft_key_exact(c, (double)v);
     if (st == TP_OK) c->key_ready = true;
     return st;
 }
