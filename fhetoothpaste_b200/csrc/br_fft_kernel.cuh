@@ -672,22 +672,25 @@ br_fft_pair_kernel(const __grid_constant__ BrFftParams prm) {
 // its key at a third of the rate that a full GPU's blocks get (they share lines on the way
 // from L2) and runs every transform itself. Here block c transforms the polynomials c PP ..
 // c PP + PP - 1 (PP = 1 at eight blocks), multiplies the slots [c n/CS, (c + 1) n/CS) and
-// recombines the same range of coefficients. Four exchanges an iteration through distributed
-// shared memory, each behind a cluster barrier: digit slots to their blocks, products to the
-// blocks of their limbs, rounded limbs to the blocks of their coefficients, words mod p to
-// the blocks whose digits need them. An area is written again only after a later barrier
-// than its last reads, so four barriers suffice.
+// recombines the same range of coefficients. Four exchanges an iteration, all as bulk copies
+// between the blocks' shared memory that complete on the receiver's barriers (cluster barriers
+// behind remote stores took 1.0k to 1.4k clocks each): digit slots to their blocks, products to
+// the blocks of their limbs, rounded limbs to the blocks of their coefficients, words mod p to the
+// blocks whose digits need them. Every block takes part in each exchange that another block's
+// next step waits for, so an area's next contents are sent only after its last reads: digits i + 1
+// follow words i of all blocks, which follow their products i, and so on round the cycle.
 // ---------------------------------------------------------------------------
 __host__ __device__ constexpr int br_fft_cluster_polys(int dl, int limbs, int cs) {
     return (2 * (dl > limbs ? dl : limbs) + cs - 1) / cs;
 }
 __host__ __device__ constexpr int br_fft_cluster_threads(int logn, int limbs) { return (1 << (logn - 4)) * limbs; }
 // Forward and backward buffers (PP polynomials each), digit slots (2l n/CS), limb and word
-// areas (2L n/CS, 2n), accumulator (2n), pass tables, monomial factors, barrier, LWE words.
+// areas (2L n/CS, also the products on their way out; 2n), accumulator (2n), words on their way out
+// (2 n/CS), pass tables, monomial factors, barriers, LWE words.
 __host__ __device__ constexpr size_t br_fft_cluster_smem(int logn, int dl, int limbs, int cs, uint32_t n) {
     const size_t k = (size_t)1 << (logn - 1);
-    return (2 * br_fft_cluster_polys(dl, limbs, cs) * k + (2 * dl + 2 * limbs) * (k / cs) + 4 * k +
-            2 * fft_table_len(logn - 1) + 9) * 16 + (((size_t)n + 4) / 4) * 16;
+    return (2 * br_fft_cluster_polys(dl, limbs, cs) * k + (2 * dl + 2 * limbs + 2) * (k / cs) + 4 * k +
+            2 * fft_table_len(logn - 1) + 10) * 16 + (((size_t)n + 4) / 4) * 16;
 }
 
 template <int LOGN, int VARIANT, int DL, int L, int CS>
@@ -703,6 +706,9 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
     constexpr int PP = br_fft_cluster_polys(DL, L, CS);
     constexpr uint32_t MASK2N = 2u * N - 1u;
     constexpr bool SIGNED = VARIANT != kCggiBinary;
+    // products and limbs as bulk copies, or (fewer blocks, more words to each) as remote stores behind
+    // a cluster barrier
+    constexpr bool BULK = CS == 8, WORDS = CS == 8 || LOGN == 10;
     static_assert(8 % CS == 0 && PP * TG <= T - 32, "block shape");
 
     extern __shared__ __align__(16) uint64_t smem[];
@@ -712,11 +718,12 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
     ulonglong2* lim = reinterpret_cast<ulonglong2*>(dig + R * NS);     // 2L NS
     ulonglong2* gb = lim + 2 * L * NS;                                 // 2 n
     ulonglong2* acc = gb + 2 * n;                                      // 2 n: plus corr (signed)
-    double2* tab_f = reinterpret_cast<double2*>(acc + 2 * n);
+    ulonglong2* gs = acc + 2 * n;                                      // 2 NS
+    double2* tab_f = reinterpret_cast<double2*>(gs + 2 * NS);
     double2* tab_i = tab_f + fft_table_len(LOGK);
     double2* mono_s = tab_i + fft_table_len(LOGK);
-    uint64_t* bar = reinterpret_cast<uint64_t*>(mono_s + 8);           // every block's digits have come
-    uint32_t* lwe_s = reinterpret_cast<uint32_t*>(mono_s + 9);
+    uint64_t* bar = reinterpret_cast<uint64_t*>(mono_s + 8);           // [4]: digits, products, limbs, words have come
+    uint32_t* lwe_s = reinterpret_cast<uint32_t*>(mono_s + 10);
 
     auto cluster = cooperative_groups::this_cluster();
     const int c = (int)cluster.block_rank();
@@ -730,13 +737,15 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
     // blocks whose forward polynomials are digits of half h
     auto first_of = [](int h) { return h * DL / PP; };
     auto last_of = [](int h) { return (h * DL + DL - 1) / PP; };
+    const uint32_t own_halves = (c >= first_of(0) && c <= last_of(0) ? 1 : 0) + (c >= first_of(1) && c <= last_of(1) ? 1 : 0);
+    const uint32_t own_limbs = c * PP >= 2 * L ? 0 : min(PP, 2 * L - c * PP);  // limb polynomials transformed back here
     uint32_t phase = 0;
-    bool ok = true;  // a wait for the blocks' digits ran out
+    bool ok = true;  // a wait for the other blocks ran out
     if (t == 0) {
-        mbar_init(bar, 1);
+        for (int q = 0; q < 4; ++q) mbar_init(bar + q, 1);
         mbar_init_fence();
     }
-    cluster.sync();  // every block of the cluster running, its barrier set, before remote stores
+    cluster.sync();  // every block of the cluster running, its barriers set, before copies to it
 
     const uint64_t clusters = gridDim.x / CS;
     for (uint64_t b = blockIdx.x / CS; b < prm.batch; b += clusters) {
@@ -777,7 +786,12 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
             prefetch(it + 2);
             const uint32_t a = lwe_s[it];
             if (a == 0) continue;
-            if (t == T - 1) mbar_expect(bar, R * NS * 16);
+            if (t == T - 1) {
+                mbar_expect(bar, R * NS * 16);
+                if (BULK && own_limbs) mbar_expect(bar + 1, own_limbs * n * 16);
+                if constexpr (BULK) mbar_expect(bar + 2, 2 * L * NS * 16);
+                if (WORDS && own_halves) mbar_expect(bar + 3, own_halves * n * 16);
+            }
 
             // ---- digits and forward transforms, slots to their blocks ----
             const int p = c * PP + grp;
@@ -826,7 +840,6 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
                 wb = __ldg(prm.roots + ((a * (1u + 32u * (__brev((uint32_t)lane) >> (35 - LOGK)))) & MASK2N));
             __syncthreads();
             ok = ok && mbar_wait(bar, phase);
-            phase ^= 1;
             double2 s[C];
 #pragma unroll
             for (int q = 0; q < NB; ++q) {
@@ -852,13 +865,22 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int qo = h * L + limb;
-                    cluster.map_shared_rank(inv, (unsigned)(qo / PP))[(qo % PP) * n + fft_pos(c * NS + lane + mm * LANES)] = v[h];
+                    if constexpr (BULK) reinterpret_cast<double2*>(lim)[qo * NS + pos] = v[h];
+                    else cluster.map_shared_rank(inv, (unsigned)(qo / PP))[(qo % PP) * n + c * NS + pos] = v[h];
                 }
             }
-            cluster.sync();
+            if constexpr (BULK) {
+                bulk_fence();
+                __syncthreads();
+                if (t < 2 * L)
+                    bulk_to_block(inv + (t % PP) * n + c * NS, lim + t * NS, NS * 16, bar + 1, (uint32_t)(t / PP));
+            } else {
+                cluster.sync();
+            }
 
             // ---- backward transforms, rounded limbs to the blocks of their coefficients ----
             if (grp < PP && p < 2 * L) {
+                if constexpr (BULK) ok = ok && mbar_wait(bar + 1, phase);
                 double2* pb = inv + grp * n;
                 F::itail(pb, tab_i, tg, grp, [&](int e) { return pb + fft_pos(e); });
                 F::group_sync(grp);
@@ -868,16 +890,23 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
                 F::ihead(x, prm.head);
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                    const int j = tg + i * TG;
-                    cluster.map_shared_rank(lim, (unsigned)(j / NS))[p * NS + j % NS] =
-                        make_ulonglong2(fft_round(x[i].x), fft_round(x[i].y));
+                    const int pos = fft_pos(tg + i * TG);
+                    const ulonglong2 r = make_ulonglong2(fft_round(x[i].x), fft_round(x[i].y));
+                    if constexpr (BULK) *reinterpret_cast<ulonglong2*>(pb + pos) = r;
+                    else cluster.map_shared_rank(lim, (unsigned)(pos / NS))[p * NS + pos % NS] = r;
+                }
+                if constexpr (BULK) {
+                    bulk_fence();
+                    F::group_sync(grp);
+                    if (tg < CS) bulk_to_block(lim + p * NS, pb + tg * NS, NS * 16, bar + 2, (uint32_t)tg);
                 }
             }
-            cluster.sync();
+            if constexpr (!BULK) cluster.sync();
 
             // ---- words mod p to the blocks that need their half ----
+            if constexpr (BULK) ok = ok && mbar_wait(bar + 2, phase);
             for (int u = t; u < 2 * NS; u += T) {
-                const int h = u / NS, j = u % NS;
+                const int h = u / NS, j = fft_pos(c * NS + u % NS) - c * NS;
                 uint64_t cx[L], cy[L];
 #pragma unroll
                 for (int l = 0; l < L; ++l) {
@@ -885,13 +914,27 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
                     cx[l] = v.x;
                     cy[l] = v.y;
                 }
-                const ulonglong2 g = make_ulonglong2(fft_recombine<L>(cx), fft_recombine<L>(cy));
-                for (int q = first_of(h); q <= last_of(h); ++q)
-                    cluster.map_shared_rank(gb, (unsigned)q)[h * n + c * NS + j] = g;
+                const ulonglong2 gw = make_ulonglong2(fft_recombine<L>(cx), fft_recombine<L>(cy));
+                if constexpr (WORDS) gs[u] = gw;
+                else
+                    for (int q = first_of(h); q <= last_of(h); ++q)
+                        cluster.map_shared_rank(gb, (unsigned)q)[h * n + c * NS + u % NS] = gw;
             }
-            cluster.sync();
+            if constexpr (WORDS) {
+                bulk_fence();
+                __syncthreads();
+            } else {
+                cluster.sync();
+            }
+            if (WORDS && t < 2 * CS) {
+                const int h = t / CS, q = t % CS;
+                if (q >= first_of(h) && q <= last_of(h))
+                    bulk_to_block(gb + h * n + c * NS, gs + h * NS, NS * 16, bar + 3, (uint32_t)q);
+            }
 
             // ---- accumulator halves of this block ----
+            if (WORDS && own_halves) ok = ok && mbar_wait(bar + 3, phase);
+            phase ^= 1;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 if (c < first_of(h) || c > last_of(h)) continue;
@@ -922,6 +965,7 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
         }
     }
     if (!ok) atomicOr(prm.err, 2u);
+    cluster.sync();  // no block leaves while its copies to others are under way
 }
 
 // ---------------------------------------------------------------------------
