@@ -226,7 +226,9 @@ __host__ __device__ constexpr int br_min_blocks(int logn, int variant, int loge)
 // RADIX4: the transforms' radix-4 passes use the fused form (three products and a
 // shift per two levels, ntt_block.cuh) instead of radix-2 butterflies: a runtime
 // choice per context (tp_br_set_radix), built for one CTA per rotation.
-template <int LOGN, int VARIANT, int LOGE, int DL = 0, int LOGS = 0, bool RADIX4 = false>
+// LOGY: log2 of the CTAs that the key is laid out for (a wider cluster reads the same key: CTA r
+// takes its threads' words out of the part that holds its slots).
+template <int LOGN, int VARIANT, int LOGE, int DL = 0, int LOGS = 0, bool RADIX4 = false, int LOGY = LOGS>
 __global__ void __launch_bounds__((1 << (LOGN - LOGS)) >> LOGE, br_min_blocks(LOGN - LOGS, VARIANT, LOGE))
 br_kernel(const BrKernelParams prm) {
     constexpr int LOGL = LOGN - LOGS;        // log2 of the coefficients / slots per CTA
@@ -247,6 +249,8 @@ br_kernel(const BrKernelParams prm) {
     constexpr bool PF = !DS && br_key_prefetch(LOGN, VARIANT, LOGE, LOGS, R4);
     static_assert(!DS || (LOGE == 2 && K == 1), "the digit stage runs with 4 coefficients per thread");
     static_assert(LOGS == 0 || (LOGE == 2 && K == 1 && !R4), "clusters run radix-2 with 4 coefficients per thread");
+    constexpr int NY = N >> LOGY, TY = NY / E;  // slots and threads of one part of the key's layout
+    static_assert(LOGY <= LOGS, "a CTA's slots lie in one part of the key's layout");
     constexpr int NF = (R4 ? kNttRadix4 : 0) | (br_table_passes(VARIANT, DS, LOGL) ? kNttTablePasses : 0);
 
     extern __shared__ __align__(16) uint64_t smem[];
@@ -355,8 +359,9 @@ br_kernel(const BrKernelParams prm) {
             } else {
                 if (a0 == 0) continue;                               // cggi_blind_rotation.cpp:369-370
             }
-            // this CTA's part of the group's key rows (row stride C*N, part offset C*NL*cr)
-            const uint64_t* kit = prm.key + (uint64_t)(i / step) * (2ull * L * N * C) + (uint64_t)cr * (C * NL);
+            // this CTA's slots in the group's key rows (row stride C*N, part stride C*NY)
+            const uint64_t* kit = prm.key + (uint64_t)(i / step) * (2ull * L * N * C) +
+                                  (uint64_t)(sbase / NY) * (C * NY) + (sbase % NY) / E * 2;
 
             // MAC accumulators (canonical: every update is a gl_fma); the digit-staged
             // form sums per slot pair after the digit loop instead
@@ -405,7 +410,7 @@ br_kernel(const BrKernelParams prm) {
 #pragma unroll
                         for (int jp = 0; jp < E / 2; ++jp) {
                             const int ko = ((c * (E / 2) + jp) * T + t) * 2;
-                            cp_async16(kst + ko, kr + ko);
+                            cp_async16(kst + ko, kr + ((c * (E / 2) + jp) * TY + t) * 2);
                         }
                     cp_async_commit();
                 }
@@ -473,7 +478,8 @@ br_kernel(const BrKernelParams prm) {
                                 const int ko = ((c * (E / 2) + jp) * T + t) * 2;
                                 const ulonglong2 kv = (PF && K == 1)
                                                           ? *reinterpret_cast<const ulonglong2*>(kst + ko)
-                                                          : __ldg(reinterpret_cast<const ulonglong2*>(kr + ko));
+                                                          : __ldg(reinterpret_cast<const ulonglong2*>(
+                                                                kr + ((c * (E / 2) + jp) * TY + t) * 2));
                                 o[c][2 * jp] = gl_fma(o[c][2 * jp], x[p][2 * jp], kv.x);
                                 o[c][2 * jp + 1] = gl_fma(o[c][2 * jp + 1], x[p][2 * jp + 1], kv.y);
                             }
@@ -522,7 +528,7 @@ br_kernel(const BrKernelParams prm) {
                 constexpr int AH = br_ds_ahead(VARIANT, LOGL);
                 auto kaddr = [&](int jp, int c, int r) {
                     return reinterpret_cast<const ulonglong2*>(kit + (uint64_t)r * (N * C) +
-                                                               ((c * (E / 2) + jp) * T + t) * 2);
+                                                               ((c * (E / 2) + jp) * TY + t) * 2);
                 };
                 auto row_x = [&](int jp, int r) -> ulonglong2 {
                     return r < R2 - 1 ? *reinterpret_cast<const ulonglong2*>(xs + r * NL + (jp * T + t) * 2)

@@ -22,8 +22,8 @@ tp_status set_error(tp_status s, const char* fmt, ...);
 // (split 1, 2, 4); 0 when that kernel is not available for the context.
 uint64_t br_concurrency(const tp_br_ctx* c, int split);
 
-// Blocks of a launch of `batch` rotations when it runs in a double-precision form (which the
-// split asked for does not change); 0 when the modular forms run.
+// Blocks of a launch of `batch` rotations when it runs in a double-precision form or on a wider
+// cluster than a large ring's default (which the split asked for does not change); 0 otherwise.
 uint64_t br_fft_blocks(const tp_br_ctx* c, uint64_t batch);
 
 // CTAs (SMs) one rotation occupies with one block per rotation: 1, or the cluster

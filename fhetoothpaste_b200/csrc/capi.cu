@@ -233,6 +233,7 @@ struct tp_br_ctx {
         size_t smem = 0;
         int cap = 0;
     };
+    Form wide[2];                 // N > 4096: clusters of 2^(logs + 1 + i) CTAs (cap in clusters)
     Form r4_row, r4_ds;           // the fused radix-4 one-block kernels (row by row, digit-staged)
     const void* pair_kernel = nullptr;
     size_t pair_smem = 0;
@@ -264,9 +265,9 @@ struct tp_br_ctx {
 // row-by-row kernel (the default) and, for 3 or 4 digits where it fits, the
 // digit-staged one; 4 coefficients per thread, no split kernels.
 static tp_status br_setup_cluster(tp_br_ctx* c) {
-    const int S = 1 << c->logs;
-    const uint32_t T = c->prm.ring_dim >> (c->logs + 2);
-    auto probe = [&](const void* k, size_t smem, int* cap) -> bool {
+    auto probe = [&](const void* k, size_t smem, int logs, int* cap) -> bool {
+        const int S = 1 << logs;
+        const uint32_t T = c->prm.ring_dim >> (logs + 2);
         if (!k || smem > 227u * 1024u) return false;
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e == cudaSuccess && S > 8) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -295,9 +296,9 @@ static tp_status br_setup_cluster(tp_br_ctx* c) {
     const void* k = tp::br_kernel_lookup(c->logn, c->prm.variant, 2, 0);
     const size_t smem = tp::br_smem_words(c->logn, c->prm.variant, c->prm.lwe_dim, 2, 0, c->logs) * 8;
     int cap = 0;
-    if (!probe(k, smem, &cap))
+    if (!probe(k, smem, c->logs, &cap))
         return fail(TP_ERR_PARAM, "the %d-CTA cluster rotation kernel does not fit (N=%u, n=%u, smem=%zu) on device %d",
-                    S, c->prm.ring_dim, c->prm.lwe_dim, smem, c->device);
+                    1 << c->logs, c->prm.ring_dim, c->prm.lwe_dim, smem, c->device);
     c->kernels[2] = k;
     c->smem[2] = smem;
     c->grid_caps[2] = cap;
@@ -307,7 +308,7 @@ static tp_status br_setup_cluster(tp_br_ctx* c) {
         const size_t sd =
             tp::br_smem_words(c->logn, c->prm.variant, c->prm.lwe_dim, 2, (int)c->prm.digits, c->logs) * 8;
         int capd = 0;
-        if (probe(kd, sd, &capd)) {
+        if (probe(kd, sd, c->logs, &capd)) {
             // selectable, not the default (with 2048 coefficients per CTA the row-by-row form
             // measured faster on a cluster: N = 8192, ternary n = 1024, 670 vs 600 rotations/s);
             // the clusters of 4096 coefficients per CTA built now have no digit-staged kernel
@@ -315,6 +316,12 @@ static tp_status br_setup_cluster(tp_br_ctx* c) {
             c->ds_smem = sd;
             c->ds_cap = capd;
         }
+    }
+    for (int i = 0; i < 2; ++i) {
+        auto& f = c->wide[i];
+        f.k = tp::br_wide_kernel_lookup(c->logn, c->prm.variant, c->logs + 1 + i);
+        f.smem = tp::br_smem_words(c->logn, c->prm.variant, c->prm.lwe_dim, 2, 0, c->logs + 1 + i) * 8;
+        if (!probe(f.k, f.smem, c->logs + 1 + i, &f.cap)) f.cap = 0;
     }
     return TP_OK;
 }
@@ -438,6 +445,19 @@ static int br_form(const tp_br_ctx* c, uint64_t batch) {
     const int polys = 2 * c->G * 2 * (int)c->prm.digits * c->fft_limbs;
     const bool full = c->logn >= 11 || batch > (uint64_t)c->fft_cap / 2;
     return c->fftp.k && (polys >= 128 || (polys >= 64 && full)) ? kFftPair : kFftOneBlock;
+}
+
+// log2 of the CTAs per rotation of a ring above 4096: the widest cluster that takes the batch in
+// one wave, unless a launch form was set by name. Half as many coefficients per CTA leave the key
+// stream and the transforms half as long for the price of one more exchange partner, and the
+// 4096-coefficient plan's spills go; a wave of smaller clusters leaves more of the GPU idle once
+// the batch outgrows it. Milliseconds of one wave, 2^12, l = 3 (up to 15 / 33 / 74 rotations):
+//   N = 8192, n = 64:  8 / 4 / 2 CTAs  ternary 1.9 / 2.8 / 5.4  binary 1.7 / 2.4 / 4.4  BMMP 1.2 / 1.8 / 3.4
+//   N = 16384, n = 32: 8 / 4 CTAs      ternary 1.6 / 2.9        binary 1.4 / 2.5        BMMP 1.1 / 1.8
+static int br_ring_logs(const tp_br_ctx* c, uint64_t batch) {
+    for (int i = 1; i >= 0; --i)
+        if (c->fft_on && batch <= (uint64_t)c->wide[i].cap) return c->logs + 1 + i;
+    return c->logs;
 }
 
 extern "C" {
@@ -2926,6 +2946,7 @@ int br_cluster_ctas(const tp_br_ctx* c) { return c ? 1 << c->logs : 1; }
 
 uint64_t br_fft_blocks(const tp_br_ctx* c, uint64_t batch) {
     const int i = c ? br_form(c, batch) : kModular;
+    if (const int logs = c ? br_ring_logs(c, batch) : 0; c && logs > c->logs) return batch << logs;
     if (i > kFftHalves) return 0;
     if (i == kFftHalves) return 2 * std::min<uint64_t>(batch, c->fft_cap);
     if (i == kFftPair) return 2 * std::min<uint64_t>((batch + 1) / 2, c->fftp.cap);
@@ -3015,27 +3036,28 @@ tp_status br_batch_launch(tp_br_ctx* c, uint64_t batch, uint64_t* results, const
         tp::note_launch();
         return TP_OK;
     }
-    const bool ds = br_uses_ds(c);
-    const unsigned grid = (unsigned)std::min<uint64_t>(batch, br_one_block(c).cap);
     if (c->logs > 0) {
         // one rotation per cluster of 2^logs CTAs
+        const int logs = br_ring_logs(c, batch);
+        const tp_br_ctx::Form f = logs > c->logs ? c->wide[logs - c->logs - 1] : br_one_block(c);
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr = {};
         attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = 1u << c->logs;
+        attr.val.clusterDim.x = 1u << logs;
         attr.val.clusterDim.y = 1;
         attr.val.clusterDim.z = 1;
-        cfg.gridDim = dim3(grid << c->logs);
-        cfg.blockDim = dim3(c->prm.ring_dim >> (c->logs + 2));
-        cfg.dynamicSmemBytes = ds ? c->ds_smem : c->smem[2];
+        cfg.gridDim = dim3((unsigned)std::min<uint64_t>(batch, f.cap) << logs);
+        cfg.blockDim = dim3(c->prm.ring_dim >> (logs + 2));
+        cfg.dynamicSmemBytes = f.smem;
         cfg.stream = (cudaStream_t)stream;
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
-        TP_CUDA(cudaLaunchKernelExC(&cfg, ds ? c->ds_kernel : c->kernels[2], args));
+        TP_CUDA(cudaLaunchKernelExC(&cfg, f.k, args));
         tp::note_launch();
         return TP_OK;
     }
     const tp_br_ctx::Form f = br_one_block(c);
+    const unsigned grid = (unsigned)std::min<uint64_t>(batch, f.cap);
     TP_CUDA(cudaLaunchKernel(f.k, dim3(grid), dim3(c->prm.ring_dim >> c->loge), args, f.smem, (cudaStream_t)stream));
     tp::note_launch();
     return TP_OK;

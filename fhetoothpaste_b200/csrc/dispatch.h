@@ -18,6 +18,8 @@ const void* br_kernel_ptr_13(int variant, int loge, int dl, bool r4);
 const void* br_kernel_ptr_14(int variant, int loge, int dl, bool r4);
 const void* br_kernel_ptr_15(int variant, int loge, int dl, bool r4);
 const void* br_kernel_ptr_16(int variant, int loge, int dl, bool r4);
+const void* br_wide_kernel_ptr_13(int variant, int logs);
+const void* br_wide_kernel_ptr_14(int variant, int logs);
 const void* ntt_kernel_ptr_12(bool forward);
 const void* ntt_kernel_ptr_13(bool forward);  // cluster kernels (ntt_cluster_kernel)
 const void* ntt_kernel_ptr_14(bool forward);
@@ -56,6 +58,16 @@ inline const void* br_kernel_lookup(int logn, int variant, int loge, int dl = 0,
         case 14: return br_kernel_ptr_14(variant, loge, dl, r4);
         case 15: return br_kernel_ptr_15(variant, loge, dl, r4);
         case 16: return br_kernel_ptr_16(variant, loge, dl, r4);
+        default: return nullptr;
+    }
+}
+
+// Rotation kernel of a ring above 4096 on a cluster of 2^logs CTAs, more than the default, on the
+// default's key layout (nullptr where not built).
+inline const void* br_wide_kernel_lookup(int logn, int variant, int logs) {
+    switch (logn) {
+        case 13: return br_wide_kernel_ptr_13(variant, logs);
+        case 14: return br_wide_kernel_ptr_14(variant, logs);
         default: return nullptr;
     }
 }

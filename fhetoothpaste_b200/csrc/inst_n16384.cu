@@ -21,6 +21,14 @@ const void* br_kernel_ptr_14(int variant, int loge, int dl, bool r4) {
     }
 }
 
+const void* br_wide_kernel_ptr_14(int variant, int logs) {
+    if (logs == 3)
+        return variant == kCggiBinary    ? (const void*)br_kernel<14, kCggiBinary, 2, 0, 3, false, 2>
+               : variant == kCggiTernary ? (const void*)br_kernel<14, kCggiTernary, 2, 0, 3, false, 2>
+                                         : (const void*)br_kernel<14, kBmmpBinary, 2, 0, 3, false, 2>;
+    return nullptr;
+}
+
 const void* ks_kernel_ptr_14(int mode, int loge) {
     if (loge != 2) return nullptr;  // clusters run with 4 coefficients per thread
     switch (mode) {

@@ -21,6 +21,18 @@ const void* br_kernel_ptr_13(int variant, int loge, int dl, bool r4) {
     }
 }
 
+const void* br_wide_kernel_ptr_13(int variant, int logs) {
+    if (logs == 2)
+        return variant == kCggiBinary    ? (const void*)br_kernel<13, kCggiBinary, 2, 0, 2, false, 1>
+               : variant == kCggiTernary ? (const void*)br_kernel<13, kCggiTernary, 2, 0, 2, false, 1>
+                                         : (const void*)br_kernel<13, kBmmpBinary, 2, 0, 2, false, 1>;
+    if (logs == 3)
+        return variant == kCggiBinary    ? (const void*)br_kernel<13, kCggiBinary, 2, 0, 3, false, 1>
+               : variant == kCggiTernary ? (const void*)br_kernel<13, kCggiTernary, 2, 0, 3, false, 1>
+                                         : (const void*)br_kernel<13, kBmmpBinary, 2, 0, 3, false, 1>;
+    return nullptr;
+}
+
 const void* ks_kernel_ptr_13(int mode, int loge) {
     if (loge != 2) return nullptr;  // clusters run with 4 coefficients per thread
     switch (mode) {
