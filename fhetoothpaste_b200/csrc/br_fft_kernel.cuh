@@ -679,18 +679,27 @@ br_fft_pair_kernel(const __grid_constant__ BrFftParams prm) {
 // blocks whose digits need them. Every block takes part in each exchange that another block's
 // next step waits for, so an area's next contents are sent only after its last reads: digits i + 1
 // follow words i of all blocks, which follow their products i, and so on round the cycle.
+// N = 4096, n = 60, one rotation on eight blocks against two: ternary l = 3 1.66 -> 0.74 ms,
+// binary l = 4 1.44 -> 0.75.
 // ---------------------------------------------------------------------------
 __host__ __device__ constexpr int br_fft_cluster_polys(int dl, int limbs, int cs) {
     return (2 * (dl > limbs ? dl : limbs) + cs - 1) / cs;
 }
-__host__ __device__ constexpr int br_fft_cluster_threads(int logn, int limbs) { return (1 << (logn - 4)) * limbs; }
+// A thread multiplies the slots lane + m LANES of one limb: n/8 lanes, at N = 4096 n/16 (512
+// threads keep 128 registers each).
+__host__ __device__ constexpr int br_fft_cluster_lanes(int logn) { return 1 << (logn - (logn > 11 ? 5 : 4)); }
+__host__ __device__ constexpr int br_fft_cluster_threads(int logn, int limbs) { return br_fft_cluster_lanes(logn) * limbs; }
+// At N = 4096 (eight blocks, one polynomial each) a block keeps only the accumulator half and the
+// words that its digit is of, and reads the pass tables through L1.
+__host__ __device__ constexpr int br_fft_cluster_halves(int logn) { return logn > 11 ? 1 : 2; }
 // Forward and backward buffers (PP polynomials each), digit slots (2l n/CS), limb and word
 // areas (2L n/CS, also the products on their way out; 2n), accumulator (2n), words on their way out
 // (2 n/CS), pass tables, monomial factors, barriers, LWE words.
 __host__ __device__ constexpr size_t br_fft_cluster_smem(int logn, int dl, int limbs, int cs, uint32_t n) {
     const size_t k = (size_t)1 << (logn - 1);
-    return (2 * br_fft_cluster_polys(dl, limbs, cs) * k + (2 * dl + 2 * limbs + 2) * (k / cs) + 4 * k +
-            2 * fft_table_len(logn - 1) + 10) * 16 + (((size_t)n + 4) / 4) * 16;
+    const int halves = br_fft_cluster_halves(logn);
+    return (2 * br_fft_cluster_polys(dl, limbs, cs) * k + (2 * dl + 2 * limbs + 2) * (k / cs) + 2 * halves * k +
+            (halves == 2 ? 2 * fft_table_len(logn - 1) : 0) + 10) * 16 + (((size_t)n + 4) / 4) * 16;
 }
 
 template <int LOGN, int VARIANT, int DL, int L, int CS>
@@ -702,14 +711,17 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
     constexpr int N = 1 << LOGN, n = F::n, TG = F::T;
     constexpr int G = br_rgsw_per_group(VARIANT);
     constexpr int C = 2 * G, R = 2 * DL;
-    constexpr int LANES = n / 8, T = LANES * L, M = 8 / CS, NS = n / CS;
+    constexpr int LANES = br_fft_cluster_lanes(LOGN), T = LANES * L, NS = n / CS, M = NS / LANES;
+    constexpr int KL = n / 8, KM = 8 / CS, SUB = KL / LANES;  // the key's lanes, its m per block, m here per key m
     constexpr int PP = br_fft_cluster_polys(DL, L, CS);
+    constexpr int H = br_fft_cluster_halves(LOGN);            // accumulator halves kept
     constexpr uint32_t MASK2N = 2u * N - 1u;
     constexpr bool SIGNED = VARIANT != kCggiBinary;
     // products and limbs as bulk copies, or (fewer blocks, more words to each) as remote stores behind
     // a cluster barrier
     constexpr bool BULK = CS == 8, WORDS = CS == 8 || LOGN == 10;
     static_assert(8 % CS == 0 && PP * TG <= T - 32, "block shape");
+    static_assert(H == 2 || (CS == 8 && PP == 1), "one half: one polynomial per block");
 
     extern __shared__ __align__(16) uint64_t smem[];
     double2* work = reinterpret_cast<double2*>(smem);                  // PP n
@@ -717,11 +729,10 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
     double2* dig = inv + PP * n;                                       // R NS
     ulonglong2* lim = reinterpret_cast<ulonglong2*>(dig + R * NS);     // 2L NS
     ulonglong2* gb = lim + 2 * L * NS;                                 // 2 n
-    ulonglong2* acc = gb + 2 * n;                                      // 2 n: plus corr (signed)
-    ulonglong2* gs = acc + 2 * n;                                      // 2 NS
-    double2* tab_f = reinterpret_cast<double2*>(gs + 2 * NS);
-    double2* tab_i = tab_f + fft_table_len(LOGK);
-    double2* mono_s = tab_i + fft_table_len(LOGK);
+    ulonglong2* acc = gb + H * n;                                      // H n: plus corr (signed)
+    ulonglong2* gs = acc + H * n;                                      // 2 NS
+    double2* tabs = reinterpret_cast<double2*>(gs + 2 * NS);
+    double2* mono_s = tabs + (H == 2 ? 2 * fft_table_len(LOGK) : 0);
     uint64_t* bar = reinterpret_cast<uint64_t*>(mono_s + 8);           // [4]: digits, products, limbs, words have come
     uint32_t* lwe_s = reinterpret_cast<uint32_t*>(mono_s + 10);
 
@@ -730,10 +741,17 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
     const int t = threadIdx.x;
     const int grp = t / TG, tg = t % TG;
     const int limb = t / LANES, lane = t % LANES;
-    for (int i = t; i < fft_table_len(LOGK); i += T) {
-        tab_f[i] = prm.tab_fwd[i];
-        tab_i[i] = prm.tab_inv[i];
+    const double2* tab_f = prm.tab_fwd;
+    const double2* tab_i = prm.tab_inv;
+    if constexpr (H == 2) {
+        for (int i = t; i < fft_table_len(LOGK); i += T) {
+            tabs[i] = prm.tab_fwd[i];
+            tabs[fft_table_len(LOGK) + i] = prm.tab_inv[i];
+        }
+        tab_f = tabs;
+        tab_i = tabs + fft_table_len(LOGK);
     }
+    auto half = [](int h) { return H == 2 ? h * n : 0; };  // where half h starts in acc and gb
     // blocks whose forward polynomials are digits of half h
     auto first_of = [](int h) { return h * DL / PP; };
     auto last_of = [](int h) { return (h * DL + DL - 1) / PP; };
@@ -763,8 +781,9 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
             // acc = acc_in X^b, plus the signed digits' corrector
             const uint64_t* ain = prm.accs + b * prm.acc_stride;
             const uint32_t s = (2u * N - lwe_s[prm.n]) & MASK2N;
-            for (int u = t; u < 2 * n; u += T) {
-                const uint64_t* a = ain + (u >> LOGK) * N;
+            const int h0 = H == 2 || c < DL ? 0 : 1;  // the half kept (H = 1)
+            for (int u = t; u < H * n; u += T) {
+                const uint64_t* a = ain + (h0 + (u >> LOGK)) * N;
                 ulonglong2 v = rot_pair<LOGK>(
                     [&](uint32_t j) { return make_ulonglong2(gl_canon(a[j]), gl_canon(a[j + n])); }, u & (n - 1), s);
                 if constexpr (SIGNED) v = make_ulonglong2(gl_add(v.x, prm.corr), gl_add(v.y, prm.corr));
@@ -774,10 +793,10 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
         cluster.sync();  // every block has read the accumulator before one writes its result over it
 
         auto prefetch = [&](uint32_t it) {  // this block's slots of an iteration's key, one thread per limb
-            constexpr uint32_t per = (uint32_t)R * C * LANES * 16;
+            constexpr uint32_t per = (uint32_t)R * C * KL * 16;
             const uint32_t l = (uint32_t)(t - (T - 32));  // of a warp that has no transform
             if (it < prm.n && l < L)
-                l2_prefetch(reinterpret_cast<const char*>(prm.key) + (((uint64_t)it * L + l) * 8 + c * M) * per, M * per);
+                l2_prefetch(reinterpret_cast<const char*>(prm.key) + (((uint64_t)it * L + l) * 8 + c * KM) * per, KM * per);
         };
         prefetch(0);
         prefetch(1);
@@ -801,14 +820,14 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
 #pragma unroll
                 for (int h = 0; h < 2; ++h)
                     if (c >= first_of(h) && c <= last_of(h))
-                        for (int u = t; u < n; u += T) gb[h * n + u] = rotated_difference<LOGK>(acc, h * n + u, a);
+                        for (int u = t; u < n; u += T) gb[half(h) + u] = rotated_difference<LOGK>(acc, half(h) + u, a);
                 src = gb;
                 __syncthreads();
             }
             if (grp < PP && p < R) {
                 const int h = p / DL, d = p - h * DL;
                 double2 x[16];
-                digit_points<LOGK>(x, src + h * n, tg, prm.dshift[d], (uint32_t)prm.dmask[d],
+                digit_points<LOGK>(x, src + half(h), tg, prm.dshift[d], (uint32_t)prm.dmask[d],
                                    4503599627370496.0 + (SIGNED ? (double)prm.ddelta[d] : 0.0));
                 F::head(x, prm.head);
                 double2* pb = work + grp * n;
@@ -819,25 +838,32 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
                 bulk_fence();
                 F::group_sync(grp);
                 if (tg < CS) bulk_to_block(dig + p * NS, pb + tg * NS, NS * 16, bar, (uint32_t)tg);
-            } else if (VARIANT == kCggiTernary && t >= T - M) {
-                const int mm = t - (T - M);
-                mono_s[mm] = __ldg(prm.roots + ((4u * a * (__brev((uint32_t)(c * M + mm)) >> 29)) & MASK2N));
+            } else if (VARIANT == kCggiTernary && t >= T - KM) {
+                const int km = t - (T - KM);
+                mono_s[km] = __ldg(prm.roots + ((4u * a * (__brev((uint32_t)(c * KM + km)) >> 29)) & MASK2N));
             }
 
             // ---- slot-wise products; slots lane + (c M + mm) LANES, one limb ----
-            constexpr int BR = C == 4 ? (R % 3 == 0 ? 3 : 2) : (R % 4 == 0 ? 4 : R), NB = M * R / BR;
-            const double2* kp = prm.key + ((((uint64_t)it * L + limb) * 8 + c * M) * (R * C)) * LANES + lane;
+            // the key's lane of mm is lane + (mm % SUB) LANES, its m is c KM + mm / SUB
+            constexpr int BR = H == 1 ? 2 : C == 4 ? (R % 3 == 0 ? 3 : 2) : (R % 4 == 0 ? 4 : R), NB = M * R / BR;
+            const double2* kp = prm.key + ((((uint64_t)it * L + limb) * 8 + c * KM) * (R * C)) * KL + lane;
             double2 kv[2][BR][C];
             auto load = [&](int q, double2 (&k)[BR][C]) {
 #pragma unroll
                 for (int r = 0; r < BR; ++r)
 #pragma unroll
-                    for (int cc = 0; cc < C; ++cc) k[r][cc] = key_ld(kp + ((q * BR + r) * C + cc) * LANES);
+                    for (int cc = 0; cc < C; ++cc) {
+                        const int mm = q * BR / R, row = q * BR % R + r;
+                        k[r][cc] = key_ld(kp + ((mm / SUB * R + row) * C + cc) * KL + mm % SUB * LANES);
+                    }
             };
             load(0, kv[0]);
-            double2 wb = make_double2(1.0, 0.0);
-            if constexpr (VARIANT == kCggiTernary)
-                wb = __ldg(prm.roots + ((a * (1u + 32u * (__brev((uint32_t)lane) >> (35 - LOGK)))) & MASK2N));
+            double2 wb[SUB];
+            if constexpr (VARIANT == kCggiTernary) {
+#pragma unroll
+                for (int q = 0; q < SUB; ++q)
+                    wb[q] = __ldg(prm.roots + ((a * (1u + 32u * (__brev((uint32_t)(lane + q * LANES)) >> (35 - LOGK)))) & MASK2N));
+            }
             __syncthreads();
             ok = ok && mbar_wait(bar, phase);
             double2 s[C];
@@ -858,7 +884,7 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
                 if ((q + 1) * BR % R != 0) continue;
                 double2 v[2] = {s[0], s[1]};
                 if constexpr (VARIANT == kCggiTernary) {
-                    const double2 w = cmul(wb, mono_s[mm]);
+                    const double2 w = cmul(wb[mm % SUB], mono_s[mm / SUB]);
 #pragma unroll
                     for (int h = 0; h < 2; ++h) v[h] = csubmul(s[h], w, s[C - 2 + h]);
                 }
@@ -918,7 +944,7 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
                 if constexpr (WORDS) gs[u] = gw;
                 else
                     for (int q = first_of(h); q <= last_of(h); ++q)
-                        cluster.map_shared_rank(gb, (unsigned)q)[h * n + c * NS + u % NS] = gw;
+                        cluster.map_shared_rank(gb, (unsigned)q)[half(h) + c * NS + u % NS] = gw;
             }
             if constexpr (WORDS) {
                 bulk_fence();
@@ -929,7 +955,7 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
             if (WORDS && t < 2 * CS) {
                 const int h = t / CS, q = t % CS;
                 if (q >= first_of(h) && q <= last_of(h))
-                    bulk_to_block(gb + h * n + c * NS, gs + h * NS, NS * 16, bar + 3, (uint32_t)q);
+                    bulk_to_block(gb + half(h) + c * NS, gs + h * NS, NS * 16, bar + 3, (uint32_t)q);
             }
 
             // ---- accumulator halves of this block ----
@@ -938,14 +964,14 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 if (c < first_of(h) || c > last_of(h)) continue;
-                const ulonglong2* gh = gb + h * n;
+                const ulonglong2* gh = gb + half(h);
                 for (int u = t; u < n; u += T) {
-                    const ulonglong2 v = acc[h * n + u], g = gh[u];
+                    const ulonglong2 v = acc[half(h) + u], g = gh[u];
                     if constexpr (VARIANT == kCggiBinary) {
-                        acc[h * n + u] = make_ulonglong2(gl_add(v.x, g.x), gl_add(v.y, g.y));
+                        acc[half(h) + u] = make_ulonglong2(gl_add(v.x, g.x), gl_add(v.y, g.y));
                     } else {
                         const ulonglong2 w = rot_pair<LOGK>([&](uint32_t j) { return gh[j]; }, u, a);
-                        acc[h * n + u] = make_ulonglong2(gl_add(v.x, gl_sub(w.x, g.x)), gl_add(v.y, gl_sub(w.y, g.y)));
+                        acc[half(h) + u] = make_ulonglong2(gl_add(v.x, gl_sub(w.x, g.x)), gl_add(v.y, gl_sub(w.y, g.y)));
                     }
                 }
             }
@@ -957,7 +983,7 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
         for (int h = 0; h < 2; ++h) {
             if (c != last_of(h)) continue;
             for (int u = t; u < n; u += T) {
-                ulonglong2 v = acc[h * n + u];
+                ulonglong2 v = acc[half(h) + u];
                 if constexpr (SIGNED) v = make_ulonglong2(gl_sub(v.x, prm.corr), gl_sub(v.y, prm.corr));
                 res[h * N + u] = v.x;
                 res[h * N + u + n] = v.y;
@@ -975,8 +1001,8 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
 // and transforms, rounds and recombines the L limb polynomials of its half, so that only slots
 // cross: half of the digits' as bulk copies, half of the products as stores. The pass tables are
 // read through L1 (no shared memory is left for them). 74 clusters are resident; ternary, l = 3, n
-// = 60: 74 rotations 4.01 -> 1.58 ms, 148 4.02 -> 3.2, one 3.96 -> 2.49 (modular -> here). Key
-// batches 1 / 2 / 3 ahead: 1.70 / 1.66 / 1.58 ms.
+// = 60: 74 rotations 4.01 -> 1.58 ms, 148 4.02 -> 3.2 (modular -> here). Key batches 1 / 2 / 3
+// ahead: 1.70 / 1.66 / 1.58 ms. Up to 15 rotations run on eight blocks each, above.
 // ---------------------------------------------------------------------------
 __host__ __device__ constexpr int br_fft_halves_threads(int logn, int limbs) { return (1 << (logn - 5)) * limbs; }
 // Transform buffers (L polynomials), receive area (l half polynomials), accumulator half, monomial

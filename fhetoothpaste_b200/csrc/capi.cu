@@ -386,8 +386,7 @@ static void br_setup_fft(tp_br_ctx* c) {
         c->fft_kernel = k;
         c->fft_smem = smem;
         c->fft_cap = halves ? per_sm : per_sm * sm_count(c->device);
-        if (halves) return;
-        {
+        if (!halves) {
             auto& f = c->fftp;
             const void* kp = tp::br_fft_pair_ptr(c->logn, c->prm.variant, c->prm.digits, limbs);
             f.smem = tp::br_fft_pair_smem(c->logn, (int)c->prm.digits, limbs, c->prm.lwe_dim);
@@ -420,8 +419,8 @@ static void br_setup_fft(tp_br_ctx* c) {
 
 // The form of a launch of `batch` rotations whose context left the choice open: clusters of
 // 2^(i + 1) blocks per rotation in double precision (i = 0 .. 2), one block (kFftOneBlock) or two
-// rotations on two blocks (kFftPair) in double precision (at N = 4096 always one rotation on two
-// blocks, kFftHalves), or the modular kernels (kModular,
+// rotations on two blocks (kFftPair) in double precision (at N = 4096 one rotation on eight blocks
+// or on two, kFftHalves), or the modular kernels (kModular,
 // kModularPair: two blocks per rotation). Milliseconds at n = 60, one wave each (15, 30, 74
 // clusters, 148 rotations) and 600 rotations:
 //                                  clusters 8 / 4 / 2    one block   pair        modular, pair
@@ -438,9 +437,9 @@ static void br_setup_fft(tp_br_ctx* c) {
 enum { kFftOneBlock = 3, kFftPair = 4, kFftHalves = 5, kModularPair = 6, kModular = 7 };
 static int br_form(const tp_br_ctx* c, uint64_t batch) {
     if (!c->fft_ready || !c->fft_on) return kModular;
-    if (c->logn == 12) return kFftHalves;
     for (int i = 2; i >= 0; --i)
         if (batch <= (uint64_t)c->fftc[i].cap) return i;
+    if (c->logn == 12) return kFftHalves;
     if (c->logn >= 11 && c->loge == 2 && batch <= (uint64_t)c->pair_cap) return kModularPair;
     const int polys = 2 * c->G * 2 * (int)c->prm.digits * c->fft_limbs;
     const bool full = c->logn >= 11 || batch > (uint64_t)c->fft_cap / 2;

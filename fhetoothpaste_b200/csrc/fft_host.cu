@@ -149,6 +149,11 @@ const void* pick_cluster(int logn, uint32_t digits, int limbs, int cs) {
         return cs == 2   ? pick_cluster<10, VARIANT, 2>(digits, limbs)
                : cs == 4 ? pick_cluster<10, VARIANT, 4>(digits, limbs)
                          : pick_cluster<10, VARIANT, 8>(digits, limbs);
+    if (logn == 12 && cs == 8 && limbs == 4)
+        return digits == 2   ? (const void*)br_fft_cluster_kernel<12, VARIANT, 2, 4, 8>
+               : digits == 3 ? (const void*)br_fft_cluster_kernel<12, VARIANT, 3, 4, 8>
+               : digits == 4 ? (const void*)br_fft_cluster_kernel<12, VARIANT, 4, 4, 8>
+                             : nullptr;
     if (logn == 11 && cs >= 4)
         return cs == 4 ? pick_cluster<11, VARIANT, 4>(digits, limbs) : pick_cluster<11, VARIANT, 8>(digits, limbs);
     return nullptr;
