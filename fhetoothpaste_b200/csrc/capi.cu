@@ -434,9 +434,23 @@ static void br_setup_fft(tp_br_ctx* c) {
 // its one wave; then one block, or the pair where the key polynomials read per slot and iteration
 // (2 G rows limbs) reach 64 and halving them pays for the exchanges (at N = 1024, where two
 // blocks share an SM, from the second block per SM on, or from 128).
-enum { kFftOneBlock = 3, kFftPair = 4, kFftHalves = 5, kModularPair = 6, kModular = 7 };
+//
+// Sets without a double-precision kernel: four blocks per rotation in one wave up to half the SMs
+// (beyond, where several clusters share an SM, two blocks are as fast), two in one wave, else one.
+// Milliseconds at n = 60, one wave:
+//                                  4 blocks (32)  2 blocks (74)  1 block (148)
+//   BMMP N = 2048, l = 4           0.63           0.87           1.13
+//   BMMP N = 1024, l = 4           0.34           0.48           0.65
+//   ternary N = 512, l = 3         0.40           0.45           0.56
+//   BMMP N = 4096, l = 3           -              1.59           2.63
+enum { kFftOneBlock = 3, kFftPair = 4, kFftHalves = 5, kModularQuad = 6, kModularPair = 7, kModular = 8 };
 static int br_form(const tp_br_ctx* c, uint64_t batch) {
-    if (!c->fft_ready || !c->fft_on) return kModular;
+    if (!c->fft_on) return kModular;
+    if (!c->fft_ready) {
+        if (c->loge != 2 || c->logs > 0) return kModular;
+        if (batch <= (uint64_t)c->quad_cap && 2 * batch <= (uint64_t)sm_count(c->device)) return kModularQuad;
+        return batch <= (uint64_t)c->pair_cap ? kModularPair : kModular;
+    }
     for (int i = 2; i >= 0; --i)
         if (batch <= (uint64_t)c->fftc[i].cap) return i;
     if (c->logn == 12) return kFftHalves;
@@ -2952,6 +2966,26 @@ uint64_t br_fft_blocks(const tp_br_ctx* c, uint64_t batch) {
     return i < kFftOneBlock ? batch << (i + 1) : std::min<uint64_t>(batch, c->fft_cap);
 }
 
+// Rotations of a batch that run in `form` before the rest gets a launch of its own: the full waves,
+// where the rest fits a wave of a wider form, which is shorter than one more wave of this one.
+// 0: one launch. Milliseconds, n = 60 (a wave, the rest in the same form, in its own):
+//   BMMP N = 2048, l = 4, 512 = 3 x 148 + 68: 1.13, 1.12, 0.87
+//   ternary N = 8192 (n = 64), 100 = 74 + 26: 5.37, 5.40, 2.70
+//   ternary N = 2048, l = 3, 160 = 148 + 12: 1.04, 1.0, 0.41
+static uint64_t br_head(const tp_br_ctx* c, int form, uint64_t batch) {
+    uint64_t wave = 0;
+    if (form == kFftOneBlock) wave = (uint64_t)c->fft_cap;
+    if (form == kFftPair) wave = 2ull * c->fftp.cap;
+    if (form == kModular && c->fft_on) wave = (uint64_t)br_one_block(c).cap;
+    if (wave == 0 || batch <= wave || batch % wave == 0) return 0;
+    const uint64_t rest = batch % wave;
+    const int f = br_form(c, rest);
+    const bool wider = form != kModular ? f < kFftOneBlock
+                       : c->logs > 0    ? br_ring_logs(c, rest) > c->logs
+                                        : f == kModularPair || f == kModularQuad;
+    return wider ? batch - rest : 0;
+}
+
 uint64_t br_concurrency(const tp_br_ctx* c, int split) {
     if (!c) return 0;
     if (split == 2) return c->loge == 2 ? (uint64_t)c->pair_cap : 0;
@@ -2971,6 +3005,14 @@ tp_status br_batch_launch(tp_br_ctx* c, uint64_t batch, uint64_t* results, const
     if (((uintptr_t)results & 15) || ((uintptr_t)accs & 7) || ((uintptr_t)lwes & 7))
         return fail(TP_ERR_PARAM, "results must be 16-byte aligned, lwes/accs 8-byte aligned");
     const int form = br_form(c, batch);
+    if (split == 0)
+        if (const uint64_t head = br_head(c, form, batch)) {
+            const tp_status s = br_batch_launch(c, head, results, lwes, lwe_stride, accs, acc_stride, out_coef, stream, 0);
+            return s != TP_OK ? s
+                              : br_batch_launch(c, batch - head, results + head * 2 * c->prm.ring_dim,
+                                                lwes + head * lwe_stride, lwe_stride, accs + head * acc_stride,
+                                                acc_stride, out_coef, stream, 0);
+        }
     if (form <= kFftHalves) {
         TP_CUDA(cudaSetDevice(c->device));
         tp::BrFftParams fp{};
@@ -3013,7 +3055,7 @@ tp_status br_batch_launch(tp_br_ctx* c, uint64_t batch, uint64_t* results, const
         tp::note_launch();
         return out_coef ? TP_OK : ntt_launch(c->prm.ring_dim, 2 * batch, results, results, stream, true);
     }
-    if (split == 0) split = form == kModularPair ? 2 : c->split;
+    if (split == 0) split = form == kModularPair ? 2 : form == kModularQuad ? 4 : c->split;
     if (split == 4 && br_concurrency(c, 4) == 0) split = 2;
     if (split == 2 && br_concurrency(c, 2) == 0) split = 1;
     TP_CUDA(cudaSetDevice(c->device));
