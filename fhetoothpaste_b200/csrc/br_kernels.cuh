@@ -57,7 +57,7 @@ struct BrKernelParams {
     uint64_t dmask[8];        // per-digit mask
     uint64_t ddelta[8];       // per-digit offset subtracted (signed) or 0 (unsigned)
     unsigned int* err;        // bit 0: an LWE word was outside [0, 2N)
-    uint32_t small_digits;    // every digit is at most 2^14 in magnitude: integer pass 0 (tile 4)
+    uint32_t small_digits;    // SmallDigits: integer pass 0 where the digits allow it (tile 4)
 };
 
 // Polynomials transformed together by the rotation kernel (the accumulator
@@ -430,11 +430,8 @@ br_kernel(const BrKernelParams prm) {
                         const uint32_t d = r < L ? r : r - L;
                         const uint32_t sh = prm.dshift[d];
                         const uint64_t mk = prm.dmask[d];
-                        const int64_t dl = SIGNED ? (int64_t)prm.ddelta[d] : 0;
-                        int64_t dv[4];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) dv[j] = (int64_t)((cx[0][j] >> sh) & mk) - dl;
-                        ntt_pass0_small(dv, reinterpret_cast<uint64_t(&)[4]>(x[0]));
+                        ntt_pass0_digit(reinterpret_cast<uint64_t(&)[4]>(cx[0]), sh, mk, SIGNED ? prm.ddelta[d] : 0,
+                                        prm.small_digits, reinterpret_cast<uint64_t(&)[4]>(x[0]));
                         pass0_done = true;
                     }
                 }

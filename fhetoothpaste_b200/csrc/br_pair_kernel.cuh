@@ -221,12 +221,17 @@ __device__ __forceinline__ void br_split_body(const BrKernelParams& prm) {
                 const uint32_t sh = prm.dshift[d];
                 const uint64_t mk = prm.dmask[d];
                 const uint64_t dl = prm.ddelta[d];
+                if (LOGE == 2 && prm.small_digits) {
+                    if constexpr (LOGE == 2) ntt_pass0_digit(cx[0], sh, mk, SIGNED ? dl : 0, prm.small_digits, x[0]);
+                } else {
 #pragma unroll
-                for (int j = 0; j < E; ++j) {
-                    const uint64_t raw = (cx[0][j] >> sh) & mk;
-                    x[0][j] = SIGNED ? gl_sub(raw, dl) : raw;
+                    for (int j = 0; j < E; ++j) {
+                        const uint64_t raw = (cx[0][j] >> sh) & mk;
+                        x[0][j] = SIGNED ? gl_sub(raw, dl) : raw;
+                    }
+                    fwd_pass_math<LOGN, 0, 1, LOGE, R4, true>(x, t, tw_f);
                 }
-                ntt_forward_k<LOGN, 1, LOGE, R4, true>(x, t, xb(), tw_f);
+                ntt_forward_after_pass0<LOGN, 1, LOGE, R4, true>(x, t, xb(), tw_f);
                 if constexpr (PF) cp_async_wait_all();
 #pragma unroll
                 for (int c = 0; c < C; ++c)

@@ -197,6 +197,12 @@ void signed_digit_consts(int beta, uint32_t digits, uint64_t& corr, uint32_t* ds
     }
 }
 
+// Digits of at most `bits` bits of magnitude for the integer pass 0 of the digit transforms: signed
+// ones lie in [-2^(beta-1), 2^(beta-1)), unsigned ones in [0, 2^beta).
+uint32_t small_digits(int bits) {
+    return bits <= 14 ? tp::kDigits14 : bits <= 15 ? tp::kDigits15 : tp::kDigitsLarge;
+}
+
 uint32_t inv_mod_2n(uint32_t t, uint32_t two_n) {
     for (uint32_t x = 1; x < two_n; x += 2)
         if ((uint64_t)x * t % two_n == 1) return x;
@@ -570,9 +576,7 @@ tp_status tp_br_create(const tp_br_params* p, int device, tp_br_ctx** out) {
         }
     }
 
-    // Digits small enough for the integer pass 0 of the digit transforms: signed digits lie in
-    // [-2^(beta-1), 2^(beta-1)), unsigned in [0, 2^beta); the pass is exact up to 2^14.
-    kp.small_digits = (p->variant == TP_BR_CGGI_BINARY ? beta <= 14 : beta <= 15) ? 1u : 0u;
+    kp.small_digits = small_digits(p->variant == TP_BR_CGGI_BINARY ? beta : beta - 1);
     if (c->logs > 0) {
         tp_status cs = br_setup_cluster(c);
         if (cs != TP_OK) {
@@ -1273,6 +1277,7 @@ static tp_status ks_create(int kind, uint32_t ring_dim, uint64_t basis, uint32_t
     kp.digits = digits;
     kp.n_inv = c->tab->n_inv;
     signed_digit_consts(beta, digits, kp.corr, kp.dshift, kp.dmask, kp.ddelta);
+    kp.small_digits = small_digits(beta - 1);
     c->smem = tp::ks_smem_words((int)ring_dim, 1 << c->logs) * 8;
     if (c->logs > 0) {
         // one item per cluster of 2^logs CTAs, 4 coefficients per thread

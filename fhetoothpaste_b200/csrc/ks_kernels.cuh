@@ -39,6 +39,7 @@ struct KsKernelParams {
     uint64_t out_stride;      // words between items' outputs
     uint64_t right_offset;    // kKsMerge: words from left node to right node; kKsSplit: to the second child
     uint32_t digits;
+    uint32_t small_digits;    // SmallDigits: integer pass 0 (4 coefficients per thread)
     uint32_t auto_index;      // t (odd)
     uint32_t auto_index_inv;  // t^-1 mod 2N
     uint32_t shift;           // kKsMerge: X^shift rotation of the left node; kKsSplit: X^-shift of the difference
@@ -109,8 +110,6 @@ __device__ __forceinline__ void ks_mac(uint64_t (&a)[1 << LOGE], const KsKernelP
         const uint64_t mk = prm.dmask[d];
         const uint64_t dl = prm.ddelta[d];
         uint64_t x[1][E];
-#pragma unroll
-        for (int j = 0; j < E; ++j) x[0][j] = gl_sub((a[j] >> sh) & mk, dl);
         const uint64_t* kr = prm.key + (uint64_t)d * (2 * N) + (uint64_t)cr * (2 * NL);
         // with 4 coefficients per thread the digit's key words (8 registers) are
         // requested before its NTT, which hides their L2 latency; with 8 they
@@ -123,7 +122,15 @@ __device__ __forceinline__ void ks_mac(uint64_t (&a)[1 << LOGE], const KsKernelP
                 for (int jp = 0; jp < E / 2; ++jp)
                     kv[c][jp] = __ldg(reinterpret_cast<const ulonglong2*>(kr + ((c * (E / 2) + jp) * T + t) * 2));
         }
-        ntt_forward_k<LOGL, 1, LOGE, false, true>(x, t, sel ? buf1 : buf0, tw_f);
+        if (LOGE == 2 && prm.small_digits) {
+            // digits as small integers, levels 0 and 1 in integer arithmetic
+            if constexpr (LOGE == 2) ntt_pass0_digit(a, sh, mk, dl, prm.small_digits, x[0]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < E; ++j) x[0][j] = gl_sub((a[j] >> sh) & mk, dl);
+            fwd_pass_math<LOGL, 0, 1, LOGE, 0, true>(x, t, tw_f);
+        }
+        ntt_forward_after_pass0<LOGL, 1, LOGE, 0, true>(x, t, sel ? buf1 : buf0, tw_f);
         sel ^= 1;
         if constexpr (LOGS > 0) {
             uint64_t* rv = *rsel ? recv1 : recv0;
