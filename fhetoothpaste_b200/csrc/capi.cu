@@ -18,6 +18,7 @@
 #include "br_fft_kernel.cuh"
 #include "fft_host.h"
 #include "ks_fft_kernel.cuh"
+#include "ks_rlwe_kernel.cuh"
 #include "misc_kernels.cuh"
 #include "util_kernels.cuh"
 #include "ks_kernels.cuh"
@@ -1199,6 +1200,8 @@ struct tp_ks_ctx {
     uint64_t* zero = nullptr;          // 2N zero words
     // double-precision form of the modes with coefficient results (packing contexts, N = 1024 and
     // 2048), where one is built and every key passes its exactness bound; off once a tile is set
+    const void* rlwe_kernel = nullptr;  // digit-staged RLWE switch, runs unless a tile was set by name
+    int rlwe_cap = 0;
     const void* fft_kernel = nullptr;
     int fft_limbs = 0, fft_cap = 0;
     const tp::FftTables* fft_tab = nullptr;
@@ -1326,6 +1329,18 @@ static tp_status ks_create(int kind, uint32_t ring_dim, uint64_t basis, uint32_t
         }
     }
     ks_setup_fft(c);
+    if (const void* k = kind == 0 ? tp::ks_rlwe_kernel_ptr(c->logn, digits) : nullptr) {
+        const size_t smem = tp::ks_rlwe_smem_words(c->logn, (int)digits) * 8;
+        int per_sm = 0;
+        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, ring_dim >> 2, smem);
+        if (e == cudaSuccess && per_sm > 0) {
+            c->rlwe_kernel = k;
+            c->rlwe_cap = per_sm * sm_count(device);
+        } else {
+            cudaGetLastError();  // clear the optional probe's error
+        }
+    }
     *out = c;
     return TP_OK;
 }
@@ -1427,6 +1442,13 @@ static tp_status ks_launch(tp_ks_ctx* c, int mode, const tp::KsKernelParams& kp,
         TP_CUDA(cudaLaunchKernel(c->fft_kernel, dim3((unsigned)std::min<uint64_t>(kp.items, c->fft_cap)),
                                  dim3(tp::ks_fft_threads(c->logn, c->fft_limbs)), fargs,
                                  tp::ks_fft_smem(c->logn, c->fft_limbs), st));
+        tp::note_launch();
+        return TP_OK;
+    }
+    if (mode == tp::kKsRlwe && c->rlwe_kernel && c->fft_on && (((uintptr_t)kp.in | (uintptr_t)kp.out) & 15) == 0) {
+        // its 16-byte accesses need the alignment; two to four digits, N = 1024 .. 4096
+        TP_CUDA(cudaLaunchKernel(c->rlwe_kernel, dim3((unsigned)std::min<uint64_t>(kp.items, c->rlwe_cap)),
+                                 dim3(c->N >> 2), args, tp::ks_rlwe_smem_words(c->logn, (int)c->digits) * 8, st));
         tp::note_launch();
         return TP_OK;
     }

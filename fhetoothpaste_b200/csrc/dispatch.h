@@ -1,6 +1,8 @@
 // Kernel lookup across the per-ring-size compilation units.
 #pragma once
 
+#include <stdint.h>
+
 namespace tp {
 
 const void* br_kernel_ptr_7(int variant, int loge, int dl, bool r4);
@@ -31,6 +33,8 @@ const void* br_pair_kernel_ptr_9(int variant, int split);
 const void* br_pair_kernel_ptr_10(int variant, int split);
 const void* br_pair_kernel_ptr_11(int variant, int split);
 const void* br_pair_kernel_ptr_12(int variant, int split);
+// Digit-staged RLWE key switch (ks_rlwe_kernel.cuh; nullptr where not built).
+const void* ks_rlwe_kernel_ptr(int logn, uint32_t digits);
 const void* ks_kernel_ptr_7(int mode, int loge);
 const void* ks_kernel_ptr_8(int mode, int loge);
 const void* ks_kernel_ptr_9(int mode, int loge);

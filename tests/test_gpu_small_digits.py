@@ -45,3 +45,31 @@ def test_rotation(native, oracle, variant, N, beta, digits, split):
     accs = words(rng, beta, 3, 2 * N)
     got = rot.blind_rotate_batch_host(lwes, accs, out_coef=True)
     np.testing.assert_array_equal(got, oracle.blind_rotate_many(variant, N, n, beta, digits, key, lwes, accs, True, 3))
+
+
+# two to four digits with and without integer first levels; more items than resident blocks; unaligned and in place
+@pytest.mark.parametrize("N,beta,digits", [(1024, 16, 4), (1024, 20, 3), (2048, 16, 4), (2048, 8, 2), (4096, 12, 3), (4096, 20, 3)])
+def test_staged_switch_equals_the_general_kernel(native, N, beta, digits):
+    import torch
+    from fhetoothpaste_b200 import GpuRLWEtoRLWEConverter
+    rng = np.random.default_rng(N + digits)
+    key = rng.integers(0, P, digits * 2 * N, dtype=np.uint64)
+    conv, ref = (GpuRLWEtoRLWEConverter(N, 1 << beta, digits, key) for _ in range(2))
+    ref.set_tile(4)  # a tile set by name runs the general kernel
+    batch = 148 * (4096 // N) + 3
+    x = torch.from_numpy(rng.integers(0, P, (batch, 2 * N), dtype=np.uint64).view(np.int64)).cuda()
+    base = torch.from_numpy(rng.integers(0, P, (batch, 2 * N), dtype=np.uint64).view(np.int64)).cuda()
+    for items in (1, batch):
+        want, got = base.clone(), base.clone()
+        ref.convert_batch(items, want.data_ptr(), x.data_ptr())
+        conv.convert_batch(items, got.data_ptr(), x.data_ptr())
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
+    odd = torch.zeros(batch * 2 * N + 1, dtype=torch.int64, device="cuda")
+    odd[1:] = base.flatten()
+    conv.convert_batch(batch, odd.data_ptr() + 8, x.data_ptr())
+    same, named = x.clone(), x.clone()
+    conv.convert_batch(batch, same.data_ptr(), same.data_ptr())
+    ref.convert_batch(batch, named.data_ptr(), named.data_ptr())
+    torch.cuda.synchronize()
+    assert torch.equal(odd[1:].view(batch, 2 * N), want) and torch.equal(same, named)
