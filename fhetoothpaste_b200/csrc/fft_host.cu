@@ -43,7 +43,7 @@ __device__ __forceinline__ Dd dd_mul(Dd a, Dd b) {
 }
 __device__ __forceinline__ Dd dd_neg(Dd a) { return {-a.h, -a.l}; }
 
-// One block per key polynomial: each limb transformed by radix-2 levels in shared memory
+// One block per limb of a key polynomial, transformed by radix-2 levels in shared memory
 // in double-double arithmetic (relative error near 2^-100), so that the stored doubles
 // carry one rounding. Run once per key upload; bound by FP64 (about 150 operations a
 // butterfly): 15120 polynomials of N = 2048 (three limbs) take a few milliseconds against
@@ -57,7 +57,9 @@ __global__ void __launch_bounds__(256) fft_key_kernel(double2* __restrict__ dst,
     const uint32_t n = 1u << logk, lanes = n >> 3;
     const int64_t base = fft_limb_base(limbs);
     const double scale = 1.0 / (double)n;
-    for (uint64_t p = blockIdx.x; p < polys; p += gridDim.x) {
+    for (uint64_t item = blockIdx.x; item < polys * limbs; item += gridDim.x) {
+        const uint64_t p = item / limbs;
+        const int l = (int)(item % limbs);
         const uint64_t* a = src + p * (2ull * n);
         const uint64_t id = first + p;
         const uint32_t h = (uint32_t)(id & 1), C = 2 * G;
@@ -65,55 +67,53 @@ __global__ void __launch_bounds__(256) fft_key_kernel(double2* __restrict__ dst,
         const uint32_t r = (uint32_t)(rig % rows);
         const uint32_t g = (uint32_t)((rig / rows) % G);
         const uint64_t it = rig / rows / G;
-        for (int l = 0; l < limbs; ++l) {
-            // limb l, balanced, of the word's representative in (-p/2, p/2)
-            auto limb = [&](uint64_t x) -> int64_t {
-                int64_t v = x > kP / 2 ? -(int64_t)(kP - x) : (int64_t)x;
-                for (int q = 0;; ++q) {
-                    if (q == limbs - 1) return v;
-                    int64_t d = v % base;
-                    if (d > base / 2) d -= base;
-                    if (d < -(base / 2)) d += base;
-                    if (q == l) return d;
-                    v = (v - d) / base;
-                }
-            };
-            unsigned long long sq = 0;
-            __syncthreads();  // the previous limb's points are stored
-            for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
-                const int64_t x = limb(a[j]), y = limb(a[j + n]);
-                sq += (unsigned long long)(x * x) + (unsigned long long)(y * y);
-                z[j] = make_double4((double)x, 0.0, (double)y, 0.0);
+        // limb l, balanced, of the word's representative in (-p/2, p/2)
+        auto limb = [&](uint64_t x) -> int64_t {
+            int64_t v = x > kP / 2 ? -(int64_t)(kP - x) : (int64_t)x;
+            for (int q = 0;; ++q) {
+                if (q == limbs - 1) return v;
+                int64_t d = v % base;
+                if (d > base / 2) d -= base;
+                if (d < -(base / 2)) d += base;
+                if (q == l) return d;
+                v = (v - d) / base;
             }
-            for (int lg = 0; lg < logk; ++lg) {
-                __syncthreads();
-                const uint32_t m = 1u << lg, half = n >> (lg + 1);
-                for (uint32_t q = threadIdx.x; q < n / 2; q += blockDim.x) {
-                    const uint32_t b = q / half, i0 = (q & (half - 1)) + b * 2 * half, i1 = i0 + half;
-                    const double4 w = tw[m + b], u = z[i0], v = z[i1];
-                    const Dd wr{w.x, w.y}, wi{w.z, w.w}, vr{v.x, v.y}, vi{v.z, v.w}, ur{u.x, u.y}, ui{u.z, u.w};
-                    const Dd pr = dd_add(dd_mul(wr, vr), dd_neg(dd_mul(wi, vi)));
-                    const Dd pi = dd_add(dd_mul(wr, vi), dd_mul(wi, vr));
-                    const Dd ar = dd_add(ur, pr), ai = dd_add(ui, pi);
-                    const Dd br = dd_add(ur, dd_neg(pr)), bi = dd_add(ui, dd_neg(pi));
-                    z[i0] = make_double4(ar.h, ar.l, ai.h, ai.l);
-                    z[i1] = make_double4(br.h, br.l, bi.h, bi.l);
-                }
-            }
+        };
+        unsigned long long sq = 0;
+        __syncthreads();  // the previous limb's points are stored
+        for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
+            const int64_t x = limb(a[j]), y = limb(a[j + n]);
+            sq += (unsigned long long)(x * x) + (unsigned long long)(y * y);
+            z[j] = make_double4((double)x, 0.0, (double)y, 0.0);
+        }
+        for (int lg = 0; lg < logk; ++lg) {
             __syncthreads();
-            double2* out = dst + (it * limbs + l) * (8ull * rows * C * lanes);
-            for (uint32_t e = threadIdx.x; e < n; e += blockDim.x) {
-                const uint32_t m = e / lanes, lane = e & (lanes - 1);
-                out[((uint64_t)(m * rows + r) * C + (2 * g + h)) * lanes + lane] =
-                    make_double2(z[e].x * scale, z[e].z * scale);
+            const uint32_t m = 1u << lg, half = n >> (lg + 1);
+            for (uint32_t q = threadIdx.x; q < n / 2; q += blockDim.x) {
+                const uint32_t b = q / half, i0 = (q & (half - 1)) + b * 2 * half, i1 = i0 + half;
+                const double4 w = tw[m + b], u = z[i0], v = z[i1];
+                const Dd wr{w.x, w.y}, wi{w.z, w.w}, vr{v.x, v.y}, vi{v.z, v.w}, ur{u.x, u.y}, ui{u.z, u.w};
+                const Dd pr = dd_add(dd_mul(wr, vr), dd_neg(dd_mul(wi, vi)));
+                const Dd pi = dd_add(dd_mul(wr, vi), dd_mul(wi, vr));
+                const Dd ar = dd_add(ur, pr), ai = dd_add(ui, pi);
+                const Dd br = dd_add(ur, dd_neg(pr)), bi = dd_add(ui, dd_neg(pi));
+                z[i0] = make_double4(ar.h, ar.l, ai.h, ai.l);
+                z[i1] = make_double4(br.h, br.l, bi.h, bi.l);
             }
-            for (int o = 16; o; o >>= 1) sq += __shfl_xor_sync(0xFFFFFFFFu, sq, o);
-            if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sq;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                for (int w = 1; w < 8; ++w) sq += part[w];
-                atomicMax(norm2, sq);
-            }
+        }
+        __syncthreads();
+        double2* out = dst + (it * limbs + l) * (8ull * rows * C * lanes);
+        for (uint32_t e = threadIdx.x; e < n; e += blockDim.x) {
+            const uint32_t m = e / lanes, lane = e & (lanes - 1);
+            out[((uint64_t)(m * rows + r) * C + (2 * g + h)) * lanes + lane] =
+                make_double2(z[e].x * scale, z[e].z * scale);
+        }
+        for (int o = 16; o; o >>= 1) sq += __shfl_xor_sync(0xFFFFFFFFu, sq, o);
+        if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = sq;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < 8; ++w) sq += part[w];
+            atomicMax(norm2, sq);
         }
     }
 }
@@ -297,7 +297,8 @@ void fft_key_launch(double2* dst, const uint64_t* src, uint64_t polys, uint64_t 
     const size_t smem = sizeof(double4) << tab.logk;  // 32 KB at 1024 points
     if (smem > 48u * 1024u)
         cudaFuncSetAttribute(fft_key_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    const unsigned blocks = (unsigned)(polys < 4096 ? polys : 4096);
+    const uint64_t items = polys * limbs;
+    const unsigned blocks = (unsigned)(items < 4096 ? items : 4096);
     fft_key_kernel<<<blocks, 256, smem, st>>>(dst, src, polys, first, G, rows, tab.logk, limbs, tab.dd, norm2);
 }
 
