@@ -45,6 +45,7 @@ struct BrFftParams {
     uint64_t dmask[8];
     uint64_t ddelta[8];
     unsigned int* err;
+    const unsigned int* exact;  // recorded launches: runs only while *exact is not 0 (the key passes the bound)
     FftHead head;
 };
 
@@ -195,6 +196,7 @@ br_fft_kernel(const __grid_constant__ BrFftParams prm) {
     constexpr uint32_t MASK2N = 2u * N - 1u;
     constexpr bool SIGNED = VARIANT != kCggiBinary;
 
+    if (prm.exact && !*prm.exact) return;
     extern __shared__ __align__(16) uint64_t smem[];
     double2* buf = reinterpret_cast<double2*>(smem);                   // P n
     ulonglong2* acc = reinterpret_cast<ulonglong2*>(buf + P * n);      // 2 n: plus corr (signed)
@@ -434,6 +436,7 @@ br_fft_pair_kernel(const __grid_constant__ BrFftParams prm) {
     constexpr uint32_t MASK2N = 2u * N - 1u;
     constexpr bool SIGNED = VARIANT != kCggiBinary;
 
+    if (prm.exact && !*prm.exact) return;
     extern __shared__ __align__(16) uint64_t smem[];
     double2* buf = reinterpret_cast<double2*>(smem);                   // P n
     double2* recv = buf + P * n;                                       // R n/2: the other rotation's digits
@@ -723,6 +726,7 @@ br_fft_cluster_kernel(const __grid_constant__ BrFftParams prm) {
     static_assert(8 % CS == 0 && PP * TG <= T - 32, "block shape");
     static_assert(H == 2 || (CS == 8 && PP == 1), "one half: one polynomial per block");
 
+    if (prm.exact && !*prm.exact) return;
     extern __shared__ __align__(16) uint64_t smem[];
     double2* work = reinterpret_cast<double2*>(smem);                  // PP n
     double2* inv = work + PP * n;                                      // PP n
@@ -1027,6 +1031,7 @@ br_fft_halves_kernel(const __grid_constant__ BrFftParams prm) {
     constexpr bool SIGNED = VARIANT != kCggiBinary;
     static_assert(DL <= L && TG * L == T && LANES * L == T, "block shape");
 
+    if (prm.exact && !*prm.exact) return;
     extern __shared__ __align__(16) uint64_t smem[];
     double2* buf = reinterpret_cast<double2*>(smem);                     // L n
     double2* recv = buf + L * n;                                         // DL n/2: the other half's digits

@@ -58,6 +58,7 @@ struct BrKernelParams {
     uint64_t ddelta[8];       // per-digit offset subtracted (signed) or 0 (unsigned)
     unsigned int* err;        // bit 0: an LWE word was outside [0, 2N)
     uint32_t small_digits;    // SmallDigits: integer pass 0 where the digits allow it (tile 4)
+    const unsigned int* exact;  // recorded behind a double-precision launch: runs only while *exact is 0
 };
 
 // Polynomials transformed together by the rotation kernel (the accumulator
@@ -253,6 +254,7 @@ br_kernel(const BrKernelParams prm) {
     static_assert(LOGY <= LOGS, "a CTA's slots lie in one part of the key's layout");
     constexpr int NF = (R4 ? kNttRadix4 : 0) | (br_table_passes(VARIANT, DS, LOGL) ? kNttTablePasses : 0);
 
+    if (prm.exact && *prm.exact) return;
     extern __shared__ __align__(16) uint64_t smem[];
     uint64_t* base = smem;
     const uint64_t* tw_f = prm.tw_fwd;

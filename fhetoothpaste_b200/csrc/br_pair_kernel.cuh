@@ -98,6 +98,7 @@ __device__ __forceinline__ void br_split_body(const BrKernelParams& prm) {
     constexpr bool PF = br_pair_key_prefetch(LOGN, VARIANT, S);
     constexpr bool TW_SMEM = br_pair_smem_twiddles(LOGN, VARIANT, LOGE, S);
 
+    if (prm.exact && *prm.exact) return;
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = (int)cluster.block_rank();
     const int h = rank & 1;   // accumulator half and gadget rows of this CTA

@@ -35,6 +35,7 @@
 namespace tp {
 static std::atomic<uint64_t> g_launches{0};
 static thread_local int t_capturing = 0;
+static thread_local uint64_t t_standby = 0;  // recorded kernels that leave their work to the one before them
 static void note_launch() {
     if (!t_capturing) g_launches.fetch_add(1, std::memory_order_relaxed);
 }
@@ -162,6 +163,13 @@ tp_status get_tables(int device, int logn, Tables** out) {
     return TP_OK;
 }
 
+// Whether work on `stream` is being recorded into a graph.
+bool recording(void* stream) {
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing((cudaStream_t)stream, &s) != cudaSuccess) cudaGetLastError();  // the launch reports it
+    return s == cudaStreamCaptureStatusActive;
+}
+
 int sm_count(int device) {
     int v = 0;
     cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, device);
@@ -222,7 +230,9 @@ struct tp_br_ctx {
     Tables* tab = nullptr;
     uint64_t* key = nullptr;      // device layout
     bool key_ready = false;
-    unsigned int* err = nullptr;  // device error word
+    unsigned int* err = nullptr;  // device words: errors, then `exact` and `norm2`
+    unsigned int* exact = nullptr;         // device copy of fft_ready, read by recorded launches
+    unsigned long long* norm2 = nullptr;   // largest squared norm of a limb polynomial of the key
     tp::BrKernelParams kp{};
     int loge = 3;                 // log2 coefficients per thread of the active tile
     const void* kernels[4] = {};  // by loge (2, 3)
@@ -262,6 +272,7 @@ struct tp_br_ctx {
     double2* fft_key = nullptr;
     bool fft_ready = false;       // the key is resident and exact in this form
     bool fft_on = true;
+    std::atomic<bool> fft_recorded{false};  // a recorded launch names fft_key
     // workspace for host-pointer calls
     uint64_t* ws = nullptr;
     uint64_t ws_words = 0;
@@ -451,13 +462,15 @@ static void br_setup_fft(tp_br_ctx* c) {
 //   ternary N = 512, l = 3         0.40           0.45           0.56
 //   BMMP N = 4096, l = 3           -              1.59           2.63
 enum { kFftOneBlock = 3, kFftPair = 4, kFftHalves = 5, kModularQuad = 6, kModularPair = 7, kModular = 8 };
+static int br_modular_form(const tp_br_ctx* c, uint64_t batch) {
+    if (c->loge != 2 || c->logs > 0) return kModular;
+    if (batch <= (uint64_t)c->quad_cap && 2 * batch <= (uint64_t)sm_count(c->device)) return kModularQuad;
+    return batch <= (uint64_t)c->pair_cap ? kModularPair : kModular;
+}
+static int br_form_split(int form) { return form == kModularPair ? 2 : form == kModularQuad ? 4 : 1; }
 static int br_form(const tp_br_ctx* c, uint64_t batch) {
     if (!c->fft_on) return kModular;
-    if (!c->fft_ready) {
-        if (c->loge != 2 || c->logs > 0) return kModular;
-        if (batch <= (uint64_t)c->quad_cap && 2 * batch <= (uint64_t)sm_count(c->device)) return kModularQuad;
-        return batch <= (uint64_t)c->pair_cap ? kModularPair : kModular;
-    }
+    if (!c->fft_ready) return br_modular_form(c, batch);
     for (int i = 2; i >= 0; --i)
         if (batch <= (uint64_t)c->fftc[i].cap) return i;
     if (c->logn == 12) return kFftHalves;
@@ -525,12 +538,15 @@ tp_status tp_br_create(const tp_br_params* p, int device, tp_br_ctx** out) {
         delete c;
         return s;
     }
-    e = cudaMalloc(&c->err, sizeof(unsigned int));
-    if (e == cudaSuccess) e = cudaMemset(c->err, 0, sizeof(unsigned int));
+    e = cudaMalloc(&c->err, 4 * sizeof(unsigned int));
+    if (e == cudaSuccess) e = cudaMemset(c->err, 0, 4 * sizeof(unsigned int));
     if (e != cudaSuccess) {
+        cudaFree(c->err);
         delete c;
         return fail(TP_ERR_CUDA, "error word: %s", cudaGetErrorString(e));
     }
+    c->exact = c->err + 1;
+    c->norm2 = reinterpret_cast<unsigned long long*>(c->err + 2);
 
     // Decomposition constants.
     tp::BrKernelParams& kp = c->kp;
@@ -702,22 +718,18 @@ tp_status tp_br_upload_key(tp_br_ctx* c, const uint64_t* brk, uint64_t words) {
     uint64_t* stage = nullptr;
     TP_CUDA(cudaMalloc(&stage, 2 * chunk * per_group * 8));
     tp_status st = TP_OK;
-    // the limbs' transforms (one double2 per two words and limb), where there is room for them
-    unsigned long long* norm2 = nullptr;
+    // the limbs' transforms (one double2 per two words and limb), where there is room for them; once
+    // there, every key is transformed: recorded launches read them
+    cudaError_t e = cudaMemset(c->exact, 0, 3 * sizeof(unsigned int));  // and norm2
     bool fft = c->fft_kernel != nullptr;
     c->fft_ready = false;
-    if (fft) {
-        cudaError_t e = cudaMalloc(&norm2, sizeof *norm2);
-        if (e == cudaSuccess) e = cudaMemset(norm2, 0, sizeof *norm2);
-        if (e == cudaSuccess && !c->fft_key) e = cudaMalloc(&c->fft_key, c->key_words * 8 * c->fft_limbs);
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            fft = false;
-        }
+    if (fft && !c->fft_key && cudaMalloc(&c->fft_key, c->key_words * 8 * c->fft_limbs) != cudaSuccess) {
+        cudaGetLastError();
+        fft = false;
     }
     cudaStream_t copy = nullptr, work = nullptr;  // ordered with the legacy stream, not with each other
     cudaEvent_t copied[2] = {}, done[2] = {};
-    cudaError_t e = cudaStreamCreate(&copy);
+    if (e == cudaSuccess) e = cudaStreamCreate(&copy);
     if (e == cudaSuccess) e = cudaStreamCreate(&work);
     for (int q = 0; q < 2 && e == cudaSuccess; ++q) {
         e = cudaEventCreateWithFlags(&copied[q], cudaEventDisableTiming);
@@ -743,7 +755,7 @@ tp_status tp_br_upload_key(tp_br_ctx* c, const uint64_t* brk, uint64_t words) {
             tp::note_launch();
             st = ntt_launch((uint32_t)N, total / N, sg, sg, work, false);
             tp::fft_key_launch(c->fft_key, sg, total / N, g0 * c->G * 4 * c->prm.digits, c->G, 2 * c->prm.digits,
-                               c->fft_limbs, *c->fft_tab, norm2, work);
+                               c->fft_limbs, *c->fft_tab, c->norm2, work);
             tp::note_launch();
         }
         e = cudaGetLastError();
@@ -751,7 +763,13 @@ tp_status tp_br_upload_key(tp_br_ctx* c, const uint64_t* brk, uint64_t words) {
     }
     unsigned long long v = 0;
     if (e == cudaSuccess) e = cudaStreamSynchronize(work);
-    if (e == cudaSuccess && fft) e = cudaMemcpy(&v, norm2, sizeof v, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess && fft) e = cudaMemcpy(&v, c->norm2, sizeof v, cudaMemcpyDeviceToHost);
+    // Without it the modular forms run; the buffer stays, a recorded launch may still name it. What
+    // such a launch must not read is made unlike any key.
+    bool exact = e == cudaSuccess && st == TP_OK && fft && br_fft_key_exact(c, (double)v);
+    const unsigned int one = 1;
+    if (exact) e = cudaMemcpy(c->exact, &one, sizeof one, cudaMemcpyHostToDevice);
+    else if (c->fft_recorded) cudaMemset(c->fft_key, 0xFF, c->key_words * 8 * c->fft_limbs);
     if (e != cudaSuccess) st = fail(TP_ERR_CUDA, "key upload: %s", cudaGetErrorString(e));
     for (int i = 0; i < 2; ++i) {
         if (copied[i]) cudaEventDestroy(copied[i]);
@@ -760,9 +778,7 @@ tp_status tp_br_upload_key(tp_br_ctx* c, const uint64_t* brk, uint64_t words) {
     if (copy) cudaStreamDestroy(copy);
     if (work) cudaStreamDestroy(work);
     cudaFree(stage);  // waits for what an error left in flight
-    cudaFree(norm2);
-    // without it the modular forms run; the buffer stays, a recorded graph may still name it
-    c->fft_ready = st == TP_OK && fft && br_fft_key_exact(c, (double)v);
+    c->fft_ready = st == TP_OK && exact;
     if (st == TP_OK) c->key_ready = true;
     return st;
 }
@@ -1049,7 +1065,7 @@ struct tp_graph {
     cudaGraphExec_t exec = nullptr;
     uint8_t* ws = nullptr; // workspace that the graph's kernels use
     int device = 0;
-    uint64_t kernels = 0;  // kernel nodes of the graph: launches per replay
+    uint64_t kernels = 0;  // launches per replay: kernel nodes but those standing by
 };
 
 static uint64_t graph_kernel_nodes(cudaGraph_t g) {
@@ -1081,6 +1097,7 @@ tp_status tp_br_batch_graph_create(tp_br_ctx* c, uint64_t batch, uint64_t* resul
         return fail(TP_ERR_CUDA, "begin capture: %s", cudaGetErrorString(e));
     }
     ++tp::t_capturing;
+    tp::t_standby = 0;
     tp_status st = tp_br_blind_rotate_batch(c, batch, results, lwes, lwe_stride, accs, acc_stride, out_coef, s);
     if (st == TP_OK && extract_out) st = tp_sample_extract_batch(c->prm.ring_dim, batch, extract_out, results, s);
     --tp::t_capturing;
@@ -1094,7 +1111,7 @@ tp_status tp_br_batch_graph_create(tp_br_ctx* c, uint64_t batch, uint64_t* resul
     if (e != cudaSuccess) return fail(TP_ERR_CUDA, "end capture: %s", cudaGetErrorString(e));
     auto* gr = new tp_graph();
     gr->device = c->device;
-    gr->kernels = graph_kernel_nodes(g);
+    gr->kernels = graph_kernel_nodes(g) - tp::t_standby;
     e = cudaGraphInstantiate(&gr->exec, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) {
@@ -2215,6 +2232,7 @@ tp_status tp_pbs_graph_create(tp_br_ctx* br, tp_lwe_ks_ctx* ks, uint64_t batch, 
         return fail(TP_ERR_CUDA, "begin capture: %s", cudaGetErrorString(e));
     }
     ++tp::t_capturing;
+    tp::t_standby = 0;
     tp_status st = tp_br_blind_rotate_batch(br, batch, rlwe_scratch, lwes, (uint64_t)br->prm.lwe_dim + 1, accs,
                                             acc_stride, 1, s);
     if (st == TP_OK) st = pbs_epilogue(ks, batch, out_lwe, rlwe_scratch, 2ull * br->prm.ring_dim, ws, s);
@@ -2234,7 +2252,7 @@ tp_status tp_pbs_graph_create(tp_br_ctx* br, tp_lwe_ks_ctx* ks, uint64_t batch, 
     auto* gr = new tp_graph();
     gr->ws = ws;
     gr->device = br->device;
-    gr->kernels = graph_kernel_nodes(g);
+    gr->kernels = graph_kernel_nodes(g) - tp::t_standby;
     e = cudaGraphInstantiate(&gr->exec, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) {
@@ -3020,73 +3038,15 @@ uint64_t br_concurrency(const tp_br_ctx* c, int split) {
     return (uint64_t)br_one_block(c).cap;
 }
 
-tp_status br_batch_launch(tp_br_ctx* c, uint64_t batch, uint64_t* results, const uint64_t* lwes,
-                          uint64_t lwe_stride, const uint64_t* accs, uint64_t acc_stride, int out_coef, void* stream,
-                          int split) {
-    if (!c) return fail(TP_ERR_PARAM, "null context");
-    if (!c->key_ready) return fail(TP_ERR_STATE, "no key uploaded");
-    if (batch == 0) return TP_OK;
-    if (!results || !lwes || !accs) return fail(TP_ERR_PARAM, "null buffer");
-    if (lwe_stride < (uint64_t)c->prm.lwe_dim + 1) return fail(TP_ERR_PARAM, "lwe_stride below n+1");
-    if (acc_stride != 0 && acc_stride < 2ull * c->prm.ring_dim) return fail(TP_ERR_PARAM, "acc_stride below 2N");
-    if (((uintptr_t)results & 15) || ((uintptr_t)accs & 7) || ((uintptr_t)lwes & 7))
-        return fail(TP_ERR_PARAM, "results must be 16-byte aligned, lwes/accs 8-byte aligned");
-    const int form = br_form(c, batch);
-    if (split == 0)
-        if (const uint64_t head = br_head(c, form, batch)) {
-            const tp_status s = br_batch_launch(c, head, results, lwes, lwe_stride, accs, acc_stride, out_coef, stream, 0);
-            return s != TP_OK ? s
-                              : br_batch_launch(c, batch - head, results + head * 2 * c->prm.ring_dim,
-                                                lwes + head * lwe_stride, lwe_stride, accs + head * acc_stride,
-                                                acc_stride, out_coef, stream, 0);
-        }
-    if (form <= kFftHalves) {
-        TP_CUDA(cudaSetDevice(c->device));
-        tp::BrFftParams fp{};
-        fp.key = c->fft_key;
-        fp.tab_fwd = c->fft_tab->pass_fwd;
-        fp.tab_inv = c->fft_tab->pass_inv;
-        fp.roots = c->fft_tab->roots;
-        fp.lwes = lwes;
-        fp.lwe_stride = lwe_stride;
-        fp.accs = accs;
-        fp.acc_stride = acc_stride;
-        fp.out = results;
-        fp.batch = batch;
-        fp.n = c->prm.lwe_dim;
-        fp.corr = c->kp.corr;
-        memcpy(fp.dshift, c->kp.dshift, sizeof fp.dshift);
-        memcpy(fp.dmask, c->kp.dmask, sizeof fp.dmask);
-        memcpy(fp.ddelta, c->kp.ddelta, sizeof fp.ddelta);
-        fp.err = c->err;
-        fp.head = c->fft_tab->head;
-        void* fargs[] = {&fp};
-        if (const int i = form; i < kFftOneBlock) {
-            cudaLaunchAttribute attr;
-            const cudaLaunchConfig_t cfg =
-                br_fftc_config(c, i, (unsigned)std::min<uint64_t>(batch, c->fftc[i].cap), (cudaStream_t)stream, &attr);
-            TP_CUDA(cudaLaunchKernelExC(&cfg, c->fftc[i].k, fargs));
-        } else if (form == kFftHalves) {
-            TP_CUDA(cudaLaunchKernel(c->fft_kernel, dim3(2 * (unsigned)std::min<uint64_t>(batch, c->fft_cap)),
-                                     dim3(tp::br_fft_halves_threads(c->logn, c->fft_limbs)), fargs, c->fft_smem,
-                                     (cudaStream_t)stream));
-        } else if (form == kFftPair) {
-            TP_CUDA(cudaLaunchKernel(c->fftp.k, dim3(2 * (unsigned)std::min<uint64_t>((batch + 1) / 2, c->fftp.cap)),
-                                     dim3(tp::br_fft_threads(c->logn, (int)c->prm.digits, c->fft_limbs)), fargs,
-                                     c->fftp.smem, (cudaStream_t)stream));
-        } else {
-            TP_CUDA(cudaLaunchKernel(c->fft_kernel, dim3((unsigned)std::min<uint64_t>(batch, c->fft_cap)),
-                                     dim3(tp::br_fft_threads(c->logn, (int)c->prm.digits, c->fft_limbs)), fargs,
-                                     c->fft_smem, (cudaStream_t)stream));
-        }
-        tp::note_launch();
-        return out_coef ? TP_OK : ntt_launch(c->prm.ring_dim, 2 * batch, results, results, stream, true);
-    }
-    if (split == 0) split = form == kModularPair ? 2 : form == kModularQuad ? 4 : c->split;
+// The modular kernels, `split` blocks per rotation. `exact`: see BrKernelParams.
+static tp_status br_modular_launch(tp_br_ctx* c, uint64_t batch, uint64_t* results, const uint64_t* lwes,
+                                   uint64_t lwe_stride, const uint64_t* accs, uint64_t acc_stride, int out_coef,
+                                   void* stream, int split, const unsigned int* exact) {
     if (split == 4 && br_concurrency(c, 4) == 0) split = 2;
     if (split == 2 && br_concurrency(c, 2) == 0) split = 1;
     TP_CUDA(cudaSetDevice(c->device));
     BrKernelParams kp = c->kp;
+    kp.exact = exact;
     kp.key = c->key;
     kp.lwes = lwes;
     kp.lwe_stride = lwe_stride;
@@ -3129,6 +3089,85 @@ tp_status br_batch_launch(tp_br_ctx* c, uint64_t batch, uint64_t* results, const
     TP_CUDA(cudaLaunchKernel(f.k, dim3(grid), dim3(c->prm.ring_dim >> c->loge), args, f.smem, (cudaStream_t)stream));
     tp::note_launch();
     return TP_OK;
+}
+
+tp_status br_batch_launch(tp_br_ctx* c, uint64_t batch, uint64_t* results, const uint64_t* lwes,
+                          uint64_t lwe_stride, const uint64_t* accs, uint64_t acc_stride, int out_coef, void* stream,
+                          int split) {
+    if (!c) return fail(TP_ERR_PARAM, "null context");
+    if (!c->key_ready) return fail(TP_ERR_STATE, "no key uploaded");
+    if (batch == 0) return TP_OK;
+    if (!results || !lwes || !accs) return fail(TP_ERR_PARAM, "null buffer");
+    if (lwe_stride < (uint64_t)c->prm.lwe_dim + 1) return fail(TP_ERR_PARAM, "lwe_stride below n+1");
+    if (acc_stride != 0 && acc_stride < 2ull * c->prm.ring_dim) return fail(TP_ERR_PARAM, "acc_stride below 2N");
+    if (((uintptr_t)results & 15) || ((uintptr_t)accs & 7) || ((uintptr_t)lwes & 7))
+        return fail(TP_ERR_PARAM, "results must be 16-byte aligned, lwes/accs 8-byte aligned");
+    const int form = br_form(c, batch);
+    if (split == 0)
+        if (const uint64_t head = br_head(c, form, batch)) {
+            const tp_status s = br_batch_launch(c, head, results, lwes, lwe_stride, accs, acc_stride, out_coef, stream, 0);
+            return s != TP_OK ? s
+                              : br_batch_launch(c, batch - head, results + head * 2 * c->prm.ring_dim,
+                                                lwes + head * lwe_stride, lwe_stride, accs + head * acc_stride,
+                                                acc_stride, out_coef, stream, 0);
+        }
+    if (form <= kFftHalves) {
+        TP_CUDA(cudaSetDevice(c->device));
+        tp::BrFftParams fp{};
+        fp.key = c->fft_key;
+        fp.tab_fwd = c->fft_tab->pass_fwd;
+        fp.tab_inv = c->fft_tab->pass_inv;
+        fp.roots = c->fft_tab->roots;
+        fp.lwes = lwes;
+        fp.lwe_stride = lwe_stride;
+        fp.accs = accs;
+        fp.acc_stride = acc_stride;
+        fp.out = results;
+        fp.batch = batch;
+        fp.n = c->prm.lwe_dim;
+        fp.corr = c->kp.corr;
+        memcpy(fp.dshift, c->kp.dshift, sizeof fp.dshift);
+        memcpy(fp.dmask, c->kp.dmask, sizeof fp.dmask);
+        memcpy(fp.ddelta, c->kp.ddelta, sizeof fp.ddelta);
+        fp.err = c->err;
+        fp.head = c->fft_tab->head;
+        // A recorded launch may be replayed over a later key, whose products need not be exact: the
+        // modular form is recorded behind it, and c->exact says on the device which of the two runs.
+        const bool rec = recording(stream);
+        if (rec) {
+            fp.exact = c->exact;
+            c->fft_recorded = true;
+        }
+        void* fargs[] = {&fp};
+        if (const int i = form; i < kFftOneBlock) {
+            cudaLaunchAttribute attr;
+            const cudaLaunchConfig_t cfg =
+                br_fftc_config(c, i, (unsigned)std::min<uint64_t>(batch, c->fftc[i].cap), (cudaStream_t)stream, &attr);
+            TP_CUDA(cudaLaunchKernelExC(&cfg, c->fftc[i].k, fargs));
+        } else if (form == kFftHalves) {
+            TP_CUDA(cudaLaunchKernel(c->fft_kernel, dim3(2 * (unsigned)std::min<uint64_t>(batch, c->fft_cap)),
+                                     dim3(tp::br_fft_halves_threads(c->logn, c->fft_limbs)), fargs, c->fft_smem,
+                                     (cudaStream_t)stream));
+        } else if (form == kFftPair) {
+            TP_CUDA(cudaLaunchKernel(c->fftp.k, dim3(2 * (unsigned)std::min<uint64_t>((batch + 1) / 2, c->fftp.cap)),
+                                     dim3(tp::br_fft_threads(c->logn, (int)c->prm.digits, c->fft_limbs)), fargs,
+                                     c->fftp.smem, (cudaStream_t)stream));
+        } else {
+            TP_CUDA(cudaLaunchKernel(c->fft_kernel, dim3((unsigned)std::min<uint64_t>(batch, c->fft_cap)),
+                                     dim3(tp::br_fft_threads(c->logn, (int)c->prm.digits, c->fft_limbs)), fargs,
+                                     c->fft_smem, (cudaStream_t)stream));
+        }
+        tp::note_launch();
+        if (rec) {
+            const tp_status s = br_modular_launch(c, batch, results, lwes, lwe_stride, accs, acc_stride, 1, stream,
+                                                  br_form_split(br_modular_form(c, batch)), c->exact);
+            if (s != TP_OK) return s;
+            ++t_standby;
+        }
+        return out_coef ? TP_OK : ntt_launch(c->prm.ring_dim, 2 * batch, results, results, stream, true);
+    }
+    if (split == 0) split = form == kModular ? c->split : br_form_split(form);
+    return br_modular_launch(c, batch, results, lwes, lwe_stride, accs, acc_stride, out_coef, stream, split, nullptr);
 }
 
 }  // namespace tp

@@ -73,7 +73,9 @@ tp_status tp_br_destroy(tp_br_ctx* ctx);
 uint64_t tp_br_key_words(const tp_br_ctx* ctx);
 
 /* Uploads a key in that reference layout from host memory (`words` must equal
- * tp_br_key_words) and re-lays it out on the device. Synchronous. */
+ * tp_br_key_words) and re-lays it out on the device. Synchronous. Launches recorded
+ * before (tp_graph, or a caller's own stream capture) rotate with the new key when
+ * they are replayed; record them again after a change of the tile. */
 tp_status tp_br_upload_key(tp_br_ctx* ctx, const uint64_t* brk_host, uint64_t words);
 
 /* Drop-in for BlindRotator::BlindRotate(result, lwe, acc, output_as_coefficients)
@@ -106,7 +108,8 @@ tp_status tp_br_blind_rotate_batch_host(tp_br_ctx* ctx, uint64_t batch, uint64_t
  * rotation with radix-8 NTT passes; 4: N/4 threads, radix-4 passes, fewer
  * registers per thread so more warps per SM). Changing it after the key is
  * uploaded re-lays the key out on the device (twice the key's memory while it
- * runs). Not thread-safe against concurrent launches on the same context. No
+ * runs); recorded launches then have to be recorded again. Not thread-safe
+ * against concurrent launches on the same context. No
  * reference counterpart (tiling is a property of the GPU kernel). */
 tp_status tp_br_set_tile(tp_br_ctx* ctx, uint32_t coef_per_thread);
 uint32_t tp_br_get_tile(const tp_br_ctx* ctx);
