@@ -1224,6 +1224,9 @@ struct tp_ks_ctx {
     const tp::FftTables* fft_tab = nullptr;
     double2* fft_key = nullptr;
     bool fft_ready = false, fft_on = true;
+    unsigned long long* norm2 = nullptr;    // device words: the keys' largest squared norm,
+    unsigned int* exact = nullptr;          // and behind it a copy of fft_ready for recorded launches
+    std::atomic<bool> fft_recorded{false};  // a recorded launch names fft_key
     std::mutex mu;
 };
 
@@ -1246,7 +1249,9 @@ static void ks_setup_fft(tp_ks_ctx* c) {
         if (e == cudaSuccess)
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, tp::ks_fft_threads(c->logn, limbs), smem);
         if (e == cudaSuccess && per_sm > 0) e = tp::fft_tables(c->device, c->logn - 1, &c->fft_tab);
+        if (e == cudaSuccess && per_sm > 0) e = cudaMalloc(&c->norm2, 2 * sizeof *c->norm2);
         if (e == cudaSuccess && per_sm > 0) {
+            c->exact = reinterpret_cast<unsigned int*>(c->norm2 + 1);
             c->fft_kernel = k;
             c->fft_cap = per_sm * sm_count(c->device);
             return;
@@ -1380,6 +1385,7 @@ tp_status tp_ks_destroy(tp_ks_ctx* c) {
     cudaSetDevice(c->device);
     cudaFree(c->key);
     cudaFree(c->fft_key);
+    cudaFree(c->norm2);
     cudaFree(c->work);
     cudaFree(c->consec_plan);
     cudaFree(c->zero);
@@ -1390,29 +1396,29 @@ tp_status tp_ks_destroy(tp_ks_ctx* c) {
 uint64_t tp_ks_key_words(const tp_ks_ctx* c) { return c ? c->key_words : 0; }
 
 // The limbs' transforms of the keys in `stage` (reference layout, overwritten), where there is
-// room for them and they pass the bound; without them the modular kernel runs.
+// room for them and they pass the bound; without them the modular kernel runs. Once there, every
+// upload rewrites them: recorded launches read them while *exact says so.
 static cudaError_t ks_upload_fft(tp_ks_ctx* c, uint64_t* stage) {
     c->fft_ready = false;
-    unsigned long long* norm2 = nullptr;
     unsigned long long v = 0;
     const uint64_t polys = c->key_words / c->N;
-    cudaError_t e = cudaMalloc(&norm2, sizeof *norm2);
-    if (e == cudaSuccess && !c->fft_key) e = cudaMalloc(&c->fft_key, c->key_words * 8 * c->fft_limbs);
-    if (e != cudaSuccess) {
+    if (!c->fft_key && cudaMalloc(&c->fft_key, c->key_words * 8 * c->fft_limbs) != cudaSuccess) {
         cudaGetLastError();
-        cudaFree(norm2);
         return cudaSuccess;
     }
-    e = cudaMemset(norm2, 0, sizeof *norm2);
+    cudaError_t e = cudaMemset(c->norm2, 0, 2 * sizeof *c->norm2);  // and *exact
     tp::scale_kernel<<<(unsigned)std::min<uint64_t>((c->key_words + 255) / 256, 65535), 256>>>(stage, stage, c->key_words, 1);
     tp::note_launch();
     if (e == cudaSuccess && ntt_launch(c->N, polys, stage, stage, nullptr, false) != TP_OK) e = cudaErrorLaunchFailure;
-    tp::fft_key_launch(c->fft_key, stage, polys, 0, 1, c->digits, c->fft_limbs, *c->fft_tab, norm2, nullptr);
+    tp::fft_key_launch(c->fft_key, stage, polys, 0, 1, c->digits, c->fft_limbs, *c->fft_tab, c->norm2, nullptr);
     tp::note_launch();
     if (e == cudaSuccess) e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpy(&v, norm2, sizeof v, cudaMemcpyDeviceToHost);
-    cudaFree(norm2);
-    if (e == cudaSuccess) c->fft_ready = ks_fft_key_exact(c, (double)v);
+    if (e == cudaSuccess) e = cudaMemcpy(&v, c->norm2, sizeof v, cudaMemcpyDeviceToHost);
+    const bool exact = e == cudaSuccess && ks_fft_key_exact(c, (double)v);
+    const unsigned int one = 1;
+    if (exact) e = cudaMemcpy(c->exact, &one, sizeof one, cudaMemcpyHostToDevice);
+    else if (c->fft_recorded) cudaMemset(c->fft_key, 0xFF, c->key_words * 8 * c->fft_limbs);  // unlike any key
+    c->fft_ready = exact && e == cudaSuccess;
     return e;
 }
 
@@ -1455,12 +1461,20 @@ static tp_status ks_launch(tp_ks_ctx* c, int mode, const tp::KsKernelParams& kp,
         fp.tab_inv = c->fft_tab->pass_inv;
         fp.mode = mode;
         fp.head = c->fft_tab->head;
+        // a recorded launch may be replayed over a later key: the modular kernel stands by behind it
+        // (as in br_batch_launch)
+        const bool rec = recording(st);
+        if (rec) {
+            fp.ks.exact = p.exact = c->exact;
+            c->fft_recorded = true;
+        }
         void* fargs[] = {&fp};
         TP_CUDA(cudaLaunchKernel(c->fft_kernel, dim3((unsigned)std::min<uint64_t>(kp.items, c->fft_cap)),
                                  dim3(tp::ks_fft_threads(c->logn, c->fft_limbs)), fargs,
                                  tp::ks_fft_smem(c->logn, c->fft_limbs), st));
         tp::note_launch();
-        return TP_OK;
+        if (!rec) return TP_OK;
+        ++tp::t_standby;
     }
     if (mode == tp::kKsRlwe && c->rlwe_kernel && c->fft_on && (((uintptr_t)kp.in | (uintptr_t)kp.out) & 15) == 0) {
         // its 16-byte accesses need the alignment; two to four digits, N = 1024 .. 4096
@@ -1771,7 +1785,8 @@ static tp_status pack_merge_levels(tp_ks_ctx* c, uint64_t packs, uint64_t count,
 // lwe_to_rlwe_packing.cpp:129-224). The double-precision kernel's first level reads the LWE rows
 // itself, which saves a pass over nodes twice their size.
 static tp_status pack_tree(tp_ks_ctx* c, uint64_t packs, uint64_t len, uint64_t* work, const uint64_t* in, cudaStream_t st) {
-    if (len > 1 && c->fft_ready && c->fft_on) return pack_merge_levels(c, packs, len, 0, work, in, st);
+    // (when recorded, the set-up is a launch of its own: the modular merges standing by need the nodes)
+    if (len > 1 && c->fft_ready && c->fft_on && !recording(st)) return pack_merge_levels(c, packs, len, 0, work, in, st);
     const uint64_t need = packs * len * 2 * c->N;
     tp::pack_l0_kernel<<<(unsigned)std::min<uint64_t>((need + 255) / 256, 65535), 256, 0, st>>>(
         work, in, packs, (uint32_t)len, (uint32_t)ilog2(len), (uint32_t)c->logn, c->tab->n_inv);

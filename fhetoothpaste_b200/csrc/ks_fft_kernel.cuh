@@ -39,6 +39,7 @@ ks_fft_kernel(const __grid_constant__ KsFftParams prm) {
     constexpr int N = 1 << LOGN, n = F::n, TG = F::T, LANES = n / 8, T = LANES * L;
     static_assert(T == TG * 2 * L && DL <= 2 * L, "block shape");
 
+    if (prm.ks.exact && !*prm.ks.exact) return;
     extern __shared__ __align__(16) uint64_t smem[];
     double2* buf = reinterpret_cast<double2*>(smem);                  // 2L n
     ulonglong2* as = reinterpret_cast<ulonglong2*>(buf + 2 * L * n);  // n: aut(diff).A plus corr

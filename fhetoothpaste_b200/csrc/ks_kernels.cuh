@@ -57,6 +57,7 @@ struct KsKernelParams {
     // up from its LWE row as pack_l0_kernel does
     const uint64_t* leaf;
     uint32_t leaf_log;
+    const unsigned int* exact;  // recorded launches: the double-precision kernel runs while *exact is not 0, else this one
     uint64_t corr;
     uint32_t dshift[8];
     uint64_t dmask[8];
@@ -170,6 +171,7 @@ ks_kernel(const KsKernelParams prm) {
     constexpr int E = 1 << LOGE;
     constexpr int T = NL / E;
     static_assert(LOGS == 0 || LOGE == 2, "clusters run with 4 coefficients per thread");
+    if (prm.exact && *prm.exact) return;
     extern __shared__ __align__(16) uint64_t smem[];
     uint64_t* tw_f = smem;          // the first NL words of the N-point tables (the NL-point tables)
     uint64_t* tw_i = smem + NL;

@@ -217,7 +217,8 @@ tp_status tp_pack_create(uint32_t ring_dim, uint64_t basis, uint32_t digits, int
 
 tp_status tp_ks_destroy(tp_ks_ctx* ctx);
 uint64_t tp_ks_key_words(const tp_ks_ctx* ctx);
-/* Host key in the reference layout above; re-laid out on the device. Synchronous. */
+/* Host key in the reference layout above; re-laid out on the device. Synchronous.
+ * Recorded launches use the new key, as with tp_br_upload_key. */
 tp_status tp_ks_upload_key(tp_ks_ctx* ctx, const uint64_t* key_host, uint64_t words);
 
 /* Coefficients per thread of the key-switching kernels (4 or 8; default 4):

@@ -67,3 +67,40 @@ def test_rotations(native, oracle, variant, N, beta, digits, limbs, batch, launc
                 np.testing.assert_array_equal(got[b].cpu().numpy().view(np.uint64), want)
     own.close()
     rot.close()
+
+
+@pytest.mark.parametrize("N,beta,digits,limbs,packs,length", [(2048, 14, 3, 3, 1, 4), (1024, 12, 3, 3, 3, 2)])
+def test_packings(native, oracle, N, beta, digits, limbs, packs, length):
+    """Merges and traces of a captured packing, allocation-free as a capture needs it."""
+    import torch
+    from fhetoothpaste_b200 import GpuLWEtoRLWEPacker, _native
+    rng = np.random.default_rng(N)
+    logn = N.bit_length() - 1
+    keys = [rng.integers(0, P, logn * digits * 2 * N, dtype=np.uint64),
+            np.tile(worst_poly(oracle, N, limbs), logn * digits * 2),
+            rng.integers(0, P, logn * digits * 2 * N, dtype=np.uint64)]
+    pk = GpuLWEtoRLWEPacker(N, 1 << beta, digits, keys[0])
+    x = rng.integers(0, P, (packs * length, N + 1), dtype=np.uint64)
+    d_x = torch.from_numpy(x.view(np.int64)).cuda()
+    out = torch.zeros((packs, 2 * N), dtype=torch.int64, device="cuda")
+
+    def pack(stream):
+        _native.check(native.tp_pack_batch_noalloc(pk._h, packs, length, out.data_ptr(), d_x.data_ptr(), stream))
+
+    pack(None)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        pack(torch.cuda.current_stream().cuda_stream)
+    # set-up, each merge and trace with its modular kernel behind it, the copy of the results
+    assert graph_nodes(graph) == 2 + 2 * logn
+    graph.instantiate()
+    for key in keys:
+        _native.check(native.tp_ks_upload_key(pk._h, _native.ptr(key), key.size))
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        got = out.cpu().numpy().view(np.uint64)
+        for p in range(packs):
+            want = oracle.pack(N, beta, digits, key, x[p * length:(p + 1) * length], length)
+            np.testing.assert_array_equal(got[p], want)
