@@ -27,7 +27,7 @@ def graph_nodes(graph) -> int:
 # counts are those whose bound the second key fails
 @pytest.mark.parametrize("variant,N,beta,digits,limbs,batch,launches", [
     (1, 2048, 12, 3, 3, 1, 1), (1, 2048, 12, 3, 3, 20, 1), (1, 2048, 12, 3, 3, 75, 1), (1, 2048, 12, 3, 3, 160, 2),
-    (1, 1024, 12, 3, 3, 75, 1), (1, 4096, 16, 4, 4, 16, 1)])
+    (1, 1024, 13, 3, 3, 75, 1), (1, 4096, 16, 4, 4, 16, 1)])
 def test_rotations(native, oracle, variant, N, beta, digits, limbs, batch, launches):
     import torch
     from fhetoothpaste_b200 import BlindRotationContext, GpuBlindRotator, _native
@@ -69,7 +69,7 @@ def test_rotations(native, oracle, variant, N, beta, digits, limbs, batch, launc
     rot.close()
 
 
-@pytest.mark.parametrize("N,beta,digits,limbs,packs,length", [(2048, 14, 3, 3, 1, 4), (1024, 12, 3, 3, 3, 2)])
+@pytest.mark.parametrize("N,beta,digits,limbs,packs,length", [(2048, 14, 3, 3, 1, 4), (1024, 15, 3, 3, 3, 2)])
 def test_packings(native, oracle, N, beta, digits, limbs, packs, length):
     """Merges and traces of a captured packing, allocation-free as a capture needs it."""
     import torch
