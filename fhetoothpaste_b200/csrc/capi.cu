@@ -1948,43 +1948,15 @@ bool byte_map(CUtensorMap* m, void* base, uint64_t kpad, uint64_t rows, uint32_t
                                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// One pass of the tensor-core key switch over up to rows() ciphertexts.
-struct LweMmaPlan {
-    uint32_t rows, rows_pad, splits;
-    uint64_t plane_bytes, part_bytes;  // digit planes, then partial sums
-    uint64_t bytes() const { return plane_bytes + part_bytes; }
-};
-LweMmaPlan lwe_mma_plan(const tp_lwe_ks_ctx* c, uint64_t batch) {
-    LweMmaPlan p{};
-    // at most 256 MB of digit planes at a time
-    const uint64_t most = std::max<uint64_t>(1, (256ull << 20) / ((uint64_t)c->planes * c->kpad * tp::kMmaRows)) * tp::kMmaRows;
-    p.rows = (uint32_t)std::min(batch, most);
-    p.rows_pad = (p.rows + tp::kMmaRows - 1) / tp::kMmaRows * tp::kMmaRows;
-    const uint32_t steps = c->kpad / tp::kMmaK;
-    const uint64_t tiles = (uint64_t)(p.rows_pad / tp::kMmaRows) * ((c->n_out + tp::kMmaWords) / tp::kMmaWords);
-    const uint64_t sms = (uint64_t)sm_count(c->device);
-    // splits of K: the fewest block-steps over the waves, a block costing about six steps
-    // beside its share (fill, drain, epilogue); at least enough for exact 32-bit sums
-    uint64_t best = ~0ull;
-    for (uint32_t s = (steps + tp::kMmaMaxSteps - 1) / tp::kMmaMaxSteps; s <= steps && s <= 64; ++s) {
-        const uint32_t share = (steps + s - 1) / s;
-        if ((steps + share - 1) / share != s) continue;  // every split has steps
-        const uint64_t cost = (tiles * s + sms - 1) / sms * (share + 6) + s / 4;
-        if (cost < best) {
-            best = cost;
-            p.splits = s;
-        }
-    }
-    p.plane_bytes = (uint64_t)c->planes * p.rows_pad * c->kpad;
-    p.part_bytes = (uint64_t)p.splits * p.rows * (c->n_out + 1) * 8;
-    return p;
+tp::LweMmaPlan lwe_mma_plan(const tp_lwe_ks_ctx* c, uint64_t batch) {
+    return tp::lwe_mma_plan(c->planes, c->kpad, c->n_out + 1, batch, (uint64_t)sm_count(c->device));
 }
 
 // The tensor-core form of a context whose key is on the device: key bytes, workspace pool.
 // Optional (digits of up to two bytes, room on the device): the scalar kernel takes the rest.
 cudaError_t lwe_mma_setup(tp_lwe_ks_ctx* c) {
     const int planes = (ilog2(c->basis) + 7) / 8;
-    if (planes > 2 || !tensor_map_encoder()) return cudaSuccess;
+    if (!tp::lwe_mma_fits(planes, (uint64_t)c->n_out + 1) || !tensor_map_encoder()) return cudaSuccess;
     const uint32_t kpad = (c->n_in * c->digits + tp::kMmaK - 1) / tp::kMmaK * tp::kMmaK;
     cudaError_t e = cudaSuccess;
     if (!c->kbytes) {
@@ -2024,7 +1996,7 @@ tp_status lwe_ks_launch(const tp_lwe_ks_ctx* c, tp::LweKsParams kp, uint8_t* ws,
     bool mma = c->planes > 0;
     uint8_t* own = nullptr;
     if (mma && *(volatile int*)c->err) return fail(TP_ERR_TIMEOUT, "a wait inside an earlier LWE key switch ran out");
-    LweMmaPlan plan{};
+    tp::LweMmaPlan plan{};
     if (mma) {
         plan = lwe_mma_plan(c, kp.batch);
         if (!ws) {

@@ -24,15 +24,13 @@
 
 #include "gl_arith.cuh"
 #include "ks_util_kernels.cuh"
+#include "lwe_mma_plan.h"
 #include "mbar.cuh"
 
 namespace tp {
 
-constexpr int kMmaRows = 128, kMmaCols = 256, kMmaK = 128;      // block tile, bytes of K per step
-constexpr int kMmaWords = kMmaCols / 8;                         // output words per tile
 constexpr int kMmaStages = 3;
 constexpr int kMmaThreads = 192;                                // warps 0-3 epilogue, 4 loads, 5 products
-constexpr uint32_t kMmaMaxSteps = 258;                          // 255^2 * 128 * 258 < 2^31
 __host__ __device__ constexpr size_t mma_stage_bytes(int planes) { return (size_t)(planes * kMmaRows + kMmaCols) * kMmaK; }
 __host__ __device__ constexpr size_t mma_smem(int planes) { return kMmaStages * mma_stage_bytes(planes) + 1024 + 128; }
 
