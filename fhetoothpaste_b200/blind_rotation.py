@@ -146,8 +146,8 @@ class GpuBlindRotator:
         nat.check(nat.lib().tp_br_set_radix(self._h, radix))
 
     def autotune(self, batch: int) -> tuple[int, float]:
-        """Times every tile (and the two- and four-block splits) on `batch` synthetic rotations and keeps
-        the fastest."""
+        """Times the form chosen by batch size, every tile and the two- and four-block splits on `batch`
+        synthetic rotations and keeps the fastest."""
         coef, rate = ctypes.c_uint32(), ctypes.c_double()
         nat.check(nat.lib().tp_br_autotune(self._h, batch, ctypes.byref(coef), ctypes.byref(rate)))
         return int(coef.value), float(rate.value)

@@ -244,6 +244,7 @@ struct tp_br_ctx {
     const void* ds_kernel = nullptr;  // digit-staged one-block kernel (digits 3 or 4, N <= 2048)
     size_t ds_smem = 0;
     int ds_cap = 0;               // its resident blocks on the device (0: unavailable)
+    int loge0 = 3, mac0 = 0;      // tile and multiply-accumulate form of a new context
     int radix = 2;                // NTT passes of the one-block kernel at tile 4: 2 or 4 (fused radix-4)
     struct Form {
         const void* k = nullptr;
@@ -271,7 +272,7 @@ struct tp_br_ctx {
     const tp::FftTables* fft_tab = nullptr;
     double2* fft_key = nullptr;
     bool fft_ready = false;       // the key is resident and exact in this form
-    bool fft_on = true;
+    bool open = true;             // no launch form named: it is chosen by batch size (br_form, br_head, br_ring_logs)
     std::atomic<bool> fft_recorded{false};  // a recorded launch names fft_key
     // workspace for host-pointer calls
     uint64_t* ws = nullptr;
@@ -469,7 +470,7 @@ static int br_modular_form(const tp_br_ctx* c, uint64_t batch) {
 }
 static int br_form_split(int form) { return form == kModularPair ? 2 : form == kModularQuad ? 4 : 1; }
 static int br_form(const tp_br_ctx* c, uint64_t batch) {
-    if (!c->fft_on) return kModular;
+    if (!c->open) return kModular;
     if (!c->fft_ready) return br_modular_form(c, batch);
     for (int i = 2; i >= 0; --i)
         if (batch <= (uint64_t)c->fftc[i].cap) return i;
@@ -489,8 +490,12 @@ static int br_form(const tp_br_ctx* c, uint64_t batch) {
 //   N = 16384, n = 32: 8 / 4 CTAs      ternary 1.6 / 2.9        binary 1.4 / 2.5        BMMP 1.1 / 1.8
 static int br_ring_logs(const tp_br_ctx* c, uint64_t batch) {
     for (int i = 1; i >= 0; --i)
-        if (c->fft_on && batch <= (uint64_t)c->wide[i].cap) return c->logs + 1 + i;
+        if (c->open && batch <= (uint64_t)c->wide[i].cap) return c->logs + 1 + i;
     return c->logs;
+}
+
+namespace tp {
+static uint64_t br_open_wave(const tp_br_ctx* c, uint64_t batch);
 }
 
 extern "C" {
@@ -601,6 +606,8 @@ tp_status tp_br_create(const tp_br_params* p, int device, tp_br_ctx** out) {
             delete c;
             return cs;
         }
+        c->loge0 = c->loge;
+        c->mac0 = c->mac;
         *out = c;
         return TP_OK;
     }
@@ -683,6 +690,8 @@ tp_status tp_br_create(const tp_br_params* p, int device, tp_br_ctx** out) {
         }
     }
     br_setup_fft(c);
+    c->loge0 = c->loge;
+    c->mac0 = c->mac;
     *out = c;
     return TP_OK;
 }
@@ -825,7 +834,7 @@ tp_status tp_br_set_tile(tp_br_ctx* c, uint32_t coef_per_thread) {
                     c->prm.ring_dim);
     TP_CUDA(cudaSetDevice(c->device));
     tp_status s = br_retile(c, coef_per_thread == 4 ? 2 : 3);
-    if (s == TP_OK) c->fft_on = false;
+    if (s == TP_OK) c->open = false;
     return s;
 }
 
@@ -845,7 +854,7 @@ tp_status tp_br_set_split(tp_br_ctx* c, uint32_t blocks_per_rotation) {
                         blocks_per_rotation);
     }
     c->split = (int)blocks_per_rotation;
-    c->fft_on = false;
+    c->open = false;
     return TP_OK;
 }
 
@@ -860,7 +869,7 @@ tp_status tp_br_set_mac_form(tp_br_ctx* c, uint32_t form) {
         return fail(TP_ERR_PARAM, "the digit-staged kernel is not built for this parameter set on this device "
                                   "(digits 3 or 4, N <= 2048, shared memory permitting)");
     c->mac = (int)form;
-    c->fft_on = false;
+    c->open = false;
     return TP_OK;
 }
 
@@ -874,7 +883,7 @@ tp_status tp_br_set_radix(tp_br_ctx* c, uint32_t radix) {
         return fail(TP_ERR_PARAM, "fused radix-4 rotation kernels are not built for this parameter set "
                                   "(N = 1024 .. 4096, shared memory permitting)");
     c->radix = (int)radix;
-    c->fft_on = false;
+    c->open = false;
     return TP_OK;
 }
 
@@ -885,9 +894,16 @@ tp_status tp_br_autotune(tp_br_ctx* c, uint64_t batch, uint32_t* best_coef_per_t
     if (!c->key_ready) return fail(TP_ERR_STATE, "no key uploaded");
     if (batch == 0) return fail(TP_ERR_PARAM, "empty batch");
     const uint64_t N = c->prm.ring_dim, n = c->prm.lwe_dim;
+    std::lock_guard<std::mutex> lk(c->mu);
+    // The caller's own batch up to four waves; of a larger one four, and what it leaves behind full
+    // waves of the open form (which may run in a form of its own).
     const uint64_t cap = (uint64_t)std::max(std::max(c->grid_caps[2], c->grid_caps[3]),
                                             std::max(c->pair_cap, c->fft_cap));  // >= quad_cap
-    const uint64_t tb = std::min<uint64_t>(batch, 2 * cap);  // at most two waves per trial
+    const bool was_open = c->open;
+    c->open = true;
+    const uint64_t wave = std::min(4 * cap, std::max<uint64_t>(1, tp::br_open_wave(c, batch)));
+    c->open = was_open;
+    const uint64_t tb = batch <= 4 * cap ? batch : 4 * cap / wave * wave + batch % wave;
     std::vector<uint64_t> lw(tb * (n + 1));
     uint64_t z = 0x5eedull;
     for (auto& w : lw) {  // splitmix64 words in [0, 2N): timing does not depend on the values
@@ -923,21 +939,19 @@ tp_status tp_br_autotune(tp_br_ctx* c, uint64_t batch, uint32_t* best_coef_per_t
         cleanup();
         return fail(TP_ERR_CUDA, "autotune set-up: %s", cudaGetErrorString(e));
     }
-    std::lock_guard<std::mutex> lk(c->mu);
     int best_split = c->split;
     int best_mac = c->mac;
     int best_radix = c->radix;
-    bool best_fft = c->fft_on;
-    // tile (coefficients per thread), blocks per rotation, multiply-accumulate form, NTT radix;
-    // or the double-precision kernel (the other settings then stay as they are)
-    struct Cand { int loge, split, mac, radix; bool fft; };
-    const Cand cands[] = {{c->loge, c->split, c->mac, c->radix, true},
+    bool best_open = c->open;
+    // tile (coefficients per thread), blocks per rotation, multiply-accumulate form, NTT radix; first
+    // the form left open, with the settings that a new context has
+    struct Cand { int loge, split, mac, radix; bool open; };
+    const Cand cands[] = {{c->loge0, 1, c->mac0, 2, true},
                           {3, 1, TP_MAC_ROWWISE, 2},      {2, 1, TP_MAC_ROWWISE, 2}, {2, 1, TP_MAC_DIGIT_STAGED, 2},
                           {2, 1, TP_MAC_ROWWISE, 4},      {2, 1, TP_MAC_DIGIT_STAGED, 4},
                           {2, 2, TP_MAC_ROWWISE, 2},      {2, 4, TP_MAC_ROWWISE, 2}};
     for (const Cand& cd : cands) {
-        if (cd.fft && !c->fft_ready) continue;
-        c->fft_on = cd.fft;
+        c->open = cd.open;
         if ((cd.split == 2 && c->pair_cap == 0) || (cd.split == 4 && c->quad_cap == 0)) continue;
         if (cd.mac == TP_MAC_DIGIT_STAGED && !c->ds_kernel) continue;
         if (cd.radix == 4 && !(cd.mac == TP_MAC_DIGIT_STAGED ? c->r4_ds.k : c->r4_row.k)) continue;
@@ -961,13 +975,14 @@ tp_status tp_br_autotune(tp_br_ctx* c, uint64_t batch, uint32_t* best_coef_per_t
             break;
         }
         const double rate = 2.0 * tb / (ms * 1e-3);
-        if (rate > best_rate) {
+        // a named form has to win by more than the trials' noise: it ends the choice by batch size
+        if (rate > best_rate * (best_open && !cd.open ? 1.01 : 1.0)) {
             best_rate = rate;
             best = cd.loge;
             best_split = cd.split;
             best_mac = cd.mac;
             best_radix = cd.radix;
-            best_fft = cd.fft;
+            best_open = cd.open;
         }
     }
     c->split = 1;
@@ -977,7 +992,7 @@ tp_status tp_br_autotune(tp_br_ctx* c, uint64_t batch, uint32_t* best_coef_per_t
         c->mac = best_mac;
         c->radix = best_radix;
     }
-    c->fft_on = best_fft;
+    c->open = best_open;
     cleanup();
     if (s != TP_OK) return s;
     if (best_coef_per_thread) *best_coef_per_thread = 1u << best;
@@ -2998,6 +3013,14 @@ uint64_t br_fft_blocks(const tp_br_ctx* c, uint64_t batch) {
     return i < kFftOneBlock ? batch << (i + 1) : std::min<uint64_t>(batch, c->fft_cap);
 }
 
+// Rotations of a full wave of `form`, where a batch may be cut behind full waves; 0 elsewhere.
+static uint64_t br_wave(const tp_br_ctx* c, int form) {
+    if (form == kFftOneBlock) return (uint64_t)c->fft_cap;
+    if (form == kFftPair) return 2ull * c->fftp.cap;
+    return form == kModular && c->open ? (uint64_t)br_one_block(c).cap : 0;
+}
+static uint64_t br_open_wave(const tp_br_ctx* c, uint64_t batch) { return br_wave(c, br_form(c, batch)); }
+
 // Rotations of a batch that run in `form` before the rest gets a launch of its own: the full waves,
 // where the rest fits a wave of a wider form, which is shorter than one more wave of this one.
 // 0: one launch. Milliseconds, n = 60 (a wave, the rest in the same form, in its own):
@@ -3005,10 +3028,7 @@ uint64_t br_fft_blocks(const tp_br_ctx* c, uint64_t batch) {
 //   ternary N = 8192 (n = 64), 100 = 74 + 26: 5.37, 5.40, 2.70
 //   ternary N = 2048, l = 3, 160 = 148 + 12: 1.04, 1.0, 0.41
 static uint64_t br_head(const tp_br_ctx* c, int form, uint64_t batch) {
-    uint64_t wave = 0;
-    if (form == kFftOneBlock) wave = (uint64_t)c->fft_cap;
-    if (form == kFftPair) wave = 2ull * c->fftp.cap;
-    if (form == kModular && c->fft_on) wave = (uint64_t)br_one_block(c).cap;
+    const uint64_t wave = br_wave(c, form);
     if (wave == 0 || batch <= wave || batch % wave == 0) return 0;
     const uint64_t rest = batch % wave;
     const int f = br_form(c, rest);

@@ -148,12 +148,15 @@ uint32_t tp_br_get_mac_form(const tp_br_ctx* ctx);
 tp_status tp_br_set_radix(tp_br_ctx* ctx, uint32_t radix);
 uint32_t tp_br_get_radix(const tp_br_ctx* ctx);
 
-/* Times every launch form (8 or 4 coefficients per thread; at 4 also the
+/* Times the form that a new context runs (chosen by batch size, see tp_br_set_tile)
+ * and every named launch form (8 or 4 coefficients per thread; at 4 also the
  * digit-staged multiply-accumulate, the fused radix-4 passes and two or four
- * blocks per rotation) on up to two waves of `batch` synthetic rotations with the
- * uploaded key, keeps the fastest and reports it (either output may be NULL; the
- * split, form and radix are read back with tp_br_get_split / tp_br_get_mac_form /
- * tp_br_get_radix). Blocks until done; the context must be idle. */
+ * blocks per rotation) on `batch` synthetic rotations with the uploaded key (of more
+ * than four waves, four and the batch's remainder), keeps the fastest and reports
+ * it (either output may be NULL; the split, form and radix are read back with
+ * tp_br_get_split / tp_br_get_mac_form / tp_br_get_radix). A named form is kept
+ * only where it is more than 1% faster than the choice by batch size.
+ * Blocks until done; the context must be idle. */
 tp_status tp_br_autotune(tp_br_ctx* ctx, uint64_t batch, uint32_t* best_coef_per_thread,
                          double* best_rotations_per_s);
 
