@@ -138,6 +138,8 @@ def lib() -> ctypes.CDLL:
         "tp_server_run_poisson": (ctypes.c_int, [VP, ctypes.c_double, ctypes.c_double, ctypes.POINTER(ctypes.c_double),
                                                  ctypes.c_uint32, ctypes.POINTER(U64P), ctypes.POINTER(U64P), U64P,
                                                  U64]),
+        "tp_debug_modular": (ctypes.c_int, [VP, ctypes.c_int]),
+        "tp_debug_ks_modular": (ctypes.c_int, [VP, ctypes.c_int]),
         "tp_debug_arith": (ctypes.c_int, [ctypes.c_int, U64, VP, VP, VP, VP, VP]),
         "tp_measure_int_peak": (ctypes.c_int, [ctypes.c_int, ctypes.POINTER(ctypes.c_double),
                                                 ctypes.POINTER(ctypes.c_double)]),

@@ -260,7 +260,7 @@ struct tp_br_ctx {
     size_t quad_smem = 0;
     int quad_cap = 0;             // resident four-CTA clusters on the device (0: unavailable)
     // Double-precision transform kernel (br_fft_kernel.cuh), where one is built for the set and
-    // the uploaded key passes its exactness bound; runs unless a launch form was set by name.
+    // the uploaded key passes its exactness bound; runs while the launch form is open.
     const void* fft_kernel = nullptr;
     int fft_limbs = 0, fft_cap = 0;
     size_t fft_smem = 0;
@@ -272,7 +272,9 @@ struct tp_br_ctx {
     const tp::FftTables* fft_tab = nullptr;
     double2* fft_key = nullptr;
     bool fft_ready = false;       // the key is resident and exact in this form
-    bool open = true;             // no launch form named: it is chosen by batch size (br_form, br_head, br_ring_logs)
+    // no launch form named but a new context's own: it is chosen by batch size (br_form, br_head, br_ring_logs)
+    bool open = true;
+    bool modular = false;         // tp_debug_modular
     std::atomic<bool> fft_recorded{false};  // a recorded launch names fft_key
     // workspace for host-pointer calls
     uint64_t* ws = nullptr;
@@ -482,7 +484,7 @@ static int br_form(const tp_br_ctx* c, uint64_t batch) {
 }
 
 // log2 of the CTAs per rotation of a ring above 4096: the widest cluster that takes the batch in
-// one wave, unless a launch form was set by name. Half as many coefficients per CTA leave the key
+// one wave, while the launch form is open. Half as many coefficients per CTA leave the key
 // stream and the transforms half as long for the price of one more exchange partner, and the
 // 4096-coefficient plan's spills go; a wave of smaller clusters leaves more of the GPU idle once
 // the batch outgrows it. Milliseconds of one wave, 2^12, l = 3 (up to 15 / 33 / 74 rotations):
@@ -822,6 +824,19 @@ static tp_status br_retile(tp_br_ctx* c, int loge) {
     return TP_OK;
 }
 
+// After a setting was named: the form is open while all are a new context's.
+static void br_named(tp_br_ctx* c) {
+    c->open = !c->modular && c->loge == c->loge0 && c->split == 1 && c->mac == c->mac0 && c->radix == 2;
+}
+
+tp_status tp_debug_modular(tp_br_ctx* c, int on) {
+    if (!c) return fail(TP_ERR_PARAM, "null context");
+    std::lock_guard<std::mutex> lk(c->mu);
+    c->modular = on != 0;
+    br_named(c);
+    return TP_OK;
+}
+
 tp_status tp_br_set_tile(tp_br_ctx* c, uint32_t coef_per_thread) {
     if (!c) return fail(TP_ERR_PARAM, "null context");
     if (coef_per_thread != 4 && coef_per_thread != 8) return fail(TP_ERR_PARAM, "coefficients per thread must be 4 or 8");
@@ -834,7 +849,7 @@ tp_status tp_br_set_tile(tp_br_ctx* c, uint32_t coef_per_thread) {
                     c->prm.ring_dim);
     TP_CUDA(cudaSetDevice(c->device));
     tp_status s = br_retile(c, coef_per_thread == 4 ? 2 : 3);
-    if (s == TP_OK) c->open = false;
+    if (s == TP_OK) br_named(c);
     return s;
 }
 
@@ -854,7 +869,7 @@ tp_status tp_br_set_split(tp_br_ctx* c, uint32_t blocks_per_rotation) {
                         blocks_per_rotation);
     }
     c->split = (int)blocks_per_rotation;
-    c->open = false;
+    br_named(c);
     return TP_OK;
 }
 
@@ -869,7 +884,7 @@ tp_status tp_br_set_mac_form(tp_br_ctx* c, uint32_t form) {
         return fail(TP_ERR_PARAM, "the digit-staged kernel is not built for this parameter set on this device "
                                   "(digits 3 or 4, N <= 2048, shared memory permitting)");
     c->mac = (int)form;
-    c->open = false;
+    br_named(c);
     return TP_OK;
 }
 
@@ -883,7 +898,7 @@ tp_status tp_br_set_radix(tp_br_ctx* c, uint32_t radix) {
         return fail(TP_ERR_PARAM, "fused radix-4 rotation kernels are not built for this parameter set "
                                   "(N = 1024 .. 4096, shared memory permitting)");
     c->radix = (int)radix;
-    c->open = false;
+    br_named(c);
     return TP_OK;
 }
 
@@ -951,6 +966,7 @@ tp_status tp_br_autotune(tp_br_ctx* c, uint64_t batch, uint32_t* best_coef_per_t
                           {2, 1, TP_MAC_ROWWISE, 4},      {2, 1, TP_MAC_DIGIT_STAGED, 4},
                           {2, 2, TP_MAC_ROWWISE, 2},      {2, 4, TP_MAC_ROWWISE, 2}};
     for (const Cand& cd : cands) {
+        if (cd.open && c->modular) continue;
         c->open = cd.open;
         if ((cd.split == 2 && c->pair_cap == 0) || (cd.split == 4 && c->quad_cap == 0)) continue;
         if (cd.mac == TP_MAC_DIGIT_STAGED && !c->ds_kernel) continue;
@@ -1218,7 +1234,7 @@ struct tp_ks_ctx {
     bool key_ready = false;
     tp::KsKernelParams kp{};
     size_t smem = 0;
-    int loge = 2;                 // log2 coefficients per thread: 2 (4) or 3 (8)
+    int loge = 2;                 // log2 coefficients per thread: 2 (4, a new context's) or 3 (8)
     int per_sm[2][tp::kKsModes] = {};
     int logs = 0;                 // log2 CTAs per item's cluster (N > 4096), else 0
     int cluster_cap[tp::kKsModes] = {};  // resident clusters per mode (logs > 0)
@@ -1230,15 +1246,17 @@ struct tp_ks_ctx {
     std::vector<uint64_t> consec_off;  // per level: offset into the plan (words)
     std::vector<uint32_t> consec_cnt;  // per level: nodes of one pack
     uint64_t* zero = nullptr;          // 2N zero words
-    // double-precision form of the modes with coefficient results (packing contexts, N = 1024 and
-    // 2048), where one is built and every key passes its exactness bound; off once a tile is set
-    const void* rlwe_kernel = nullptr;  // digit-staged RLWE switch, runs unless a tile was set by name
+    const void* rlwe_kernel = nullptr;  // digit-staged RLWE switch, runs while fft_on
     int rlwe_cap = 0;
+    // double-precision form of the modes with coefficient results (packing contexts, N = 1024 and
+    // 2048), where one is built and every key passes its exactness bound; runs while fft_on
     const void* fft_kernel = nullptr;
     int fft_limbs = 0, fft_cap = 0;
     const tp::FftTables* fft_tab = nullptr;
     double2* fft_key = nullptr;
-    bool fft_ready = false, fft_on = true;
+    bool fft_ready = false;
+    bool fft_on = true;                     // no tile named but a new context's: fft_kernel and rlwe_kernel run
+    bool modular = false;                   // tp_debug_ks_modular
     unsigned long long* norm2 = nullptr;    // device words: the keys' largest squared norm,
     unsigned int* exact = nullptr;          // and behind it a copy of fft_ready for recorded launches
     std::atomic<bool> fft_recorded{false};  // a recorded launch names fft_key
@@ -1525,12 +1543,19 @@ static tp_status ks_launch(tp_ks_ctx* c, int mode, const tp::KsKernelParams& kp,
     return TP_OK;
 }
 
+tp_status tp_debug_ks_modular(tp_ks_ctx* c, int on) {
+    if (!c) return fail(TP_ERR_PARAM, "null context");
+    std::lock_guard<std::mutex> lk(c->mu);
+    c->modular = on != 0;
+    c->fft_on = !c->modular && c->loge == 2;
+    return TP_OK;
+}
+
 tp_status tp_ks_set_tile(tp_ks_ctx* c, uint32_t coef_per_thread) {
     if (!c) return fail(TP_ERR_PARAM, "null context");
     if (coef_per_thread != 4 && coef_per_thread != 8) return fail(TP_ERR_PARAM, "tile must be 4 or 8");
     const int loge = coef_per_thread == 4 ? 2 : 3;
     std::lock_guard<std::mutex> lk(c->mu);
-    c->fft_on = false;  // a tile set by name runs the modular kernels
     if (loge == c->loge) return TP_OK;
     if (c->logs > 0) return fail(TP_ERR_PARAM, "ring sizes above 4096 run on clusters with 4 coefficients per thread");
     TP_CUDA(cudaSetDevice(c->device));
@@ -1550,6 +1575,7 @@ tp_status tp_ks_set_tile(tp_ks_ctx* c, uint32_t coef_per_thread) {
         c->key = nk;
     }
     c->loge = loge;
+    c->fft_on = !c->modular && loge == 2;
     return TP_OK;
 }
 

@@ -88,7 +88,8 @@ tp_status tp_br_upload_key(tp_br_ctx* ctx, const uint64_t* brk_host, uint64_t wo
 tp_status tp_br_blind_rotate(tp_br_ctx* ctx, uint64_t* result, const uint64_t* lwe, const uint64_t* acc,
                              int out_coef);
 
-/* Batched form of the same call on device buffers: rotation b reads
+/* Batched form of the same call on device buffers (the launch form is chosen as
+ * under tp_br_set_tile): rotation b reads
  * lwes + b*lwe_stride and accs + b*acc_stride (acc_stride 0 = one accumulator
  * shared by the whole batch) and writes results + b*2N. Asynchronous on
  * `stream`; runs as one persistent launch whose accumulators stay on chip for
@@ -104,7 +105,17 @@ tp_status tp_br_blind_rotate_batch_host(tp_br_ctx* ctx, uint64_t batch, uint64_t
                                         const uint64_t* lwes, uint64_t lwe_stride, const uint64_t* accs,
                                         uint64_t acc_stride, int out_coef, void* stream);
 
-/* Tile of the rotation kernel: coefficients per thread (8: N/8 threads per
+/* Launch forms. A new context chooses its kernel by the size of each batch: for
+ * CGGI at N = 1024 .. 4096 with two to four digits the double-precision transforms
+ * (exact for keys that pass an error bound checked at upload), a rotation on one to
+ * eight blocks; for other sets the modular kernels on one, two or four blocks, or
+ * at N = 8192 and 16384 wider clusters; the rest behind full waves may run in a
+ * launch of its own. The settings below (tile, split, form, radix) name a modular
+ * kernel instead. While all of them are a new context's own values the choice by
+ * batch size stands, and setting them back restores it; the getters report these
+ * settings, whatever form a batch runs in. Every form gives the same words.
+ *
+ * Tile of the rotation kernel: coefficients per thread (8: N/8 threads per
  * rotation with radix-8 NTT passes; 4: N/4 threads, radix-4 passes, fewer
  * registers per thread so more warps per SM). Changing it after the key is
  * uploaded re-lays the key out on the device (twice the key's memory while it
@@ -114,7 +125,8 @@ tp_status tp_br_blind_rotate_batch_host(tp_br_ctx* ctx, uint64_t batch, uint64_t
 tp_status tp_br_set_tile(tp_br_ctx* ctx, uint32_t coef_per_thread);
 uint32_t tp_br_get_tile(const tp_br_ctx* ctx);
 
-/* Thread blocks per rotation: 1 (default), 2 or 4. With 2, a cluster of two
+/* Thread blocks per rotation of the modular kernels: 1 (default: chosen by batch
+ * size), 2 or 4. With 2, a cluster of two
  * blocks on two SMs rotates each ciphertext, each block owning one accumulator
  * half and its gadget rows and exchanging partial sums with the other through
  * distributed shared memory: about half the latency per rotation, for batches
@@ -224,7 +236,9 @@ uint64_t tp_ks_key_words(const tp_ks_ctx* ctx);
  * Recorded launches use the new key, as with tp_br_upload_key. */
 tp_status tp_ks_upload_key(tp_ks_ctx* ctx, const uint64_t* key_host, uint64_t words);
 
-/* Coefficients per thread of the key-switching kernels (4 or 8; default 4):
+/* Coefficients per thread of the modular key-switching kernels (4 or 8; default 4,
+ * which leaves the choice of the kernel open: digit-staged RLWE switches, and
+ * double-precision merges, traces and splits at N = 1024 and 2048):
  * N/4 or N/8 threads per ciphertext. The resident key is re-laid out for the
  * new tile. Results do not depend on it. */
 tp_status tp_ks_set_tile(tp_ks_ctx* ctx, uint32_t coef_per_thread);
@@ -414,6 +428,12 @@ const char* tp_server_last_error(void);
 tp_status tp_server_run_poisson(tp_server* srv, double rate, double seconds, const double* mix, uint32_t nsets,
                                 const uint64_t* const* pool_lwe, const uint64_t* const* pool_acc,
                                 const uint64_t* pool_n, uint64_t seed);
+
+/* For tests and profiles: keeps a context on the modular kernels of its settings,
+ * whatever the batch size, as for a key whose double-precision products are not
+ * proven exact (0: the choice stands again). */
+tp_status tp_debug_modular(tp_br_ctx* ctx, int on);
+tp_status tp_debug_ks_modular(tp_ks_ctx* ctx, int on);
 
 /* Diagnostic: element-wise Goldilocks primitives of the kernels on device
  * buffers, for testing them against exact integer arithmetic. op: 0 a+b,
