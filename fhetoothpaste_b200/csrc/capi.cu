@@ -372,17 +372,18 @@ static cudaLaunchConfig_t br_fftc_config(const tp_br_ctx* c, int i, unsigned clu
     return cfg;
 }
 
-// Picks the double-precision kernel of a parameter set: the fewest limbs whose error bound
-// holds for keys of random words (fewer limbs: less key to read and fewer transforms). The
-// key itself is checked at upload. Without a kernel the modular forms run.
+// Picks the double-precision kernel of a parameter set: the fewest limbs whose error bound holds for
+// keys of random words, the largest of their polynomials included (kFftLimbs). The key itself is
+// checked at upload. Without a kernel the modular forms run.
 static void br_setup_fft(tp_br_ctx* c) {
     if (c->prm.variant == TP_BR_BMMP_BINARY) return;
-    for (int limbs = 3; limbs <= 4; ++limbs) {
+    for (const auto& [limbs, share] : tp::kFftLimbs) {
         const bool halves = c->logn == 12;
         const void* k = halves ? tp::br_fft_halves_ptr(c->logn, c->prm.variant, c->prm.digits, limbs)
                                : tp::br_fft_kernel_ptr(c->logn, c->prm.variant, c->prm.digits, limbs);
         c->fft_limbs = limbs;
-        if (!k || !br_fft_key_exact(c, tp::fft_typical_norm2(c->logn - 1, limbs))) continue;
+        const uint64_t polys = c->key_words / c->prm.ring_dim;
+        if (!k || !br_fft_key_exact(c, tp::fft_random_norm2(c->logn - 1, limbs, polys, share))) continue;
         const size_t smem = halves ? tp::br_fft_halves_smem(c->logn, (int)c->prm.digits, limbs, c->prm.lwe_dim)
                                    : tp::br_fft_smem(c->logn, (int)c->prm.digits, limbs, c->prm.lwe_dim);
         int per_sm = 0;
@@ -775,12 +776,16 @@ tp_status tp_br_upload_key(tp_br_ctx* c, const uint64_t* brk, uint64_t words) {
     unsigned long long v = 0;
     if (e == cudaSuccess) e = cudaStreamSynchronize(work);
     if (e == cudaSuccess && fft) e = cudaMemcpy(&v, c->norm2, sizeof v, cudaMemcpyDeviceToHost);
-    // Without it the modular forms run; the buffer stays, a recorded launch may still name it. What
-    // such a launch must not read is made unlike any key.
+    // Without it the modular forms run, and the transforms go. Where a recorded launch names them they
+    // stay, made unlike any key: it must not read them.
     bool exact = e == cudaSuccess && st == TP_OK && fft && br_fft_key_exact(c, (double)v);
     const unsigned int one = 1;
     if (exact) e = cudaMemcpy(c->exact, &one, sizeof one, cudaMemcpyHostToDevice);
     else if (c->fft_recorded) cudaMemset(c->fft_key, 0xFF, c->key_words * 8 * c->fft_limbs);
+    else if (c->fft_key) {
+        cudaFree(c->fft_key);
+        c->fft_key = nullptr;
+    }
     if (e != cudaSuccess) st = fail(TP_ERR_CUDA, "key upload: %s", cudaGetErrorString(e));
     for (int i = 0; i < 2; ++i) {
         if (copied[i]) cudaEventDestroy(copied[i]);
@@ -1272,10 +1277,10 @@ static bool ks_fft_key_exact(const tp_ks_ctx* c, double norm2) {
 
 static void ks_setup_fft(tp_ks_ctx* c) {
     if (c->kind != 2) return;
-    for (int limbs = 3; limbs <= 4; ++limbs) {
+    for (const auto& [limbs, share] : tp::kFftLimbs) {
         const void* k = tp::ks_fft_kernel_ptr(c->logn, c->digits, limbs);
         c->fft_limbs = limbs;
-        if (!k || !ks_fft_key_exact(c, tp::fft_typical_norm2(c->logn - 1, limbs))) continue;
+        if (!k || !ks_fft_key_exact(c, tp::fft_random_norm2(c->logn - 1, limbs, c->key_words / c->N, share))) continue;
         const size_t smem = tp::ks_fft_smem(c->logn, limbs);
         int per_sm = 0;
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1451,6 +1456,10 @@ static cudaError_t ks_upload_fft(tp_ks_ctx* c, uint64_t* stage) {
     const unsigned int one = 1;
     if (exact) e = cudaMemcpy(c->exact, &one, sizeof one, cudaMemcpyHostToDevice);
     else if (c->fft_recorded) cudaMemset(c->fft_key, 0xFF, c->key_words * 8 * c->fft_limbs);  // unlike any key
+    else {
+        cudaFree(c->fft_key);
+        c->fft_key = nullptr;
+    }
     c->fft_ready = exact && e == cudaSuccess;
     return e;
 }

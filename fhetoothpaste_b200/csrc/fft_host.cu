@@ -287,9 +287,16 @@ bool fft_exact(int logk, uint32_t rows, double dmax, double norm2, int limbs, in
     return s * units * std::ldexp(1.0, -53) < 0.49 && largest < std::ldexp(1.0, 51);
 }
 
-double fft_typical_norm2(int logk, int limbs) {
-    const double b = (double)fft_limb_base(limbs);
-    return 1.05 * std::ldexp(b * b / 12.0, logk + 1);
+double fft_random_norm2(int logk, int limbs, uint64_t polys, double share) {
+    // N squares of numbers uniform in [-b/2, b/2]: mean N b^2 / 12, deviation sqrt(0.8 / N) of it, close
+    // to normal; the largest of m such sums exceeds z deviations in m Q(z) of the keys (m Q(z) small)
+    const double b = (double)fft_limb_base(limbs), N = std::ldexp(1.0, logk + 1), m = (double)polys * limbs;
+    double lo = 0.0, hi = 20.0;
+    for (int i = 0; i < 60; ++i) {
+        const double z = 0.5 * (lo + hi);
+        (m * 0.5 * std::erfc(z / std::sqrt(2.0)) > share ? lo : hi) = z;
+    }
+    return N * b * b / 12.0 * (1.0 + hi * std::sqrt(0.8 / N));
 }
 
 void fft_key_launch(double2* dst, const uint64_t* src, uint64_t polys, uint64_t first, uint32_t G, uint32_t rows,

@@ -36,8 +36,14 @@ cudaError_t fft_tables(int device, int logk, const FftTables** out);
 // The magnitude condition of the rounding (below 2^51) is part of the test.
 bool fft_exact(int logk, uint32_t rows, double dmax, double norm2, int limbs, int sets);
 
-// The squared norm that uniformly random key words give, and a little more.
-double fft_typical_norm2(int logk, int limbs);
+// The squared norm that the largest limb polynomial of a key of `polys` polynomials of uniformly
+// random words exceeds in `share` of the keys.
+double fft_random_norm2(int logk, int limbs, uint64_t polys, double share);
+
+// Limb counts in the order of preference: the fewest (less key to read, fewer transforms) whose bound
+// one key of a thousand fails, four where most keys pass, three where most keys pass.
+struct FftLimbs { int limbs; double share; };
+constexpr FftLimbs kFftLimbs[] = {{3, 1e-3}, {4, 0.5}, {3, 0.5}};
 
 // Transforms `polys` key polynomials of N = 2n canonical coefficient words: polynomial
 // first + i sits at src + i N and is ((it G + g) rows + r) 2 + h of the key, stored as
