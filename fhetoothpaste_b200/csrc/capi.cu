@@ -220,6 +220,19 @@ uint32_t inv_mod_2n(uint32_t t, uint32_t two_n) {
 
 }  // namespace
 
+// Device memory for a key's limb transforms (three or four times the key) into *p, unless it is there.
+// They are optional, so they take an eighth of the free memory at most: what a program allocates
+// later, other contexts among it, finds the room it had. False: the modular forms run.
+static bool transforms_alloc(double2** p, uint64_t bytes) {
+    if (*p) return true;
+    size_t room = 0, total = 0;
+    if (cudaMemGetInfo(&room, &total) == cudaSuccess && tp::fft_key_fits(bytes, room) && cudaMalloc(p, bytes) == cudaSuccess)
+        return true;
+    cudaGetLastError();
+    *p = nullptr;
+    return false;
+}
+
 struct tp_br_ctx {
     tp_br_params prm{};
     int device = 0;
@@ -735,10 +748,7 @@ tp_status tp_br_upload_key(tp_br_ctx* c, const uint64_t* brk, uint64_t words) {
     cudaError_t e = cudaMemset(c->exact, 0, 3 * sizeof(unsigned int));  // and norm2
     bool fft = c->fft_kernel != nullptr;
     c->fft_ready = false;
-    if (fft && !c->fft_key && cudaMalloc(&c->fft_key, c->key_words * 8 * c->fft_limbs) != cudaSuccess) {
-        cudaGetLastError();
-        fft = false;
-    }
+    if (fft) fft = transforms_alloc(&c->fft_key, c->key_words * 8 * c->fft_limbs);
     cudaStream_t copy = nullptr, work = nullptr;  // ordered with the legacy stream, not with each other
     cudaEvent_t copied[2] = {}, done[2] = {};
     if (e == cudaSuccess) e = cudaStreamCreate(&copy);
@@ -1440,10 +1450,7 @@ static cudaError_t ks_upload_fft(tp_ks_ctx* c, uint64_t* stage) {
     c->fft_ready = false;
     unsigned long long v = 0;
     const uint64_t polys = c->key_words / c->N;
-    if (!c->fft_key && cudaMalloc(&c->fft_key, c->key_words * 8 * c->fft_limbs) != cudaSuccess) {
-        cudaGetLastError();
-        return cudaSuccess;
-    }
+    if (!transforms_alloc(&c->fft_key, c->key_words * 8 * c->fft_limbs)) return cudaSuccess;
     cudaError_t e = cudaMemset(c->norm2, 0, 2 * sizeof *c->norm2);  // and *exact
     tp::scale_kernel<<<(unsigned)std::min<uint64_t>((c->key_words + 255) / 256, 65535), 256>>>(stage, stage, c->key_words, 1);
     tp::note_launch();

@@ -45,6 +45,10 @@ double fft_random_norm2(int logk, int limbs, uint64_t polys, double share);
 struct FftLimbs { int limbs; double share; };
 constexpr FftLimbs kFftLimbs[] = {{3, 1e-3}, {4, 0.5}, {3, 0.5}};
 
+// Whether a key's transforms of `bytes` may be allocated out of `room` free bytes.
+constexpr bool fft_key_fits(uint64_t bytes, uint64_t room) { return bytes <= room / 8; }
+static_assert(fft_key_fits(1, 8) && !fft_key_fits(2, 15) && fft_key_fits(1ull << 32, 1ull << 35));
+
 // Transforms `polys` key polynomials of N = 2n canonical coefficient words: polynomial
 // first + i sits at src + i N and is ((it G + g) rows + r) 2 + h of the key, stored as
 // [it][limb][m < 8][r][2g + h][lane < n/8] double2 (slot lane + m n/8), scaled by 1/n.

@@ -75,7 +75,11 @@ uint64_t tp_br_key_words(const tp_br_ctx* ctx);
 /* Uploads a key in that reference layout from host memory (`words` must equal
  * tp_br_key_words) and re-lays it out on the device. Synchronous. Launches recorded
  * before (tp_graph, or a caller's own stream capture) rotate with the new key when
- * they are replayed; record them again after a change of the tile. */
+ * they are replayed; record them again after a change of the tile. The device holds
+ * the key once and, where a double-precision form exists for the set, three or four
+ * more times as transforms (ternary N = 2048, l = 3, n = 630: 0.25 + 0.74 GB; N = 4096,
+ * n = 900: 0.7 + 2.8 GB). These are left out, and the modular kernels run, where they
+ * would take more than an eighth of the free device memory. */
 tp_status tp_br_upload_key(tp_br_ctx* ctx, const uint64_t* brk_host, uint64_t words);
 
 /* Drop-in for BlindRotator::BlindRotate(result, lwe, acc, output_as_coefficients)
@@ -233,7 +237,8 @@ tp_status tp_pack_create(uint32_t ring_dim, uint64_t basis, uint32_t digits, int
 tp_status tp_ks_destroy(tp_ks_ctx* ctx);
 uint64_t tp_ks_key_words(const tp_ks_ctx* ctx);
 /* Host key in the reference layout above; re-laid out on the device. Synchronous.
- * Recorded launches use the new key, as with tp_br_upload_key. */
+ * Recorded launches use the new key, and packing keys have transforms beside them,
+ * as with tp_br_upload_key. */
 tp_status tp_ks_upload_key(tp_ks_ctx* ctx, const uint64_t* key_host, uint64_t words);
 
 /* Coefficients per thread of the modular key-switching kernels (4 or 8; default 4,
@@ -327,7 +332,9 @@ typedef struct tp_lwe_ks_ctx tp_lwe_ks_ctx;
 /* LWE -> LWE key switching, LWEConversionContext(distr, modulus, n_in, n_out,
  * basis, digits, std) (lib/include/operators/endo_glwe_conversion.h:28), on the
  * Goldilocks modulus. Key: the converter's m_ksk, n_in x digits x (n_out+1)
- * (KeyGen, lib/src/operators/lwe_conversion.cpp:174-203), used as laid out. */
+ * (KeyGen, lib/src/operators/lwe_conversion.cpp:174-203), used as laid out and, for
+ * digits of up to 16 bits, held a second time as bytes for the tensor cores; the
+ * context keeps up to 512 MB of workspace between calls. */
 tp_status tp_lwe_ks_create(uint64_t modulus, uint32_t n_in, uint32_t n_out, uint64_t basis, uint32_t digits,
                            int device, tp_lwe_ks_ctx** out);
 tp_status tp_lwe_ks_destroy(tp_lwe_ks_ctx* ctx);
