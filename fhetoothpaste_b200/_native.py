@@ -140,6 +140,7 @@ def lib() -> ctypes.CDLL:
                                                  U64]),
         "tp_debug_modular": (ctypes.c_int, [VP, ctypes.c_int]),
         "tp_debug_ks_modular": (ctypes.c_int, [VP, ctypes.c_int]),
+        "tp_debug_lwe_timeout": (ctypes.c_int, [VP, VP]),
         "tp_debug_arith": (ctypes.c_int, [ctypes.c_int, U64, VP, VP, VP, VP, VP]),
         "tp_measure_int_peak": (ctypes.c_int, [ctypes.c_int, ctypes.POINTER(ctypes.c_double),
                                                 ctypes.POINTER(ctypes.c_double)]),

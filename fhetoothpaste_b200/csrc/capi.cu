@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -220,6 +221,24 @@ uint32_t inv_mod_2n(uint32_t t, uint32_t two_n) {
 
 }  // namespace
 
+// A host-mapped word that a kernel sets when one of its waits ran out, shared by a context and the
+// graphs recorded from it.
+using TimeoutWord = std::shared_ptr<int>;
+const char* const kLweTimeout = "a wait inside an earlier LWE key switch ran out; its results are not valid";
+static TimeoutWord timeout_word() {
+    int* p = nullptr;
+    if (cudaHostAlloc(&p, sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    *p = 0;
+    return TimeoutWord(p, [](int* q) { cudaFreeHost(q); });
+}
+// Whether a wait ran out since the last question, which is reported once.
+static bool timed_out(const TimeoutWord& w) {
+    return w && *(volatile int*)w.get() && __atomic_exchange_n(w.get(), 0, __ATOMIC_ACQ_REL);
+}
+
 // Device memory for a key's limb transforms (three or four times the key) into *p, unless it is there.
 // They are optional, so they take an eighth of the free memory at most: what a program allocates
 // later, other contexts among it, finds the room it had. False: the modular forms run.
@@ -289,6 +308,7 @@ struct tp_br_ctx {
     bool open = true;
     bool modular = false;         // tp_debug_modular
     std::atomic<bool> fft_recorded{false};  // a recorded launch names fft_key
+    TimeoutWord epilogue_timeout;           // of the key switch last recorded behind a rotation
     // workspace for host-pointer calls
     uint64_t* ws = nullptr;
     uint64_t ws_words = 0;
@@ -1038,6 +1058,7 @@ tp_status tp_br_check(tp_br_ctx* c, void* stream) {
     unsigned int flags = 0;
     TP_CUDA(cudaMemcpy(&flags, c->err, sizeof flags, cudaMemcpyDeviceToHost));
     TP_CUDA(cudaMemset(c->err, 0, sizeof flags));
+    if (timed_out(c->epilogue_timeout)) return fail(TP_ERR_TIMEOUT, kLweTimeout);
     if (flags & 2u) return fail(TP_ERR_TIMEOUT, "a wait between the blocks of a rotation ran out; its results are not valid");
     if (flags & 1u) return fail(TP_ERR_PARAM, "an LWE word was outside [0, 2N); it was reduced mod 2N");
     return TP_OK;
@@ -1109,6 +1130,7 @@ tp_status tp_sample_extract_batch(uint32_t ring_dim, uint64_t batch, uint64_t* o
 
 struct tp_graph {
     cudaGraphExec_t exec = nullptr;
+    TimeoutWord timeout;   // of the key switch among its kernels
     uint8_t* ws = nullptr; // workspace that the graph's kernels use
     int device = 0;
     uint64_t kernels = 0;  // launches per replay: kernel nodes but those standing by
@@ -1170,6 +1192,7 @@ tp_status tp_br_batch_graph_create(tp_br_ctx* c, uint64_t batch, uint64_t* resul
 
 tp_status tp_graph_launch(tp_graph* g, void* stream) {
     if (!g) return fail(TP_ERR_PARAM, "null graph");
+    if (timed_out(g->timeout)) return fail(TP_ERR_TIMEOUT, kLweTimeout);
     TP_CUDA(cudaSetDevice(g->device));
     TP_CUDA(cudaGraphLaunch(g->exec, (cudaStream_t)stream));
     if (!tp::t_capturing) tp::g_launches.fetch_add(g->kernels, std::memory_order_relaxed);
@@ -1973,7 +1996,7 @@ struct tp_lwe_ks_ctx {
     uint32_t kpad = 0;            // n_in * digits rounded up to the K step
     uint8_t* kbytes = nullptr;    // key bytes, 8 (n_out + 1) rows of kpad
     cudaMemPool_t pool = nullptr; // workspaces of the calls in flight; kept up to 512 MB, gone with the context
-    int* err = nullptr;           // host-mapped: a kernel's wait ran out
+    TimeoutWord err;              // a kernel's wait ran out
 };
 
 namespace {
@@ -2028,13 +2051,12 @@ cudaError_t lwe_mma_setup(tp_lwe_ks_ctx* c) {
                                                (int)tp::mma_smem(2));
         if (e == cudaSuccess && !c->pool) e = cudaMemPoolCreate(&c->pool, &pp);
         if (e == cudaSuccess) e = cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep);
-        if (e == cudaSuccess && !c->err) e = cudaHostAlloc(&c->err, sizeof(int), cudaHostAllocMapped);
+        if (e == cudaSuccess && !c->err && !(c->err = timeout_word())) e = cudaErrorMemoryAllocation;
         if (e == cudaSuccess) e = cudaMalloc(&c->kbytes, 8ull * (c->n_out + 1) * kpad);
         if (e != cudaSuccess) {
             cudaGetLastError();
             return cudaSuccess;
         }
-        *c->err = 0;
         c->planes = planes;
         c->kpad = kpad;
     }
@@ -2052,7 +2074,7 @@ cudaError_t lwe_mma_setup(tp_lwe_ks_ctx* c) {
 tp_status lwe_ks_launch(const tp_lwe_ks_ctx* c, tp::LweKsParams kp, uint8_t* ws, cudaStream_t st) {
     bool mma = c->planes > 0;
     uint8_t* own = nullptr;
-    if (mma && *(volatile int*)c->err) return fail(TP_ERR_TIMEOUT, "a wait inside an earlier LWE key switch ran out");
+    if (timed_out(c->err)) return fail(TP_ERR_TIMEOUT, kLweTimeout);
     tp::LweMmaPlan plan{};
     if (mma) {
         plan = lwe_mma_plan(c, kp.batch);
@@ -2083,7 +2105,7 @@ tp_status lwe_ks_launch(const tp_lwe_ks_ctx* c, tp::LweKsParams kp, uint8_t* ws,
         const uint32_t rows = (uint32_t)std::min<uint64_t>(plan.rows, kp.batch - r0);
         const unsigned db = (unsigned)std::min<uint64_t>(((uint64_t)rows * (c->kpad / 16) + 255) / 256, 65535);
         const unsigned fb = (unsigned)std::min<uint64_t>(((uint64_t)rows * width + 255) / 256, 65535);
-        tp::LweMmaParams mp{part, rows, plan.rows_pad, width, c->kpad / tp::kMmaK, plan.splits, c->err};
+        tp::LweMmaParams mp{part, rows, plan.rows_pad, width, c->kpad / tp::kMmaK, plan.splits, c->err.get()};
         const dim3 grid((rows + tp::kMmaRows - 1) / tp::kMmaRows, (width + tp::kMmaWords - 1) / tp::kMmaWords, plan.splits);
         if (c->planes == 1) {
             tp::lwe_digits_kernel<1><<<db, 256, 0, st>>>(ws, kp, r0, rows, plan.rows_pad, c->kpad);
@@ -2158,7 +2180,6 @@ tp_status tp_lwe_ks_destroy(tp_lwe_ks_ctx* c) {
     cudaFree(c->cterm);
     cudaFree(c->kbytes);
     if (c->pool) cudaMemPoolDestroy(c->pool);
-    cudaFreeHost(c->err);
     delete c;
     return TP_OK;
 }
@@ -2185,6 +2206,16 @@ tp_status tp_lwe_ks_upload_key(tp_lwe_ks_ctx* c, const uint64_t* ksk, uint64_t w
     TP_CUDA(cudaDeviceSynchronize());
     c->kp.cterm = c->cterm;
     c->key_ready = true;
+    return TP_OK;
+}
+
+tp_status tp_debug_lwe_timeout(tp_lwe_ks_ctx* c, void* stream) {
+    if (!c) return fail(TP_ERR_PARAM, "null context");
+    if (!c->planes) return fail(TP_ERR_STATE, "the context has no tensor-core form");
+    TP_CUDA(cudaSetDevice(c->device));
+    tp::lwe_timeout_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(c->err.get());
+    tp::note_launch();
+    TP_CUDA(cudaGetLastError());
     return TP_OK;
 }
 
@@ -2295,6 +2326,7 @@ tp_status tp_pbs_graph_create(tp_br_ctx* br, tp_lwe_ks_ctx* ks, uint64_t batch, 
     }
     auto* gr = new tp_graph();
     gr->ws = ws;
+    gr->timeout = br->epilogue_timeout = ks->err;
     gr->device = br->device;
     gr->kernels = graph_kernel_nodes(g) - tp::t_standby;
     e = cudaGraphInstantiate(&gr->exec, g, 0);

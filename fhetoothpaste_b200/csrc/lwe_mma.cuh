@@ -191,6 +191,14 @@ lwe_mma_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__
     }
 }
 
+// tp_debug_lwe_timeout: a wait on a barrier that nothing completes, reported as lwe_mma_kernel reports its own.
+__global__ void lwe_timeout_kernel(int* err) {
+    __shared__ uint64_t bar;
+    mbar_init(&bar, 1);
+    mbar_init_fence();
+    if (!mbar_wait(&bar, 0, 64)) *(volatile int*)err = 1;
+}
+
 // Byte planes of the digits of rows row0 .. row0 + rows - 1: plane d, row r, position
 // k = i l + j holds byte d of (x_i + corr) >> dshift[j] & dmask[j]; zero past n_in l. A
 // thread makes 16 neighbouring positions (16-byte stores).

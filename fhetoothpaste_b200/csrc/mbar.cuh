@@ -15,8 +15,8 @@ __device__ __forceinline__ void mbar_expect(uint64_t* b, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
 }
 // Waits for the phase of parity `ph`; gives up (false) after a few seconds.
-__device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t ph) {
-    for (uint32_t i = 0; i < (1u << 22); ++i) {
+__device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t ph, uint32_t tries = 1u << 22) {
+    for (uint32_t i = 0; i < tries; ++i) {
         uint32_t ok;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"

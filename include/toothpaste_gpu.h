@@ -33,7 +33,8 @@ typedef enum {
     TP_ERR_PARAM = 1,   /* invalid argument or unsupported parameter set */
     TP_ERR_OOM = 2,     /* device allocation failed */
     TP_ERR_CUDA = 3,    /* a CUDA call failed (message in tp_last_error) */
-    TP_ERR_TIMEOUT = 4, /* a bounded host-side wait ran out (serving: a result or a drain) */
+    TP_ERR_TIMEOUT = 4, /* a bounded wait ran out: on the host (serving: a result or a drain), or inside an
+                           earlier launch whose results are then not valid */
     TP_ERR_LAYOUT = 5,  /* key size or layout does not match the context */
     TP_ERR_STATE = 6    /* call order: e.g. rotate before a key was uploaded */
 } tp_status;
@@ -177,7 +178,9 @@ tp_status tp_br_autotune(tp_br_ctx* ctx, uint64_t batch, uint32_t* best_coef_per
                          double* best_rotations_per_s);
 
 /* Waits for the context's work on `stream` and reports device-side input
- * errors seen since the last check (TP_ERR_PARAM for out-of-range LWE words). */
+ * errors seen since the last check (TP_ERR_PARAM for out-of-range LWE words,
+ * TP_ERR_TIMEOUT for a wait that ran out in a rotation or in the key switch of a
+ * bootstrap graph recorded from the context). */
 tp_status tp_br_check(tp_br_ctx* ctx, void* stream);
 
 /* SampleExtract at index 0 of a batch of RLWE ciphertexts in the coefficient
@@ -344,7 +347,9 @@ tp_status tp_lwe_ks_upload_key(tp_lwe_ks_ctx* ctx, const uint64_t* key_host, uin
 /* Batched LWEtoLWEConverter::Convert(out, in) (lwe_conversion.cpp:205-239):
  * in b has n_in+1 words, out b has n_out+1 words; out[n_out] = in[n_in] and
  * out -= sum of signed digits times key rows (the reference expects out[0..n_out)
- * pre-zeroed). Asynchronous. */
+ * pre-zeroed). Asynchronous. A wait that ran out inside an earlier switch of the
+ * context is reported once, by the next call or graph launch (TP_ERR_TIMEOUT,
+ * nothing launched). */
 tp_status tp_lwe_ks_batch(tp_lwe_ks_ctx* ctx, uint64_t batch, uint64_t* out_dev, const uint64_t* in_dev, void* stream);
 
 /* ModulusSwitch (lib/src/static/modulus_switching.cpp:36-93) in place on a
@@ -441,6 +446,8 @@ tp_status tp_server_run_poisson(tp_server* srv, double rate, double seconds, con
  * proven exact (0: the choice stands again). */
 tp_status tp_debug_modular(tp_br_ctx* ctx, int on);
 tp_status tp_debug_ks_modular(tp_ks_ctx* ctx, int on);
+/* For tests: a kernel whose short wait runs out reports it as a key switch would. */
+tp_status tp_debug_lwe_timeout(tp_lwe_ks_ctx* ctx, void* stream);
 
 /* Diagnostic: element-wise Goldilocks primitives of the kernels on device
  * buffers, for testing them against exact integer arithmetic. op: 0 a+b,
