@@ -177,6 +177,17 @@ int sm_count(int device) {
     return v > 0 ? v : 1;
 }
 
+// Lets launches of `k` use up to `bytes` of dynamic shared memory. The limit is the kernel's, and what a
+// rotation needs grows with the LWE dimension: contexts share it, so it is never lowered.
+cudaError_t allow_smem(const void* k, size_t bytes) {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    cudaFuncAttributes a;
+    const cudaError_t e = cudaFuncGetAttributes(&a, k);
+    if (e != cudaSuccess || (size_t)a.maxDynamicSharedSizeBytes >= bytes) return e;
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
 // Signed-digit constants of SignedGadgetDecomposeRepNTT on a 64-bit modulus
 // (lib/include/static/gadget_decomp.h:16-28,156-205).
 void signed_digit_consts(int beta, uint32_t digits, uint64_t& corr, uint32_t* dshift, uint64_t* dmask,
@@ -323,7 +334,7 @@ static tp_status br_setup_cluster(tp_br_ctx* c) {
         const int S = 1 << logs;
         const uint32_t T = c->prm.ring_dim >> (logs + 2);
         if (!k || smem > 227u * 1024u) return false;
-        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_smem(k, smem);
         if (e == cudaSuccess && S > 8) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         int clusters = 0;
         if (e == cudaSuccess) {
@@ -421,7 +432,7 @@ static void br_setup_fft(tp_br_ctx* c) {
                                    : tp::br_fft_smem(c->logn, (int)c->prm.digits, limbs, c->prm.lwe_dim);
         int per_sm = 0;
         cudaError_t e = smem <= 227u * 1024u
-                            ? cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                            ? allow_smem(k, smem)
                             : cudaErrorInvalidValue;
         if (e == cudaSuccess && halves) {  // clusters of two blocks
             cudaLaunchConfig_t cfg = {};
@@ -450,7 +461,7 @@ static void br_setup_fft(tp_br_ctx* c) {
             cfg.blockDim = dim3(tp::br_fft_threads(c->logn, (int)c->prm.digits, limbs));
             cfg.dynamicSmemBytes = f.smem;
             e = kp && f.smem <= 227u * 1024u
-                    ? cudaFuncSetAttribute(kp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem)
+                    ? allow_smem(kp, f.smem)
                     : cudaErrorInvalidValue;
             if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&f.cap, kp, &cfg);
             if (e == cudaSuccess && f.cap > 0) f.k = kp;
@@ -463,7 +474,7 @@ static void br_setup_fft(tp_br_ctx* c) {
             if (!kc || f.smem > 227u * 1024u) continue;
             cudaLaunchAttribute attr;
             const cudaLaunchConfig_t cfg = br_fftc_config(c, i, 1, nullptr, &attr);
-            e = cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem);
+            e = allow_smem(kc, f.smem);
             if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&f.cap, kc, &cfg);
             if (e == cudaSuccess && f.cap > 0) f.k = kc;
             else cudaGetLastError();
@@ -650,7 +661,7 @@ tp_status tp_br_create(const tp_br_params* p, int device, tp_br_ctx** out) {
     for (int lg = 2; lg <= 3; ++lg) {
         const void* k = tp::br_kernel_lookup(c->logn, p->variant, lg);
         const size_t smem = tp::br_smem_words(c->logn, p->variant, p->lwe_dim, lg) * 8;
-        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = allow_smem(k, smem);
         int per_sm = 0;
         if (e == cudaSuccess)
             e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, (int)(N >> lg), smem);
@@ -672,7 +683,7 @@ tp_status tp_br_create(const tp_br_params* p, int device, tp_br_ctx** out) {
         const size_t smem = tp::br_smem_words(c->logn, p->variant, p->lwe_dim, 2, (int)p->digits) * 8;
         int per_sm = 0;
         cudaError_t de = k && smem <= 227u * 1024u
-                             ? cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                             ? allow_smem(k, smem)
                              : cudaErrorInvalidValue;
         if (de == cudaSuccess) de = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, (int)(N >> 2), smem);
         if (de == cudaSuccess && per_sm > 0) {
@@ -691,7 +702,7 @@ tp_status tp_br_create(const tp_br_params* p, int device, tp_br_ctx** out) {
         const size_t smem = tp::br_smem_words(c->logn, p->variant, p->lwe_dim, 2, dl, 0, true) * 8;
         int per_sm = 0;
         cudaError_t re = k && smem <= 227u * 1024u
-                             ? cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                             ? allow_smem(k, smem)
                              : cudaErrorInvalidValue;
         if (re == cudaSuccess) re = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, (int)(N >> 2), smem);
         if (re == cudaSuccess && per_sm > 0) {
@@ -708,7 +719,7 @@ tp_status tp_br_create(const tp_br_params* p, int device, tp_br_ctx** out) {
         const void* k = tp::br_pair_kernel_lookup(c->logn, p->variant, split);
         const size_t smem = tp::br_pair_smem_words(c->logn, p->variant, p->lwe_dim, 2, split) * 8;
         int clusters = 0;
-        cudaError_t pe = k ? cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+        cudaError_t pe = k ? allow_smem(k, smem)
                            : cudaErrorInvalidValue;
         if (pe == cudaSuccess) {
             cudaLaunchConfig_t cfg = {};
