@@ -492,14 +492,17 @@ static void br_setup_fft(tp_br_ctx* c) {
 //                                  clusters 8 / 4 / 2    one block   pair        modular, pair
 //   ternary N = 2048, l = 3        0.43 / 0.56 / -       1.10 5.66   1.04 5.19   1.53  1.09
 //   binary N = 2048, l = 4         0.49 / 0.60 / -       1.32 6.58   1.22 5.99   1.72  1.04
-//   binary N = 2048, l = 3 (2^12)  0.44 / 0.54 / -       0.86 4.27   0.91 4.42   1.40  -
+//   binary N = 2048, l = 3 (2^12)  0.44 / 0.53 / -       0.83 4.27   0.91 4.42   1.40  0.84
 //   ternary N = 2048, l = 4 (2^16) 0.49 / 0.76 / -       2.08 11.4   1.46 7.65   2.06  1.31
 //   binary N = 1024, l = 4         0.37 / 0.43 / 0.57    0.63 2.65   0.66 2.54   0.98  -
 //   ternary N = 1024, l = 4 (2^16) 0.36 / 0.43 / 0.68    1.56 5.54   1.01 3.60   1.24  -
 // So: the widest cluster that takes the batch in one wave; then, at N = 2048, the modular pair in
-// its one wave; then one block, or the pair where the key polynomials read per slot and iteration
-// (2 G rows limbs) reach 64 and halving them pays for the exchanges (at N = 1024, where two
-// blocks share an SM, from the second block per SM on, or from 128).
+// its one wave, but for ternary l = 3 with three limbs, where no group of threads of the
+// double-precision pair idles forward or backward (50 rotations, n = 200: 3.39 against 3.47 in the
+// modular pair; binary, one block of the same shape, 2.80 against 2.75; n = 60: l = 2 0.72 against 0.67
+// and 0.85 against 0.85, l = 4 and all sets of four limbs 11 to 20% slower); then one block, or the pair where the key polynomials
+// read per slot and iteration (2 G rows limbs) reach 64 and halving them pays for the exchanges (at
+// N = 1024, where two blocks share an SM, from the second block per SM on, or from 128).
 //
 // Sets without a double-precision kernel: four blocks per rotation in one wave up to half the SMs
 // (beyond, where several clusters share an SM, two blocks are as fast), two in one wave, else one.
@@ -522,7 +525,8 @@ static int br_form(const tp_br_ctx* c, uint64_t batch) {
     for (int i = 2; i >= 0; --i)
         if (batch <= (uint64_t)c->fftc[i].cap) return i;
     if (c->logn == 12) return kFftHalves;
-    if (c->logn >= 11 && c->loge == 2 && batch <= (uint64_t)c->pair_cap) return kModularPair;
+    const bool pair = c->logn >= 11 && c->loge == 2 && !(c->G == 2 && c->prm.digits == 3 && c->fft_limbs == 3);
+    if (pair && batch <= (uint64_t)c->pair_cap) return kModularPair;
     const int polys = 2 * c->G * 2 * (int)c->prm.digits * c->fft_limbs;
     const bool full = c->logn >= 11 || batch > (uint64_t)c->fft_cap / 2;
     return c->fftp.k && (polys >= 128 || (polys >= 64 && full)) ? kFftPair : kFftOneBlock;

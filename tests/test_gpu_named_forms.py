@@ -76,7 +76,7 @@ def test_modular_rotations_match_reference(native, oracle, golden, name):
 
 
 # strides, a shared accumulator, results in place, evaluation-domain results, batches past a wave
-@pytest.mark.parametrize("variant,N,beta,digits,batch", [(*s, b) for s in SETS for b in (20, 310)] +
+@pytest.mark.parametrize("variant,N,beta,digits,batch", [(*s, b) for s in SETS for b in (20, 310)] + [(*SETS[0], 40)] +
                          [(v, N, 14, 3, b) for v, N in ((0, 8192), (1, 8192), (2, 8192), (1, 16384)) for b in (1, 17)])
 def test_open_forms_equal_modular_kernels(native, variant, N, beta, digits, batch):
     import torch
