@@ -17,6 +17,12 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (runs the sm_100a kernels)")
 
 
+def pytest_collection_modifyitems(items):
+    """The reference's own callers come last: their library is built from sources that are not on every
+    machine, and a run that stops at its first error should not stop there before the other files."""
+    items.sort(key=lambda item: item.path.name == "test_gpu_reference_adapter.py")
+
+
 @pytest.fixture(scope="session")
 def oracle():
     from oracle.oracle import Oracle
