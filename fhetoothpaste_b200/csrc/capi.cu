@@ -252,12 +252,14 @@ static bool timed_out(const TimeoutWord& w) {
 
 // Device memory for a key's limb transforms (three or four times the key) into *p, unless it is there.
 // They are optional, so they take an eighth of the free memory at most: what a program allocates
-// later, other contexts among it, finds the room it had. False: the modular forms run.
+// later, other contexts among it, finds the room it had (up to 32 MB are not worth the question, 80 us).
+// False: the modular forms run.
 static bool transforms_alloc(double2** p, uint64_t bytes) {
     if (*p) return true;
     size_t room = 0, total = 0;
-    if (cudaMemGetInfo(&room, &total) == cudaSuccess && tp::fft_key_fits(bytes, room) && cudaMalloc(p, bytes) == cudaSuccess)
-        return true;
+    const bool fits = bytes <= 32ull << 20 ||
+                      (cudaMemGetInfo(&room, &total) == cudaSuccess && tp::fft_key_fits(bytes, room));
+    if (fits && cudaMalloc(p, bytes) == cudaSuccess) return true;
     cudaGetLastError();
     *p = nullptr;
     return false;
