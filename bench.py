@@ -4,14 +4,14 @@ Workload (default): batched CGGI blind rotation with a ternary LWE secret,
 n = 630, N = 2048, Goldilocks, signed gadget base 2^12 with l = 3; 4096
 independent LWE ciphertexts per step, each with its own seeded 16-entry LUT
 test polynomial (trivial RLWE, coefficient domain), NTT-domain output. One
-step = one persistent launch over the whole batch.
+step = one replay of the recorded rotation of the whole batch.
 
   value  blind rotations/s with inputs resident in HBM (kernel time, CUDA events)
   e2e    the same through the host-buffer C-ABI call (tp_br_blind_rotate_batch_host):
          host->device copy of the step's LWEs and test polynomials, the launch,
          device->host copy of the results, all inside the timed region
   plain  the one-rotation-per-launch form (batch 1) for the batched/plain ratio, also
-         with the rotation split over two and four SMs (cluster kernels)
+         with the modular kernels that split a rotation over two and four SMs
 
 `--impl reference` times the reference library's own CPU blind rotation (built
 from its sources into oracle/_ref/, one rotator per host thread) on a bounded
@@ -64,6 +64,22 @@ def modmul_per_iteration(variant: int, N: int, l: int) -> int:
     if variant == 1:
         return (2 + 2 * l) * ntt_mm(N) + 8 * l * N + 4 * N
     return (2 + 2 * l) * ntt_mm(N) + 12 * l * N + 6 * N
+
+
+# key limbs of the double-precision form that each workload's rotations run (csrc/fft_host.h); BMMP has none
+FFT_LIMBS = {"cggi_ternary_n2048": 3, "cggi_binary_n1024": 4, "cggi_ternary_n4096": 4}
+FP64_PER_SM_CLOCK = 64  # FP64 fused multiply-adds
+
+
+def fp64_per_iteration(variant: int, N: int, l: int, limbs: int) -> int:
+    """FP64 instructions of one iteration in double precision: 6 a forward and 8 a backward butterfly, digit
+    conversions and roundings, 4 a complex product term, the ternary combination of two products."""
+    n = N // 2
+    stages = n // 2 * (n.bit_length() - 1)
+    comps = 2 if variant == 0 else 4
+    forward = 2 * l * (6 * stages + 2 * n)
+    backward = 2 * limbs * (8 * stages + 2 * n)
+    return forward + backward + n * 2 * l * comps * 4 * limbs + (12 * n * limbs if variant == 1 else 0)
 
 
 def workload_modmuls(variant: int, N: int, n: int, l: int, lwes: np.ndarray) -> int:
@@ -221,8 +237,12 @@ def run_reference(args, wl):
     accs = lut_polys(N, batch, 8)
     vals = []
     for s in range(args.warmup + args.steps):
-        v, threads, count, secs = cpu_reference_sample(variant, N, n, bl, l, lwes, accs,
-                                                       seconds_target=args.ref_seconds)[:4]
+        try:
+            v, threads, count, secs = cpu_reference_sample(variant, N, n, bl, l, lwes, accs,
+                                                           seconds_target=args.ref_seconds)[:4]
+        except OSError as exc:  # its library is built from the reference's sources, which are not on every machine
+            print(json.dumps({"impl": "reference", "unavailable": f"reference library not built here: {exc}"}), flush=True)
+            return
         if s >= args.warmup:
             vals.append((v, threads, count, secs))
     v = statistics.median([x[0] for x in vals])
@@ -604,8 +624,8 @@ def main():
     h2d = lwes_h.nbytes + accs_h.nbytes
     d2h = batch * 2 * N * 8
 
-    # plain form: one rotation per launch (one thread block, as the batched kernel
-    # runs it), and the same with the rotation split over two and four SMs
+    # plain form: one rotation per launch (in the form chosen for a batch of one), and by name the
+    # modular kernels on two and four SMs
     one_out = torch.empty((1, 2 * N), dtype=torch.int64, device="cuda")
     plain_reps = 3
 
@@ -631,8 +651,8 @@ def main():
         pass
     rot.set_split(1)
 
-    # roofline: algorithmic modmuls per launch over the kernel's launch time,
-    # against the measured 64x64->128 product rate of this GPU
+    # roofline: the double-precision form's FP64 instructions against the FP64 pipe at the sampled clock, or the
+    # modular form's products against the measured 64x64->128 product rate of this GPU
     import ctypes
     prod, imad = ctypes.c_double(), ctypes.c_double()
     _native.check(L.tp_measure_int_peak(local, ctypes.byref(prod), ctypes.byref(imad)))
@@ -640,6 +660,30 @@ def main():
     achieved = mm / (ms * 1e-3)
     traffic, tsrc = traffic_from_profiles(wl)
     key_bytes = kw * 8
+    fft = wl in FFT_LIMBS and timed_launches == 2 * args.steps  # the rotations, and the results' transform
+    clocks = clk.summary()
+    imad8 = imad.value / 8  # 8 IMAD issues per 64x64 modmul at the measured IMAD rate
+    products = {"achieved_gmodmul_s": round(achieved / 1e9, 1), "peak_gmodmul_s": round(prod.value / 1e9, 1),
+                "peak_source": "measured 64x64->128 IMAD-chain product rate of this GPU (tp_measure_int_peak)",
+                "frac": round(achieved / prod.value, 4), "frac_imad8": round(achieved / imad8, 4),
+                "peak_imad8": round(imad8 / 1e9, 1),
+                "imad8_source": "measured mad.lo.u32 rate / 8 IMAD per modmul (the scope table's formula)",
+                "imad_per_s": round(imad.value / 1e12, 2), "algorithmic_modmul_per_launch": mm}
+    if fft:
+        sms = torch.cuda.get_device_properties(local).multi_processor_count
+        fp64 = fp64_per_iteration(variant, N, l, FFT_LIMBS[wl]) * int(np.count_nonzero(lwes_h[:, :n]))
+        fp64_peak = FP64_PER_SM_CLOCK * sms * (clocks["sm_mhz"] or 1965.0) * 1e6
+        key_bytes *= FFT_LIMBS[wl]  # limb transforms, 8 bytes per word and limb
+        roofline = {"bound": "fp64", "achieved": round(fp64 / (ms * 1e-3) / 1e9, 1), "peak": round(fp64_peak / 1e9, 1),
+                    "unit": "G FP64 instructions/s", "frac": round(fp64 / (ms * 1e-3) / fp64_peak, 4),
+                    "peak_source": f"{FP64_PER_SM_CLOCK} a clock and SM at the sampled clock",
+                    "limiter": "L1 / shared-memory passes of the transforms (profiles/double_precision_and_tensor_kernels.md)",
+                    "modular_products": products}  # work of the modular algorithm, which this form does not do
+    else:
+        roofline = {"bound": "int32", "achieved": products["achieved_gmodmul_s"], "peak": products["peak_gmodmul_s"],
+                    "unit": "Gmodmul/s", "frac": products["frac"], "modular_products": products}
+    roofline |= {"traffic": traffic, "traffic_source": tsrc,
+                 "key_hbm": {"bytes_per_launch": key_bytes, "achieved_gbs": round(key_bytes / (ms * 1e-3) / 1e9, 1)}}
 
     plain = {"value": round(1e3 / plain_ms, 3), "unit": "BR/s", "ms_per_rotation": round(plain_ms, 3),
              "batched_over_plain": round(value / world / (1e3 / plain_ms), 1),
@@ -648,29 +692,20 @@ def main():
              "four_blocks": None if plain4_ms is None else {
                  "value": round(1e3 / plain4_ms, 3), "ms_per_rotation": round(plain4_ms, 3),
                  "batched_over_plain": round(value / world / (1e3 / plain4_ms), 1)}}
-    imad8 = imad.value / 8  # 8 IMAD issues per 64x64 modmul at the measured IMAD rate
     line = {
         "metric": "blind rotations/sec", "value": round(value, 2), "unit": "BR/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": round(ms, 3), "higher_is_better": True,
         "scaling": "weak", "vs_baseline": None, "dtype": "u64 (mod p)", "data": "synthetic",
         "gpu_launches": int(timed_launches),
         "config": bench_config(wl, batch, n),
-        "roofline": {"bound": "int32", "achieved": round(achieved / 1e9, 1), "peak": round(prod.value / 1e9, 1),
-                     "unit": "Gmodmul/s", "frac": round(achieved / prod.value, 4), "traffic": traffic,
-                     "traffic_source": tsrc,
-                     "peak_source": "measured 64x64->128 IMAD-chain product rate of this GPU (tp_measure_int_peak)",
-                     "frac_imad8": round(achieved / imad8, 4),
-                     "peak_imad8": round(imad8 / 1e9, 1),
-                     "imad8_source": "measured mad.lo.u32 rate / 8 IMAD per modmul (the scope table's formula)",
-                     "imad_per_s": round(imad.value / 1e12, 2),
-                     "algorithmic_modmul_per_launch": mm,
-                     "key_hbm": {"bytes_per_launch": key_bytes,
-                                 "achieved_gbs": round(key_bytes / (ms * 1e-3) / 1e9, 1)}},
+        "roofline": roofline,
         "e2e": {"value": round(e2e_val, 2), "unit": "BR/s", "h2d_bytes_per_step": int(h2d),
                 "d2h_bytes_per_step": int(d2h), "steps": e2e_steps},
-        "clocks": clk.summary(),
-        "launch": {"form": "CUDA graph, one kernel per step", "coef_per_thread": rot.tile,
+        "clocks": clocks,
+        "launch": {"form": f"CUDA graph, {timed_launches // args.steps} kernel(s) at work per step",
+                   "transforms": "double precision" if fft else "modular", "coef_per_thread": rot.tile,
                    "blocks_per_rotation": rot.split, "mac_form": rot.mac_form, "radix": rot.radix,
+                   "settings": "of the modular kernels; the form is chosen by batch size",
                    "key": "uniform random key words (timing does not depend on key values)"},
     }
     if rank == 0 and world == 1 and not args.no_serving:

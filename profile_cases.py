@@ -27,12 +27,11 @@ def _dev(torch, a: np.ndarray):
     return torch.from_numpy(np.ascontiguousarray(a, np.uint64).view(np.int64)).cuda()
 
 
-def _rotation(torch, variant: int, N: int, n: int, beta: int, digits: int, batch: int, tile: int = 0):
-    from fhetoothpaste_b200 import BlindRotationContext, GpuBlindRotator
+def _rotation(torch, variant: int, N: int, n: int, beta: int, digits: int, batch: int, modular: bool = True):
+    from fhetoothpaste_b200 import BlindRotationContext, GpuBlindRotator, _native
     ctx = BlindRotationContext(variant, N, n, 1 << beta, digits)
     rot = GpuBlindRotator(ctx, _u64(1, ctx.key_words()))  # key_relayout_kernel
-    if tile:
-        rot.set_tile(tile)                                 # key_retile_kernel
+    _native.check(_native.lib().tp_debug_modular(rot.handle, int(modular)))
     lw = _dev(torch, _u64(2, (batch, n + 1), 2 * N))
     ac = _dev(torch, _u64(3, (batch, 2 * N)))
     out = torch.empty((batch, 2 * N), dtype=torch.int64, device="cuda")
@@ -65,6 +64,26 @@ def case_br_ternary_n4096(torch):
 def case_br_ternary_n8192(torch):
     """br_kernel on two-CTA clusters, CGGI ternary N=8192 base 2^12 l=3, n reduced to 32, one wave (74)."""
     _rotation(torch, 1, 8192, 32, 12, 3, 74)
+
+
+def case_br_fft_pair_ternary_n2048(torch):
+    """br_fft_pair_kernel (two rotations on two blocks), CGGI ternary N=2048 l=3, n reduced to 12, two waves (296)."""
+    _rotation(torch, 1, 2048, 12, 12, 3, 296, modular=False)
+
+
+def case_br_fft_binary_n1024(torch):
+    """br_fft_kernel (one block per rotation), CGGI binary N=1024 base 2^12 l=3, n reduced to 32, two waves (592)."""
+    _rotation(torch, 0, 1024, 32, 12, 3, 592, modular=False)
+
+
+def case_br_fft_cluster_ternary_n2048(torch):
+    """br_fft_cluster_kernel (one rotation on eight blocks), CGGI ternary N=2048 l=3, n reduced to 64, batch 15."""
+    _rotation(torch, 1, 2048, 64, 12, 3, 15, modular=False)
+
+
+def case_br_fft_halves_ternary_n4096(torch):
+    """br_fft_halves_kernel (one rotation on two blocks), CGGI ternary N=4096 l=3, n reduced to 12, two waves (148)."""
+    _rotation(torch, 1, 4096, 12, 12, 3, 148, modular=False)
 
 
 def case_br_pair_ternary_n2048(torch):
@@ -101,7 +120,7 @@ def case_br_quad_ternary_n2048(torch):
 
 
 def case_pbs_epilogue_n1024(torch):
-    """lwe_ks_kernel as the bootstrap epilogue: 4096 RLWEs N=1024 -> extract -> KS to n=500
+    """lwe_mma_kernel and its digit and update kernels as the bootstrap epilogue: 4096 RLWEs N=1024 -> extract -> KS to n=500
     (base 2^16, l=4, 16 MB key) -> FLOOR switch to 2N."""
     from fhetoothpaste_b200 import GpuLWEtoLWEConverter
     N, n, l, batch = 1024, 500, 4, 4096
@@ -125,17 +144,23 @@ def case_ntt_n2048(torch):
     torch.cuda.synchronize()
 
 
-def case_rlwe_ks_n2048(torch):
-    """ks_kernel (RLWE->RLWE), 4096 ciphertexts of N=2048, base 2^16 l=4."""
-    from fhetoothpaste_b200 import GpuRLWEtoRLWEConverter
+def case_rlwe_ks_n2048(torch, modular: int = 0):
+    """ks_rlwe_kernel (RLWE->RLWE), 4096 ciphertexts of N=2048, base 2^16 l=4."""
+    from fhetoothpaste_b200 import GpuRLWEtoRLWEConverter, _native
     N, l, batch = 2048, 4, 4096
     conv = GpuRLWEtoRLWEConverter(N, 1 << 16, l, _u64(5, 2 * N * l))
+    _native.check(_native.lib().tp_debug_ks_modular(conv._h, modular))
     x = _dev(torch, _u64(6, (batch, 2 * N)))
     y = torch.zeros((batch, 2 * N), dtype=torch.int64, device="cuda")
     for _ in range(2):
         conv.convert_batch(batch, y.data_ptr(), x.data_ptr())
     torch.cuda.synchronize()
     conv.close()
+
+
+def case_rlwe_ks_general_n2048(torch):
+    """ks_kernel (RLWE->RLWE, the general form), as rlwe_ks_n2048."""
+    case_rlwe_ks_n2048(torch, modular=1)
 
 
 def case_auto_n2048(torch):
@@ -151,11 +176,12 @@ def case_auto_n2048(torch):
     ev.close()
 
 
-def case_pack_n2048(torch):
-    """pack_l0_kernel + ks_kernel merge levels: 8 packs of 2048 LWEs (n=N=2048), l=4."""
-    from fhetoothpaste_b200 import GpuLWEtoRLWEPacker
+def case_pack_n2048(torch, modular: int = 0):
+    """ks_fft_kernel merge levels: 8 packs of 2048 LWEs (n=N=2048), l=4."""
+    from fhetoothpaste_b200 import GpuLWEtoRLWEPacker, _native
     N, L, packs, l = 2048, 2048, 8, 4
     packer = GpuLWEtoRLWEPacker(N, 1 << 16, l, _u64(9, 11 * 2 * N * l))
+    _native.check(_native.lib().tp_debug_ks_modular(packer._h, modular))
     x = _dev(torch, _u64(10, (packs * L, N + 1)))
     y = torch.empty((packs, 2 * N), dtype=torch.int64, device="cuda")
     for _ in range(2):
@@ -164,17 +190,27 @@ def case_pack_n2048(torch):
     packer.close()
 
 
-def case_lwe_ks_2048_630(torch):
-    """lwe_ks_kernel: 4096 LWE ciphertexts n=2048 -> n=630, base 2^16 l=4 (41 MB key)."""
+def case_pack_modular_n2048(torch):
+    """pack_l0_kernel + ks_kernel merge levels, as pack_n2048."""
+    case_pack_n2048(torch, modular=1)
+
+
+def case_lwe_ks_2048_630(torch, beta: int = 16, l: int = 4):
+    """lwe_digits, lwe_mma and lwe_mma_finish kernels: 4096 LWE ciphertexts n=2048 -> n=630, base 2^16 l=4 (41 MB key)."""
     from fhetoothpaste_b200 import GpuLWEtoLWEConverter
-    n_in, n_out, l, batch = 2048, 630, 4, 4096
-    conv = GpuLWEtoLWEConverter(n_in, n_out, 1 << 16, l, _u64(11, n_in * l * (n_out + 1)))
+    n_in, n_out, batch = 2048, 630, 4096
+    conv = GpuLWEtoLWEConverter(n_in, n_out, 1 << beta, l, _u64(11, n_in * l * (n_out + 1)))
     x = _dev(torch, _u64(12, (batch, n_in + 1)))
     y = torch.zeros((batch, n_out + 1), dtype=torch.int64, device="cuda")
     for _ in range(2):
         conv.convert_batch(batch, y.data_ptr(), x.data_ptr())
     torch.cuda.synchronize()
     conv.close()
+
+
+def case_lwe_ks_scalar_2048_630(torch):
+    """lwe_ks_kernel (digits above 16 bits): 4096 LWE ciphertexts n=2048 -> n=630, base 2^20 l=3 (31 MB key)."""
+    case_lwe_ks_2048_630(torch, 20, 3)
 
 
 def case_sample_extract_n2048(torch):
@@ -200,8 +236,8 @@ def case_key_retile_n2048(torch):
 
 def case_lwe_to_rgsw_n2048(torch):
     """LWE -> RGSW scheme switching, 256 LWEs (CGGI binary n=100, N=2048, gadgets 2^14 l=4, out 4
-    digits): br_kernel, ss_rows_kernel, 11 trace ks_kernel launches, ntt_batch_kernel x2,
-    ks_kernel (s^2 -> s), ss_assemble_kernel per conversion call."""
+    digits): br_fft_pair_kernel, ss_rows_kernel, 11 trace ks_fft_kernel launches, ntt_batch_kernel x2,
+    ks_rlwe_kernel (s^2 -> s), ss_assemble_kernel per conversion call."""
     from fhetoothpaste_b200 import BlindRotationContext, GpuLWEtoRGSWConverter
     N, n, beta, l, D, batch = 2048, 100, 14, 4, 4, 256
     words = BlindRotationContext(0, N, n, 1 << beta, l).key_words()
@@ -217,8 +253,8 @@ def case_lwe_to_rgsw_n2048(torch):
 
 def case_sap_n4096(torch):
     """SAP digit decomposition, 16 LWEs (CGGI binary n=10, N=4096, gadgets 2^16 l=4, radix 32,
-    inputs mod 2^40: 8 digits): br_kernel, ks_kernel (trace and split modes), ntt_batch_kernel,
-    lwe_ks_kernel and the element-wise SAP kernels, per decomposition call."""
+    inputs mod 2^40: 8 digits): br_fft_halves_kernel or br_fft_cluster_kernel, ks_kernel (trace and split
+    modes), ntt_batch_kernel, the LWE switch's kernels and the element-wise SAP kernels, per call."""
     from fhetoothpaste_b200 import BlindRotationContext, GpuSAPDecomposer
     N, n, l, batch = 4096, 10, 4, 16
     words = BlindRotationContext(0, N, n, 1 << 16, l).key_words()
