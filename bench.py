@@ -284,8 +284,8 @@ BMMP_BATCHES = (1, 37, 512, 2048, 8192)
 
 def bmmp_batch_sweep(device: int) -> dict:
     """BMMP (binary n=768 as 384 pairs, N=2048, base 2^16 l=4) at uneven batch sizes,
-    identity test polynomials; per batch size the autotuner picks the tile and the
-    blocks per rotation, then one graph-recorded launch per step is timed."""
+    identity test polynomials; per batch size the autotuner picks the launch form,
+    then one graph-recorded launch per step is timed."""
     import torch
     from fhetoothpaste_b200 import BlindRotationContext, GpuBlindRotator
     from oracle.oracle import lwe_inputs
@@ -295,7 +295,9 @@ def bmmp_batch_sweep(device: int) -> dict:
     stream = torch.cuda.current_stream().cuda_stream
     ident = np.zeros(2 * N, np.uint64)
     ident[N:] = np.arange(N, dtype=np.uint64)
-    out = {"workload": "BMMP n=768 (384 pairs), N=2048, base 2^16 l=4, identity LUT", "unit": "BR/s"}
+    out = {"workload": "BMMP n=768 (384 pairs), N=2048, base 2^16 l=4, identity LUT", "unit": "BR/s",
+           "tile": "settings of the modular kernels; at 4 per thread, 1 block and form 1 (a new context's) the form is "
+                   "chosen by batch size"}
     lw_all = torch.from_numpy(lwe_inputs(N, n, max(BMMP_BATCHES), 33).view(np.int64)).cuda()
     ac = torch.from_numpy(ident.view(np.int64)).cuda()
     res = torch.empty((max(BMMP_BATCHES), 2 * N), dtype=torch.int64, device="cuda")

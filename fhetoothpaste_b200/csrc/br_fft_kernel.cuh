@@ -1,6 +1,7 @@
 // CGGI blind rotation with double-precision transforms (fft_block.cuh): same words as
 // br_kernels.cuh, whose modular transforms it replaces where the key passes the error
-// bound (binary and ternary, N = 1024 and 2048, 2 to 4 digits).
+// bound (binary and ternary, 2 to 4 digits; one block and the pair at N = 1024 and 2048, clusters at
+// 1024 to 4096, halves on two blocks at 4096).
 //
 // One block per rotation, the accumulator in shared memory as coefficients (pairs j,
 // j + N/2) for all n iterations. Per iteration (cggi_blind_rotation.cpp:364-432):
@@ -12,9 +13,10 @@
 // The products by monomials outside the transforms are index shifts.
 //
 // What bounds it: the key words grow from 8 bytes a coefficient to 8 per limb (1.18 MB an
-// iteration, ternary N = 2048), read at 71 of the 75 bytes a clock that one SM gets from L2;
-// that phase takes 45% of an iteration, the FP64 pipe is busy for a third of it, and the rest
-// are the transforms' passes through shared memory and their barriers. Measured against the
+// iteration, ternary N = 2048); by clock counters in the kernel the products take 45% of an
+// iteration, which is 71 of the 75 bytes a clock that a copy loop on every SM gets from L2. The FP64
+// pipe is busy for a third of the time, and the rest are the transforms' passes through shared memory
+// and their barriers (L1 and shared memory at 66 to 85% of their peak, by ncu). Measured against the
 // modular kernels: ternary N = 2048, n = 630, 4096 rotations 452.7 -> 317.3 ms; 1024
 // bootstraps of binary N = 1024, n = 500 55.7 -> 40.6 ms.
 //

@@ -15,8 +15,9 @@
 // 1084 clocks of the tensor pipe, 60 of the 75 bytes a clock that an SM gets from L2; two
 // accumulators of 256 columns fill TMEM. K is split over several blocks per tile where the
 // tiles alone leave the last wave, or the GPU, idle. Measured against lwe_ks_kernel (2048 -> 630,
-// base 2^16, l = 4): 4096 ciphertexts 10.67 ms -> 0.285 ms (1.19 P byte products a second, half
-// of the tensor pipe's rate), 100 of them 1803 -> 25 us, one 1764 -> 25 us.
+// base 2^16, l = 4): 4096 ciphertexts 10.80 ms -> 0.329 ms (the product alone 0.242 ms: 1.40 P byte
+// products a second, the tensor pipe busy three quarters of the time), 100 of them 1803 -> 25 us,
+// one 1764 -> 25 us. A context's first call maps its workspace as well: 1.3 ms at this size.
 #pragma once
 
 #include <cuda.h>
