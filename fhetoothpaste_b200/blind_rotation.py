@@ -115,7 +115,8 @@ class GpuBlindRotator:
 
     @property
     def tile(self) -> int:
-        """Coefficients per thread of the rotation kernel (8 or 4)."""
+        """Coefficients per thread of the modular rotation kernel (8 or 4). While tile, split, mac_form and
+        radix are a new rotator's own the launch form is chosen by batch size, whatever they say."""
         return int(nat.lib().tp_br_get_tile(self._h))
 
     def set_tile(self, coef_per_thread: int) -> None:
@@ -123,7 +124,7 @@ class GpuBlindRotator:
 
     @property
     def split(self) -> int:
-        """Thread blocks per rotation (1, or 2 / 4 for the cluster kernels)."""
+        """Thread blocks per rotation of the modular kernels (1, or 2 / 4 for the cluster kernels)."""
         return int(nat.lib().tp_br_get_split(self._h))
 
     def set_split(self, blocks_per_rotation: int) -> None:

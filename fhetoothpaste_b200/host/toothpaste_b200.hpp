@@ -115,7 +115,9 @@ public:
                           uint64_t acc_stride, bool output_as_coefficients = false);
     // GPU launch form (no reference counterpart; same output words in every form):
     // coefficients per thread (4 or 8), thread blocks per rotation (1, 2 or 4; 2 and 4
-    // need 4 per thread), or both chosen by timing `batch` synthetic rotations.
+    // need 4 per thread), or both chosen by timing `batch` synthetic rotations. While these
+    // settings are a new rotator's own the form is chosen by batch size; setting them back
+    // restores that.
     void SetTile(uint32_t coef_per_thread);
     void SetSplit(uint32_t blocks_per_rotation);
     // multiply-accumulate form (TP_MAC_ROWWISE / TP_MAC_DIGIT_STAGED) and NTT radix (2 or 4)
